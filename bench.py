@@ -780,8 +780,8 @@ def kernel_name(degree, arith):
     pol = "ArithDF" if arith == 1 else "ArithF64"
     return {0: f"bk5_kernel<{n},{pol}>", 1: f"bk5_pt_kernel<{n},{pol}>",
             2: f"bk5_tma_kernel<{n},{pol}>", 3: f"bk5_kernel_mb<{n},{pol}>",
-            4: f"bk5_tma_kernel<{n},alt,{pol}>", 5: f"bk5fx_tma_kernel<{n}>",
-            6: f"bk5fx_tma_kernel<{n},alt>"}.get(shape.value, "bk5")
+            4: f"bk5_tma_kernel<{n},alt,{pol}>", 5: f"bk5fx_kernel<{n}>",
+            6: f"bk5fx_kernel<{n},alt>"}.get(shape.value, "bk5")
 
 
 def main():

@@ -194,7 +194,7 @@ mfgb_status vmult_impl(mfgb_operator *op, double *dst, const double *src, int ar
 // shape per degree measured on a GB300 at ~3e7 DoFs (autotune.py re-measures).
 static int g_shape[3][10] = {
     {0, 0, 4, 3, 2, 4, 2, 1, 2, 1},  // FP64
-    {2, 2, 6, 6, 6, 5, 6, 6, 5, 5},  // double-float (5, 6: offset accumulation)
+    {2, 2, 5, 5, 5, 5, 5, 5, 5, 5},  // double-float (5, 6: offset accumulation)
     {0, 0, 3, 3, 0, 3, 2, 4, 4, 2},  // FP32
 };
 
@@ -829,8 +829,13 @@ mfgb_status mfgb_vmult_host(const mfgb_operator *cop, double *h_dst, const doubl
         return cuda_status(cudaErrorUnknown, "mfgb_vmult_host: streams");
   const int p = op->degree;
   const int nz = op->is_box ? op->box.nz : 1;
-  // >= 2 cell layers a slab; 16 slabs unless set by mfgb_set_host_pipeline
-  const int want = g_host_slabs > 0 ? g_host_slabs : 16;
+  // >= 2 cell layers a slab.  Every slab costs two copies and two launches, and the first copy in
+  // and the last one out are not overlapped: the best count grows with the square root of the
+  // vector.  Measured best counts (double-float, us against 16 slabs): 8 MB 2 (120 / 189), 17 MB 3
+  // (193 / 342), 33 MB 6 (303 / 415), 65 MB 6-10 (530 / 541), 136 MB 8 (999 / 1020), 159 MB 10
+  // (1166 / 1184), 456 MB 16-24 (3006 / 3021).
+  const int fit = std::max(2, (int)std::lround(0.75 * std::sqrt(8e-6 * (double)op->n_dofs)));
+  const int want = g_host_slabs > 0 ? g_host_slabs : std::min(fit, 24);
   const int S = op->is_box ? std::max(1, std::min(want, nz / 2)) : 1;
   const int Lz = (nz + S - 1) / S;
   const int n_ev = 3 * S + 1;  // S <= 64

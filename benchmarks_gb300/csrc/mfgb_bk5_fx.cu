@@ -11,24 +11,35 @@
 
 namespace mfgb {
 
-// cells per CTA and resident CTAs per SM of the two thread-block shapes
-// (shape 4 = the alternative cells per CTA of mfgb_launch.cuh)
-template <int N> struct FxElems { static constexpr int value = ElemsPerCtaTma<N, ArithDF>::value; };
-template <int N> struct FxMinBlocks { static constexpr int value = TmaMinBlocks<N, ArithDF>::value; };
-template <int N> struct FxAltElems { static constexpr int value = AltElemsN<N>::value; };
-template <int N> struct FxAltMinBlocks {
-  static constexpr int value = AltMinBlocks<N, FxAltElems<N>::value, ArithDF>::value;
+// Cells per CTA, resident CTAs per SM and work arrays of the two thread-block shapes (5 and 6 of
+// the shape table).  Cells per CTA fill whole warps as far as they can (n = 5: 125 of 128 lanes,
+// n = 6: 108 of 128, n = 7: 147 of 160); from n = 5 the two-array form buys one more resident CTA
+// (n = 5: 44.8 KB a CTA, 96 registers, 5 CTAs: 0.649 ms at 3e7 DoFs; three arrays, 4 CTAs: 0.654).
+// ms at 3e7 DoFs, shape 5 / 6: n = 2 3.05 / 3.11, 3 1.21 / 1.21, 4 0.74 / 0.75, 5 0.65 / 0.65,
+// 6 0.70 / 0.73, 7 0.72 / 0.81, 8 0.63 / 0.65, 9 0.80 / 0.80 (the kernel with one contraction
+// output per thread and step that this one replaced, its better shape: 3.90, 1.97, 1.06, 1.00,
+// 1.14, 1.33, 1.07, 1.83).
+template <int E_, int MB_, int NB_> struct FxShape {
+  static constexpr int E = E_, MB = MB_, NB = NB_;
 };
-// n = 7..9: fewer cells per CTA and more resident CTAs (registers from -Xptxas
-// -v: n = 7, 2 cells, 3 CTAs: 158, no spill; n = 8, 1 cell, 4 CTAs: 179, no
-// spill; n = 9, 2 cells, 2 CTAs: 168 with a 48-byte spill, 1 cell, 3 CTAs: 168
-// with 32 bytes), where the wide cells of 1-CTA shapes left too few warps
-template <> struct FxElems<7> { static constexpr int value = 2; };
-template <> struct FxMinBlocks<7> { static constexpr int value = 3; };
-template <> struct FxAltMinBlocks<8> { static constexpr int value = 4; };
-template <> struct FxMinBlocks<9> { static constexpr int value = 2; };
-template <> struct FxAltElems<9> { static constexpr int value = 1; };
-template <> struct FxAltMinBlocks<9> { static constexpr int value = 3; };
+template <int N> struct FxDefault;
+template <int N> struct FxAlt;
+template <> struct FxDefault<2> : FxShape<32, 4, 3> {};
+template <> struct FxDefault<3> : FxShape<7, 6, 3> {};
+template <> struct FxDefault<4> : FxShape<4, 7, 3> {};
+template <> struct FxDefault<5> : FxShape<5, 5, 2> {};
+template <> struct FxDefault<6> : FxShape<3, 5, 2> {};
+template <> struct FxDefault<7> : FxShape<3, 3, 2> {};
+template <> struct FxDefault<8> : FxShape<2, 3, 2> {};
+template <> struct FxDefault<9> : FxShape<1, 4, 2> {};
+template <> struct FxAlt<2> : FxShape<16, 6, 3> {};
+template <> struct FxAlt<3> : FxShape<14, 4, 3> {};
+template <> struct FxAlt<4> : FxShape<8, 4, 3> {};
+template <> struct FxAlt<5> : FxShape<5, 4, 3> {};
+template <> struct FxAlt<6> : FxShape<5, 3, 2> {};
+template <> struct FxAlt<7> : FxShape<2, 4, 2> {};
+template <> struct FxAlt<8> : FxShape<1, 5, 2> {};
+template <> struct FxAlt<9> : FxShape<2, 2, 2> {};
 
 // test hook: applications left whose first copy wait is made to run out
 static std::atomic<int> g_expire{0};
@@ -39,187 +50,118 @@ static bool take_expire() {
   return false;
 }
 
-template <int N, int E, int MB, bool MT>
-static cudaError_t fx_launch(int64_t n_cells, const uint32_t *map, const float2 *G, const int *gexp,
-                             const double *src, double *dst, const BasisFX<N> &b, cudaStream_t s,
-                             const int *done) {
-  constexpr size_t smem = TmaLayout<N, E, ArithDF>::total;
+template <int N, int SYM>
+static bool fx_basis(const double *D, FxBasis<N, SYM> &b) {
+  double Dt[N * N];
+  for (int i = 0; i < N; ++i)
+    for (int m = 0; m < N; ++m) Dt[i * N + m] = D[m * N + i];
+  b.K = (float)(2.0 * (1.0 + std::ldexp(1.0, -20)));
+  return fx_line_matrix<N, N, SYM>(D, b.G) && fx_line_matrix<N, N, SYM>(Dt, b.T);
+}
+
+// one launch of the kernel: all resident CTAs, capped by the batches
+template <int N, class Sh, class GT, bool EVEC, int NC, int SYM, bool MT, bool EXPIRE = false>
+static cudaError_t fx_run(int64_t n_cells, const uint32_t *map, const GT *G, const int *gexp,
+                          const double *src, double *dst, const FxBasis<N, SYM> &b, cudaStream_t s,
+                          const int *done) {
+  constexpr int E = Sh::E, T = E * N * N;
+  constexpr size_t smem = FxLayout<N, E, GT, EVEC, Sh::NB>::total;
+  const auto kernel = bk5fx_kernel<N, E, Sh::MB, Sh::NB, GT, EVEC, NC, SYM, MT, EXPIRE>;
   static int per_sm = -1;
-  if (per_sm < 0)
-    per_sm = std::max(1, ctas_per_sm(bk5fx_tma_kernel<N, E, MB, MT>, E * N * N, smem));
+  if (per_sm < 0) per_sm = std::max(1, ctas_per_sm(kernel, T, smem));
   const int64_t nb = (n_cells + E - 1) / E;
   const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(nb, (int64_t)per_sm * num_sms()));
-  if (n_cells <= 0) return cudaSuccess;
-  bk5fx_tma_kernel<N, E, MB, MT><<<grid, E * N * N, smem, s>>>(n_cells, map, G, gexp, src, dst, b,
-                                                                done, device_error_flag());
+  kernel<<<grid, T, smem, s>>>(n_cells, map, G, gexp, src, dst, b, done, device_error_flag());
   return cudaGetLastError();
 }
 
-// one application with the copy-wait test hook (the default cells per CTA)
-template <int N>
-static cudaError_t fx_launch_expire(int64_t n_cells, const uint32_t *map, const float2 *G,
-                                    const int *gexp, const double *src, double *dst,
-                                    const BasisFX<N> &b, cudaStream_t s, const int *done) {
-  constexpr int E = FxElems<N>::value, MB = FxMinBlocks<N>::value;
-  constexpr size_t smem = TmaLayout<N, E, ArithDF>::total;
-  ctas_per_sm(bk5fx_tma_kernel<N, E, MB, false, true>, E * N * N, smem);  // sets the smem limit
-  const int64_t nb = (n_cells + E - 1) / E;
-  const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(nb, (int64_t)num_sms()));
-  bk5fx_tma_kernel<N, E, MB, false, true><<<grid, E * N * N, smem, s>>>(
-      n_cells, map, G, gexp, src, dst, b, done, device_error_flag());
-  return cudaGetLastError();
-}
-
-template <int N>
-static cudaError_t fx_with_basis(int64_t n_cells, const uint32_t *map, const float2 *G,
-                                 const int *gexp, const double *src, double *dst, const double *D,
-                                 cudaStream_t s, const int *done) {
-  BasisFX<N> b;
-  const double K = 2.0 * (1.0 + std::ldexp(1.0, -20));
-  for (int q = 0; q < N * N; ++q) {
-    b.Dh[q] = (float)D[q];
-    b.Dl[q] = (float)(D[q] - (double)b.Dh[q]);
-  }
-  for (int i = 0; i < N; ++i) {
-    double rs = 0.0, cs = 0.0;
-    for (int m = 0; m < N; ++m) {
-      rs += std::fabs((double)b.Dh[i * N + m]);
-      cs += std::fabs((double)b.Dh[m * N + i]);
-    }
-    b.cg[i] = (float)(K * rs);
-    b.ci[i] = (float)(K * cs);
-  }
-  b.K = (float)K;
-  // bulk copies of the dof-map tiles need a 16-byte aligned map
+// The kernel on the library's own scaled pairs.  Bulk copies of the dof-map tiles need a 16-byte
+// aligned map.
+template <int N, int NC>
+static cudaError_t fx_pairs(int64_t n_cells, const uint32_t *map, const float2 *G, const int *gexp,
+                            const double *src, double *dst, const double *D, cudaStream_t s,
+                            const int *done) {
+  FxBasis<N, -1> b;
+  if (!fx_basis<N, -1>(D, b)) return cudaErrorInvalidValue;  // the GLL derivative has the symmetry
+  using Sh = FxDefault<N>;
   const bool mt = (reinterpret_cast<uintptr_t>(map) & 15u) == 0;
-  const bool alt = kernel_shape(ArithClass<ArithDF>::value, N) == SHAPE_FX_ALT;
-  constexpr int E = FxElems<N>::value, MB = FxMinBlocks<N>::value;
-  constexpr int EA = FxAltElems<N>::value, MBA = FxAltMinBlocks<N>::value;
-  if (take_expire()) return fx_launch_expire<N>(n_cells, map, G, gexp, src, dst, b, s, done);
-  if (alt)
-    return mt ? fx_launch<N, EA, MBA, true>(n_cells, map, G, gexp, src, dst, b, s, done)
-              : fx_launch<N, EA, MBA, false>(n_cells, map, G, gexp, src, dst, b, s, done);
-  return mt ? fx_launch<N, E, MB, true>(n_cells, map, G, gexp, src, dst, b, s, done)
-            : fx_launch<N, E, MB, false>(n_cells, map, G, gexp, src, dst, b, s, done);
+  if (NC == 1 && take_expire())
+    return fx_run<N, Sh, float2, false, 1, -1, false, true>(n_cells, map, G, gexp, src, dst, b, s,
+                                                            done);
+  if constexpr (NC == 1) {
+    using Alt = FxAlt<N>;
+    if (kernel_shape(ArithClass<ArithDF>::value, N) == SHAPE_FX_ALT)
+      return mt ? fx_run<N, Alt, float2, false, 1, -1, true>(n_cells, map, G, gexp, src, dst, b, s, done)
+                : fx_run<N, Alt, float2, false, 1, -1, false>(n_cells, map, G, gexp, src, dst, b, s, done);
+  }
+  return mt ? fx_run<N, Sh, float2, false, NC, -1, true>(n_cells, map, G, gexp, src, dst, b, s, done)
+            : fx_run<N, Sh, float2, false, NC, -1, false>(n_cells, map, G, gexp, src, dst, b, s, done);
 }
 
-// the basis pairs and bound factors of the collocation kernels
+// The kernel on the caller's FP64 G (16-byte aligned): L-vectors through map, or element vectors
+// (map == nullptr).  A derivative matrix without the mirror symmetry of symmetric points keeps
+// the general form.
+template <int N, int SYM>
+static cudaError_t fx_seam(int64_t n_cells, const uint32_t *map, const double *G, const double *src,
+                           double *dst, const FxBasis<N, SYM> &b, cudaStream_t s) {
+  // FP64 tiles take twice the shared memory of pairs: fewer resident CTAs
+  using Sh = FxShape<FxDefault<N>::E, (FxDefault<N>::MB + 1) / 2, FxDefault<N>::NB>;
+  if (map == nullptr)
+    return fx_run<N, Sh, double, true, 1, SYM, false>(n_cells, nullptr, G, nullptr, src, dst, b, s, nullptr);
+  if (reinterpret_cast<uintptr_t>(map) & 15u)
+    return fx_run<N, Sh, double, false, 1, SYM, false>(n_cells, map, G, nullptr, src, dst, b, s, nullptr);
+  return fx_run<N, Sh, double, false, 1, SYM, true>(n_cells, map, G, nullptr, src, dst, b, s, nullptr);
+}
+
 template <int N>
-static BasisFX<N> basis_fx(const double *D) {
-  BasisFX<N> b;
-  const double K = 2.0 * (1.0 + std::ldexp(1.0, -20));
-  for (int q = 0; q < N * N; ++q) {
-    b.Dh[q] = (float)D[q];
-    b.Dl[q] = (float)(D[q] - (double)b.Dh[q]);
-  }
-  for (int i = 0; i < N; ++i) {
-    double rs = 0.0, cs = 0.0;
-    for (int m = 0; m < N; ++m) {
-      rs += std::fabs((double)b.Dh[i * N + m]);
-      cs += std::fabs((double)b.Dh[m * N + i]);
-    }
-    b.cg[i] = (float)(K * rs);
-    b.ci[i] = (float)(K * cs);
-  }
-  b.K = (float)K;
-  return b;
+static cudaError_t fx_seam_any(int64_t n_cells, const uint32_t *map, const double *G,
+                               const double *src, double *dst, const double *D, cudaStream_t s) {
+  FxBasis<N, -1> b;
+  if (fx_basis<N, -1>(D, b)) return fx_seam<N, -1>(n_cells, map, G, src, dst, b, s);
+  FxBasis<N, 0> general;
+  fx_basis<N, 0>(D, general);
+  return fx_seam<N, 0>(n_cells, map, G, src, dst, general, s);
 }
 
-// the L-vector form on the caller's FP64 G (16-byte aligned)
-template <int N, bool MT>
-static cudaError_t fx_g64_launch(int64_t n_cells, const uint32_t *map, const double *G,
-                                 const double *src, double *dst, const double *D,
-                                 cudaStream_t s) {
-  const BasisFX<N> b = basis_fx<N>(D);
-  constexpr int E = FxElems<N>::value, MB = FxMinBlocks<N>::value;
-  constexpr size_t smem = TmaLayout<N, E, ArithF64>::total;
-  static int per_sm = -1;
-  if (per_sm < 0) per_sm = std::max(1, ctas_per_sm(bk5fx_g64_kernel<N, E, MB, MT>, E * N * N, smem));
-  const int64_t nb = (n_cells + E - 1) / E;
-  const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(nb, (int64_t)per_sm * num_sms()));
-  bk5fx_g64_kernel<N, E, MB, MT><<<grid, E * N * N, smem, s>>>(n_cells, map, G, src, dst, b,
-                                                                device_error_flag());
-  return cudaGetLastError();
-}
+#define MFGB_FX_DEGREES(CALL) \
+  switch (N) {                \
+    case 2: return CALL(2);   \
+    case 3: return CALL(3);   \
+    case 4: return CALL(4);   \
+    case 5: return CALL(5);   \
+    case 6: return CALL(6);   \
+    case 7: return CALL(7);   \
+    case 8: return CALL(8);   \
+    case 9: return CALL(9);   \
+    default: return cudaErrorInvalidValue; \
+  }
 
 cudaError_t bk5_fx_g64(int N, int64_t n_cells, const uint32_t *map, const double *G,
                        const double *src, double *dst, const double *D, cudaStream_t s) {
   if (n_cells <= 0) return cudaSuccess;
   if (map == nullptr || (reinterpret_cast<uintptr_t>(G) & 15u)) return cudaErrorInvalidValue;
-  const bool mt = (reinterpret_cast<uintptr_t>(map) & 15u) == 0;
-  switch (N) {
-#define MFGB_FXG(NN)                                                      \
-  case NN:                                                                \
-    return mt ? fx_g64_launch<NN, true>(n_cells, map, G, src, dst, D, s) \
-              : fx_g64_launch<NN, false>(n_cells, map, G, src, dst, D, s);
-    MFGB_FXG(2) MFGB_FXG(3) MFGB_FXG(4) MFGB_FXG(5) MFGB_FXG(6) MFGB_FXG(7) MFGB_FXG(8) MFGB_FXG(9)
-#undef MFGB_FXG
-    default: return cudaErrorInvalidValue;
-  }
-}
-
-// the E-vector form: FP64 G (16-byte aligned), contiguous input and output
-template <int N>
-static cudaError_t fx_evec_with_basis(int64_t nelmt, const double *G, const double *src,
-                                      double *dst, const double *D, cudaStream_t s) {
-  const BasisFX<N> b = basis_fx<N>(D);
-  constexpr int E = FxElems<N>::value, MB = FxMinBlocks<N>::value;
-  constexpr size_t smem = TmaLayout<N, E, ArithF64>::total;
-  static int per_sm = -1;
-  if (per_sm < 0) per_sm = std::max(1, ctas_per_sm(bk5fx_evec_kernel<N, E, MB>, E * N * N, smem));
-  const int64_t nb = (nelmt + E - 1) / E;
-  const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(nb, (int64_t)per_sm * num_sms()));
-  bk5fx_evec_kernel<N, E, MB><<<grid, E * N * N, smem, s>>>(nelmt, G, src, dst, b,
-                                                            device_error_flag());
-  return cudaGetLastError();
+#define MFGB_CALL(NN) (fx_seam_any<NN>(n_cells, map, G, src, dst, D, s))
+  MFGB_FX_DEGREES(MFGB_CALL)
+#undef MFGB_CALL
 }
 
 cudaError_t bk5_fx_evec(int N, int64_t nelmt, const double *G, const double *src, double *dst,
                         const double *D, cudaStream_t s) {
   if (nelmt <= 0) return cudaSuccess;
   if (reinterpret_cast<uintptr_t>(G) & 15u) return cudaErrorInvalidValue;  // bulk copies
-  switch (N) {
-#define MFGB_FXEV(NN) \
-  case NN: return fx_evec_with_basis<NN>(nelmt, G, src, dst, D, s);
-    MFGB_FXEV(2) MFGB_FXEV(3) MFGB_FXEV(4) MFGB_FXEV(5) MFGB_FXEV(6) MFGB_FXEV(7) MFGB_FXEV(8)
-    MFGB_FXEV(9)
-#undef MFGB_FXEV
-    default: return cudaErrorInvalidValue;
-  }
+#define MFGB_CALL(NN) (fx_seam_any<NN>(nelmt, nullptr, G, src, dst, D, s))
+  MFGB_FX_DEGREES(MFGB_CALL)
+#undef MFGB_CALL
 }
 
 // the BK6 vector Laplacian: 3 interleaved components per DoF on one scaled G
-template <int N, bool MT>
-static cudaError_t fx_bk6_launch(int64_t n_cells, const uint32_t *map, const float2 *G,
-                                 const int *gexp, const double *src, double *dst, const double *D,
-                                 cudaStream_t s) {
-  const BasisFX<N> b = basis_fx<N>(D);
-  constexpr int E = FxElems<N>::value, MB = FxMinBlocks<N>::value;
-  constexpr size_t smem = TmaLayout<N, E, ArithDF>::total;
-  static int per_sm = -1;
-  if (per_sm < 0)
-    per_sm = std::max(1, ctas_per_sm(bk6fx_tma_kernel<N, E, MB, MT, 3>, E * N * N, smem));
-  const int64_t nb = (n_cells + E - 1) / E;
-  const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(nb, (int64_t)per_sm * num_sms()));
-  bk6fx_tma_kernel<N, E, MB, MT, 3><<<grid, E * N * N, smem, s>>>(n_cells, map, G, gexp, src, dst,
-                                                                  b, device_error_flag());
-  return cudaGetLastError();
-}
-
 cudaError_t bk6_fx(int N, int64_t n_cells, const uint32_t *map, const float2 *G, const int *gexp,
                    const double *src, double *dst, const double *D, cudaStream_t s) {
   if (n_cells <= 0) return cudaSuccess;
   if (map == nullptr || (reinterpret_cast<uintptr_t>(G) & 15u)) return cudaErrorInvalidValue;
-  const bool mt = (reinterpret_cast<uintptr_t>(map) & 15u) == 0;
-  switch (N) {
-#define MFGB_FX6(NN)                                                              \
-  case NN:                                                                        \
-    return mt ? fx_bk6_launch<NN, true>(n_cells, map, G, gexp, src, dst, D, s) \
-              : fx_bk6_launch<NN, false>(n_cells, map, G, gexp, src, dst, D, s);
-    MFGB_FX6(2) MFGB_FX6(3) MFGB_FX6(4) MFGB_FX6(5) MFGB_FX6(6) MFGB_FX6(7) MFGB_FX6(8) MFGB_FX6(9)
-#undef MFGB_FX6
-    default: return cudaErrorInvalidValue;
-  }
+#define MFGB_CALL(NN) (fx_pairs<NN, 3>(n_cells, map, G, gexp, src, dst, D, s, nullptr))
+  MFGB_FX_DEGREES(MFGB_CALL)
+#undef MFGB_CALL
 }
 
 cudaError_t bk5_fx(int N, int64_t n_cells, const uint32_t *map, const float2 *G, const int *gexp,
@@ -227,14 +169,9 @@ cudaError_t bk5_fx(int N, int64_t n_cells, const uint32_t *map, const float2 *G,
                    const int *done) {
   if (n_cells <= 0) return cudaSuccess;
   if (map == nullptr || (reinterpret_cast<uintptr_t>(G) & 15u)) return cudaErrorInvalidValue;
-  switch (N) {
-#define MFGB_FXCASE(NN) \
-  case NN: return fx_with_basis<NN>(n_cells, map, G, gexp, src, dst, D, s, done);
-    MFGB_FXCASE(2) MFGB_FXCASE(3) MFGB_FXCASE(4) MFGB_FXCASE(5) MFGB_FXCASE(6) MFGB_FXCASE(7)
-    MFGB_FXCASE(8) MFGB_FXCASE(9)
-#undef MFGB_FXCASE
-    default: return cudaErrorInvalidValue;
-  }
+#define MFGB_CALL(NN) (fx_pairs<NN, 1>(n_cells, map, G, gexp, src, dst, D, s, done))
+  MFGB_FX_DEGREES(MFGB_CALL)
+#undef MFGB_CALL
 }
 
 // Per-cell scaled split of the FP64 geometric factors: one warp per cell finds

@@ -6,7 +6,7 @@
 // transpose, atomic scatter; reference CEED_BK/include/kernels/BK5/
 // templated_cuda_kernels.cuh:50-122 and bakeoff_problems_dealii/include/
 // bk3_kokkos_kernel.h:129-151, 406-426) with the same bulk-TMA pipeline.  What
-// differs is the arithmetic:
+// differs is the arithmetic and the split of the contractions over the threads:
 //
 // * Scaling.  Every cell's gathered values are multiplied by 2^-su, su chosen
 //   from the largest binary exponent among them so that |u| < 1, and the
@@ -25,60 +25,29 @@
 //   and at the end hi = T - C is exact (Sterbenz), lo = S.  That is 6 FP32-pipe
 //   instructions per multiply-add (5 for the first), against 12 for the
 //   TwoSum-based form of ArithDF, with an error of about 2^-46 of C.  The bounds
-//   B come from the data at hand: |u| < 1 for the gradient (B = sum_m |D[i][m]|),
-//   max |q| times the row sum of |G| per point for the metric, and the line
-//   maxima of |v| times the column sums of |D| for the transpose.
+//   B come from the data at hand: |u| < 1 for the gradient, max |q| times the
+//   row sum of |G| per point for the metric, and each line's maximum for the
+//   transpose.
 //
-// A float32 restatement of this arithmetic with its error bound is in
-// tests/test_fx_arith.py.
+// * Line ownership (mfgb_fxline.cuh).  In every contraction a thread owns a whole
+//   line, with the derivative matrix in even-odd form.
+//
+// What bounds it (p = 4, ncu at 3e7 DoFs, before the lines were dealt to banks): 1,250
+// warp-instructions a cell against 1,637 of the kernel with one output per thread and step (FADD +
+// FFMA 751 against 963, shared loads and stores 82 against 133), 70 % of the issue slots, 73 % of
+// the shared-memory pipe, 5 CTAs an SM instead of 4.  67.6M DoFs: a vmult 2.22 -> 1.59 ms; 43 -> 45 GDoF/s at
+// 3e7 with the dealt lines, 79 % of the measured copy bandwidth; p = 6 and 8 (n^4 arithmetic per
+// n^3 bytes) stay at 62 % and 51 %, bound by issue.
+//
+// Float32 restatements of this arithmetic with their error bounds are in
+// tests/test_fx_arith.py and tests/test_fx_line.py.
 #pragma once
+#include <type_traits>
+
 #include "mfgb_bk5.cuh"
+#include "mfgb_fxline.cuh"
 
 namespace mfgb {
-
-// D split into float pairs plus the bound factors of the two contractions:
-//   cg[i] = K * sum_m |Dh[i][m]|  (gradient output i, |data| < 1)
-//   ci[i] = K * sum_m |Dh[m][i]|  (transpose output i, per unit of line maximum)
-//   K = 2 (1 + 2^-20): the factor 2 of the offset, plus a margin for the float
-//   rounding of the bound itself
-template <int N>
-struct BasisFX {
-  float Dh[N * N], Dl[N * N];
-  float cg[N], ci[N];
-  float K;
-};
-
-// offset accumulator: value = (T - C) + S
-struct fxacc {
-  float T, S;
-};
-
-__device__ __forceinline__ void fx_first(fxacc &a, float xh, float xl, float yh, float yl,
-                                         float C) {
-  a.T = __fmaf_rn(xh, yh, C);
-  const float d = __fsub_rn(a.T, C);
-  const float r = __fmaf_rn(xh, yh, -d);
-  a.S = __fmaf_rn(xl, yh, __fmaf_rn(xh, yl, r));
-}
-
-// the low-order terms of one product (its rounding error and the two cross
-// products) are summed first and join S with one addition: the two chains a
-// sum carries (T and S) advance by one dependent instruction per term
-__device__ __forceinline__ void fx_fma(fxacc &a, float xh, float xl, float yh, float yl) {
-  const float t = __fmaf_rn(xh, yh, a.T);
-  const float d = __fsub_rn(t, a.T);
-  const float r = __fmaf_rn(xh, yh, -d);
-  const float e = __fmaf_rn(xl, yh, __fmaf_rn(xh, yl, r));
-  a.S = __fadd_rn(a.S, e);
-  a.T = t;
-}
-
-__device__ __forceinline__ df fx_finish(const fxacc &a, float C) {
-  df r;
-  r.hi = __fsub_rn(a.T, C);
-  r.lo = a.S;
-  return r;
-}
 
 // biased binary exponent of a double (0 for zero and subnormals, 2047 for inf/NaN)
 __device__ __forceinline__ int dexp(double x) {
@@ -142,77 +111,196 @@ __device__ __forceinline__ double fx_f2d_fast(float f, unsigned k) {
   return __hiloint2double((int)hi, (int)lo);
 }
 
-// a float pair from shared memory, kept at its place in the batch loop (the
-// compiler would otherwise hoist loop-invariant rows of D into registers for
-// the whole kernel)
-__device__ __forceinline__ float2 lds_pair(const float2 *p) {
-  float2 v;
-  asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];"
-               : "=f"(v.x), "=f"(v.y)
-               : "r"((unsigned)__cvta_generic_to_shared(p)));
-  return v;
-}
-
 // the scale offset of a cell from its largest biased exponent
 __device__ __forceinline__ int fx_offset(int emax) { return emax > 0 ? emax - 1022 : 0; }
 
-// Column kernel (thread (e, j, k) owns the i-column of cell e) with the bulk-TMA
-// pipeline of bk5_tma_kernel: per batch, barrier A waits for G(b) (the u(b)
-// gather was prefetched into registers during batch b-1, its largest exponent
-// per cell reduced into s_emax by shared atomics), then the scaled u goes to
-// shared memory (barrier B), map(b+next) is requested, gradient + metric run
-// (barrier C), G(b+next) is requested, u(b+next) is prefetched and the
-// transpose + atomic scatter of batch b runs.  MAPTMA = false loads the dof map
-// with plain loads (a map array that is not 16-byte aligned).  gexp[cell] is
-// the per-cell exponent offset of the scaled G.
-// EXPIRE (test hook): the first G copy is armed but not issued, and every wait
-// gives up after 1 ms, so the timeout path runs with no copy in flight.
-template <int N, int E, int MB, bool MAPTMA, bool EXPIRE = false>
+// The same for the gathered values of a cell whose largest exponent is that of a
+// normal finite number (0 < emax < 0x7FF), without branches: values more than 126
+// binades below the cell's largest come out as denormal floats instead of zeros,
+// which the rounding to the grid of 2^-22 removes.  Returns the pair on that grid
+// (offset 3, |x| < 1).
+__device__ __forceinline__ df fx_from_double_grid(double x, int off) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+  const unsigned hw = (unsigned)(b >> 32), lw = (unsigned)b;
+  const unsigned sign = hw & 0x80000000u;
+  const int f = max((int)((hw >> 20) & 0x7FFu) - (off + 896), 0);  // float exponent field
+  const unsigned hm = __funnelshift_l(lw, hw, 3) & 0x7FFFFFu;
+  const unsigned scale = sign | ((unsigned)(max(f, 53) - 52) << 23);  // 2^-23 ulp units of lo
+  df r;
+  r.hi = __uint_as_float(sign | ((unsigned)f << 23) | hm);
+  r.lo = __fmul_rn(__uint2float_rn(lw & 0x1FFFFFFFu), __uint_as_float(scale));
+  return fx_grid(r, 3.f);
+}
+
+// The derivative matrix in both directions: G for the gradient, T transposed.
+// SYM = -1: even-odd form (the GLL derivative), 0: a caller's general matrix.
+template <int N, int SYM>
+struct FxBasis {
+  FxMat<N, N, SYM> G, T;
+  float K;  // 2 (1 + 2^-20): the factor 2 of the offset, plus a margin for the bound's rounding
+};
+
+// Strides of a cell's work array (cell, i, j; k contiguous) and the lines' owners.  A column
+// is owned by the thread that gathered it; which thread owns which s- or t-line is free, so the
+// lines are dealt to half-warps with different 8-byte banks each (fx_lines), after a small padding
+// where the plain strides leave too few banks.  Shared-memory wavefronts of a batch's work-array
+// accesses, counted on the host, against lines dealt in order over the plain array (and the least
+// possible): n = 4 240 / 624 (240), 5 600 / 900 (600), 6 654 / 1050 (630), 8 512 / 1504 (480),
+// 9 882 / 990 (810).
+template <int N> struct FxStride;
+#define MFGB_FXSTRIDE(NN, CELL, I, J) \
+  template <> struct FxStride<NN> { static constexpr int cell = CELL, i = I, j = J; };
+MFGB_FXSTRIDE(2, 12, 5, 2) MFGB_FXSTRIDE(3, 27, 9, 3) MFGB_FXSTRIDE(4, 68, 17, 4)
+MFGB_FXSTRIDE(5, 153, 29, 5) MFGB_FXSTRIDE(6, 244, 39, 6) MFGB_FXSTRIDE(7, 369, 51, 7)
+MFGB_FXSTRIDE(8, 568, 71, 8) MFGB_FXSTRIDE(9, 738, 82, 9)
+#undef MFGB_FXSTRIDE
+
+// work-array offsets of the s-line (values j apart) and the t-line (contiguous) each thread owns
+template <int N, int E>
+struct FxLines {
+  unsigned short s[E * N * N], t[E * N * N];
+};
+
+// deals the lines a[0..T) over half-warps: each takes lines from the banks (offset mod 16) that
+// have most left, a bank twice only when every other one is used up
+template <int T>
+constexpr void fx_deal(const int (&a)[T], unsigned short (&out)[T]) {
+  bool used[T] = {};
+  int left[16] = {};
+  for (int v : a) ++left[v % 16];
+  for (int h = 0; h < T; h += 16) {
+    bool bank[16] = {};
+    for (int t = h; t < T && t < h + 16; ++t) {
+      int best = -1;
+      for (int b = 0; b < 16; ++b)
+        if (left[b] > 0 && !bank[b] && (best < 0 || left[b] > left[best])) best = b;
+      if (best < 0)
+        for (int b = 0; b < 16; ++b)
+          if (left[b] > 0 && (best < 0 || left[b] > left[best])) best = b;
+      bank[best] = true;
+      --left[best];
+      for (int q = 0; q < T; ++q)
+        if (!used[q] && a[q] % 16 == best) {
+          used[q] = true;
+          out[t] = (unsigned short)a[q];
+          break;
+        }
+    }
+  }
+}
+
+template <int N, int E>
+constexpr FxLines<N, E> fx_lines() {
+  using S = FxStride<N>;
+  FxLines<N, E> r{};
+  int s[E * N * N] = {}, t[E * N * N] = {};
+  for (int q = 0; q < E * N * N; ++q) {
+    const int e = q / (N * N), a = q / N % N, b = q % N;
+    s[q] = e * S::cell + a * S::i + b;
+    t[q] = e * S::cell + a * S::i + b * S::j;
+  }
+  fx_deal(s, r.s);
+  fx_deal(t, r.t);
+  return r;
+}
+template <int N, int E>
+__device__ const FxLines<N, E> fx_line_table = fx_lines<N, E>();
+
+// shared memory of one CTA: G tile, dof-map tile (L-vectors), NB work arrays, two mbarriers
+template <int N, int E, class GT, bool EVEC, int NB>
+struct FxLayout {
+  static constexpr int N3 = N * N * N;
+  static constexpr size_t g_bytes = sizeof(GT) * E * 6 * N3;
+  static constexpr size_t map_bytes = EVEC ? 0 : ((size_t)E * N3 * 4 + 12 + 15) / 16 * 16;
+  static constexpr size_t work_bytes = sizeof(df) * NB * E * FxStride<N>::cell;
+  static constexpr size_t total = g_bytes + map_bytes + (work_bytes + 15) / 16 * 16 + 16;
+};
+
+template <class GT> struct FxGArith;
+template <> struct FxGArith<float2> { using type = ArithDF; };
+template <> struct FxGArith<double> { using type = ArithF64; };
+
+// One CTA works on E cells at a time with N^2 threads per cell.  Per batch:
+//   barrier A   G(b) has landed; u(b) was gathered into registers during batch b-1, its
+//               largest exponent per cell reduced into s_emax by shared atomics
+//   column      thread (j, k) converts its column u(., j, k) to pairs on a common grid, writes
+//               it to shared memory and contracts it: q_r stays in registers
+//   barrier B   map(b+next) is requested (bulk TMA)
+//   lines       thread (a, b) owns the line u(a, ., b), then u(a, b, .): q_s, q_t to shared
+//               memory (NB = 2: q_t over u, after one more barrier)
+//   barrier     thread (j, k) applies the metric to its column: v_r in registers, v_s, v_t over
+//               q_s, q_t
+//   barrier C   G(b+next) is requested, u(b+next) gathered into registers
+//   lines       the transposed contractions of the s- and t-lines, in place
+//   barrier     thread (j, k) contracts v_r and adds the shares of the three directions;
+//               conversion to double and atomic scatter
+// GT = float2: G as scaled pairs with the exponent offset gexp[cell] (operators); double: the
+// caller's FP64 G, whose largest exponent per cell is reduced in shared memory and which the
+// metric converts as it reads it (kernel seams).  EVEC: contiguous element vectors, dst is
+// written, not added to; otherwise through the dof map.  NC interleaved components share one G
+// tile, each with its own exponent per cell (the slots of s_emax alternate with the component).
+// MAPTMA = false loads the dof map with plain loads (a map array that is not 16-byte aligned).
+// EXPIRE (test hook): the first G copy is armed but not issued, and every wait gives up after
+// 1 ms, so the timeout path runs with no copy in flight.
+template <int N, int E, int MB, int NB, class GT, bool EVEC, int NC, int SYM, bool MAPTMA,
+          bool EXPIRE = false>
 __global__ void __launch_bounds__(E * N * N, MB)
-    bk5fx_tma_kernel(const int64_t n_cells, const uint32_t *__restrict__ map,
-                     const float2 *__restrict__ G, const int *__restrict__ gexp,
-                     const double *__restrict__ src, double *__restrict__ dst,
-                     const BasisFX<N> basis, const int *__restrict__ done_flag,
-                     int *__restrict__ err_flag) {
+    bk5fx_kernel(const int64_t n_cells, const uint32_t *__restrict__ map,
+                 const GT *__restrict__ G, const int *__restrict__ gexp,
+                 const double *__restrict__ src, double *__restrict__ dst,
+                 const FxBasis<N, SYM> basis, const int *__restrict__ done_flag,
+                 int *__restrict__ err_flag) {
   if (done_flag != nullptr && *done_flag) return;
-  using L = TmaLayout<N, E, ArithDF>;
+  using L = FxLayout<N, E, GT, EVEC, NB>;
+  using S = FxStride<N>;
   constexpr int N2 = N * N, N3 = N * N * N;
+  constexpr bool G64 = std::is_same<GT, double>::value;
   extern __shared__ __align__(128) unsigned char smem[];
-  float2 *sG = reinterpret_cast<float2 *>(smem);
+  GT *sG = reinterpret_cast<GT *>(smem);
   uint32_t *sMap = reinterpret_cast<uint32_t *>(smem + L::g_bytes);
   df *s_u = reinterpret_cast<df *>(smem + L::g_bytes + L::map_bytes);
-  df *s_vs = s_u + E * N3;
-  df *s_vt = s_vs + E * N3;
-  uint64_t *mbar = reinterpret_cast<uint64_t *>(smem + L::g_bytes + L::map_bytes + L::work_bytes);
+  df *s_s = s_u + E * S::cell;
+  df *s_t = NB == 3 ? s_s + E * S::cell : s_u;
+  uint64_t *mbar = reinterpret_cast<uint64_t *>(smem + L::total - 16);
   uint64_t *mbar_g = mbar, *mbar_m = mbar + 1;
   __shared__ int s_emax[2][E];
+  __shared__ int s_gmax[E];  // G64: largest biased exponent of the cell's G
 
   const int tid = threadIdx.x;
   const int el = tid / N2;
   const int jk = tid - el * N2;
   const int j = jk / N;
   const int k = jk - j * N;
+  const int col = el * S::cell + j * S::j + k;     // own column u(., j, k): + i * S::i
+  const int sline = fx_line_table<N, E>.s[tid];    // own line u(a, ., b) of some cell: + m * S::j
+  const int tline = fx_line_table<N, E>.t[tid];    // own line u(a, b, .) of some cell: + m
   const int64_t n_batches = (n_cells + E - 1) / E;
   int64_t batch = blockIdx.x;
   if (batch >= n_batches) return;  // uniform across the CTA
 
-  // D as (hi, lo) pairs: the rows and columns this thread needs with a runtime
-  // index are read from here at the start of the phase that uses them, so only
-  // one phase's 4N of them are live at a time
-  __shared__ float2 s_D[N * N];
-  for (int t = tid; t < N * N; t += blockDim.x) s_D[t] = make_float2(basis.Dh[t], basis.Dl[t]);
-  const float cgj = basis.cg[j], cgk = basis.cg[k], cij = basis.ci[j], cik = basis.ci[k];
-
-  TmaTiles<N, E, ArithDF> T{n_cells, map, G, src, sG, sMap, mbar_g, mbar_m};
-  T.map_ok = MAPTMA;
+  TmaTiles<N, E, typename FxGArith<GT>::type> T{n_cells, map, G, src, sG, sMap, mbar_g, mbar_m};
+  // the dof-map tile of batch b arrives as the 16-byte aligned window around it, which starts
+  // (b E N^3) mod 4 entries before the tile; the last one by plain loads when its window would
+  // pass the map's end
+  auto map_window = [&](int64_t b) -> uint32_t {  // bytes, 0: no bulk copy
+    const int64_t first = b * E * N3, last = first + (int64_t)T.cells_of(b) * N3;
+    const int64_t end = (last + 3) & ~(int64_t)3;
+    return MAPTMA && end <= n_cells * N3 ? (uint32_t)(end - (first & ~(int64_t)3)) * 4u : 0u;
+  };
+  auto issue_map = [&](int64_t b) {
+    const uint32_t bytes = map_window(b);
+    mbar_arrive_expect_tx(mbar_m, bytes);
+    if (bytes) bulk_g2s(sMap, map + ((b * E * N3) & ~(int64_t)3), bytes, mbar_m);
+  };
   constexpr uint64_t wlim = EXPIRE ? 1000000ull : MFGB_WAIT_LIMIT_NS;
   auto fail = [&](uint32_t pg, uint32_t pm) {
     if (tid == 0 && err_flag) atomicOr(err_flag, 1);
     mbar_wait(mbar_g, pg, wlim);  // bounded waits for copies still in flight
-    mbar_wait(mbar_m, pm, wlim);
+    if (!EVEC) mbar_wait(mbar_m, pm, wlim);
   };
 
   if (tid < 2 * E) (&s_emax[0][0])[tid] = 0;
+  if (G64 && tid < E) s_gmax[tid] = 0;
   if (tid == 0) {
     mbar_init(mbar_g, 1);
     mbar_init(mbar_m, 1);
@@ -224,234 +312,7 @@ __global__ void __launch_bounds__(E * N * N, MB)
       mbar_arrive_expect_tx(mbar_g, 16u);
     else
       T.issue_g(batch);
-    T.issue_map(batch);
-  }
-  uint32_t ph_g = 0, ph_m = 0;
-  uint32_t idx[N];
-  double raw[N];
-  int ge = 0;  // G exponent offset of this thread's cell in the prefetched batch
-  // gathered column -> its largest exponent into the cell's slot
-  auto reduce_exp = [&](int slot) {
-    int em = 0;
-#pragma unroll
-    for (int i = 0; i < N; ++i) em = max(em, idx[i] != MFGB_INVALID_DOF ? dexp(raw[i]) : 0);
-    if (em) atomicMax(&s_emax[slot][el], em);
-  };
-  {
-    const bool ok = mbar_wait(mbar_m, ph_m, wlim);
-    if (__syncthreads_or(!ok)) { fail(ph_g, ph_m); return; }
-    ph_m ^= 1u;
-    T.gather(batch, el, jk, idx, raw);
-    reduce_exp(0);
-    if (el < T.cells_of(batch)) ge = __ldg(gexp + batch * E + el);
-  }
-
-  for (int it = 0; batch < n_batches; batch += gridDim.x, ++it) {
-    const int slot = it & 1;
-    const int64_t next = batch + gridDim.x;
-    const bool has_next = next < n_batches;
-    const bool okg = mbar_wait(mbar_g, ph_g, wlim);
-    if (__syncthreads_or(!okg)) { fail(ph_g, ph_m); return; }  // barrier A
-    ph_g ^= 1u;
-    T.load_g_plain(batch, tid, blockDim.x);  // ordered before the metric phase by barrier B
-    const int su = fx_offset(s_emax[slot][el]);
-    const int sc = su + ge;  // the cell's result scale
-    const bool fast_out = (unsigned)(sc + 896) <= 1792u;
-    const unsigned kout = (unsigned)(896 + sc) << 20;
-    df u[N];
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-      u[i] = idx[i] != MFGB_INVALID_DOF ? fx_from_double(raw[i], su) : df{0.f, 0.f};
-      s_u[el * N3 + i * N2 + jk] = u[i];
-    }
-    __syncthreads();  // barrier B: s_u ready, s_emax[slot] read; the map tile is free
-    if (jk == 0) s_emax[slot][el] = 0;  // next written after barrier C of the next batch
-    if (tid == 0 && has_next) {
-      fence_proxy_async_smem();
-      T.issue_map(next);
-    }
-
-    const bool valid = el < T.cells_of(batch);
-    float Djh[N], Djl[N], Dkh[N], Dkl[N];
-#pragma unroll
-    for (int m = 0; m < N; ++m) {
-      const float2 a = lds_pair(s_D + j * N + m), b = lds_pair(s_D + k * N + m);
-      Djh[m] = a.x, Djl[m] = a.y, Dkh[m] = b.x, Dkl[m] = b.y;
-    }
-    df vr[N];
-    const float2 *Gc = sG + el * 6 * N3 + jk;
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-      // ---- gradient: q_r = D[i][.] u(., j, k), q_s = D[j][.] u(i, ., k), q_t = D[k][.] u(i, j, .)
-      fxacc ar, as, at;
-      const float cr = basis.cg[i];
-      fx_first(ar, basis.Dh[i * N], basis.Dl[i * N], u[0].hi, u[0].lo, cr);
-      {
-        const df a = s_u[el * N3 + i * N2 + k], b = s_u[el * N3 + i * N2 + j * N];
-        fx_first(as, Djh[0], Djl[0], a.hi, a.lo, cgj);
-        fx_first(at, Dkh[0], Dkl[0], b.hi, b.lo, cgk);
-      }
-#pragma unroll
-      for (int m = 1; m < N; ++m) {
-        fx_fma(ar, basis.Dh[i * N + m], basis.Dl[i * N + m], u[m].hi, u[m].lo);
-        const df a = s_u[el * N3 + i * N2 + m * N + k], b = s_u[el * N3 + i * N2 + j * N + m];
-        fx_fma(as, Djh[m], Djl[m], a.hi, a.lo);
-        fx_fma(at, Dkh[m], Dkl[m], b.hi, b.lo);
-      }
-      const df qr = fx_finish(ar, cr), qs = fx_finish(as, cgj), qt = fx_finish(at, cgk);
-      // ---- metric, bound per point: max |q| times the row sums of |G|
-      float2 grr = make_float2(0.f, 0.f), grs = grr, grt = grr, gss = grr, gst = grr, gtt = grr;
-      if (valid) {
-        grr = Gc[0 * N3 + i * N2];
-        grs = Gc[1 * N3 + i * N2];
-        grt = Gc[2 * N3 + i * N2];
-        gss = Gc[3 * N3 + i * N2];
-        gst = Gc[4 * N3 + i * N2];
-        gtt = Gc[5 * N3 + i * N2];
-      }
-      const float kq = basis.K * fmaxf(fmaxf(fabsf(qr.hi), fabsf(qs.hi)), fabsf(qt.hi));
-      const float Cr = (fabsf(grr.x) + fabsf(grs.x) + fabsf(grt.x)) * kq;
-      const float Cs = (fabsf(grs.x) + fabsf(gss.x) + fabsf(gst.x)) * kq;
-      const float Ct = (fabsf(grt.x) + fabsf(gst.x) + fabsf(gtt.x)) * kq;
-      fxacc br, bs, bt;
-      fx_first(br, grr.x, grr.y, qr.hi, qr.lo, Cr);
-      fx_fma(br, grs.x, grs.y, qs.hi, qs.lo);
-      fx_fma(br, grt.x, grt.y, qt.hi, qt.lo);
-      fx_first(bs, grs.x, grs.y, qr.hi, qr.lo, Cs);
-      fx_fma(bs, gss.x, gss.y, qs.hi, qs.lo);
-      fx_fma(bs, gst.x, gst.y, qt.hi, qt.lo);
-      fx_first(bt, grt.x, grt.y, qr.hi, qr.lo, Ct);
-      fx_fma(bt, gst.x, gst.y, qs.hi, qs.lo);
-      fx_fma(bt, gtt.x, gtt.y, qt.hi, qt.lo);
-      vr[i] = fx_finish(br, Cr);
-      s_vs[el * N3 + i * N2 + jk] = fx_finish(bs, Cs);
-      s_vt[el * N3 + i * N2 + jk] = fx_finish(bt, Ct);
-    }
-    __syncthreads();  // barrier C: G tile consumed, s_vs / s_vt ready
-    if (tid == 0 && has_next) {
-      fence_proxy_async_smem();
-      T.issue_g(next);
-    }
-
-    // this batch's scatter targets; then prefetch the next batch's gather
-    uint32_t cur[N];
-#pragma unroll
-    for (int i = 0; i < N; ++i) cur[i] = idx[i];
-    if (has_next) {
-      const bool okm = mbar_wait(mbar_m, ph_m, wlim);
-      if (!okm && err_flag) atomicOr(err_flag, 1);  // the launch's result is void
-      ph_m ^= 1u;
-      if (okm) {
-        T.gather(next, el, jk, idx, raw);
-      } else {
-#pragma unroll
-        for (int i = 0; i < N; ++i) { idx[i] = MFGB_INVALID_DOF; raw[i] = 0.0; }
-      }
-      ge = el < T.cells_of(next) ? __ldg(gexp + next * E + el) : 0;
-    }
-
-    // ---- transpose: y = sum_m D[m][i] v_r(m,j,k) + D[m][j] v_s(i,m,k) + D[m][k] v_t(i,j,m);
-    // the bound of output i: max |v_r| of the own column and the maxima of the
-    // s- and t-lines it reads
-    float Dtjh[N], Dtjl[N], Dtkh[N], Dtkl[N];
-#pragma unroll
-    for (int m = 0; m < N; ++m) {
-      const float2 a = lds_pair(s_D + m * N + j), b = lds_pair(s_D + m * N + k);
-      Dtjh[m] = a.x, Dtjl[m] = a.y, Dtkh[m] = b.x, Dtkl[m] = b.y;
-    }
-    float mr = 0.f;
-#pragma unroll
-    for (int m = 0; m < N; ++m) mr = fmaxf(mr, fabsf(vr[m].hi));
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-      df ls[N], lt[N];
-      float ms = 0.f, mt = 0.f;
-#pragma unroll
-      for (int m = 0; m < N; ++m) {
-        ls[m] = s_vs[el * N3 + i * N2 + m * N + k];
-        lt[m] = s_vt[el * N3 + i * N2 + j * N + m];
-        ms = fmaxf(ms, fabsf(ls[m].hi));
-        mt = fmaxf(mt, fabsf(lt[m].hi));
-      }
-      const float C = __fmaf_rn(mt, cik, __fmaf_rn(ms, cij, mr * basis.ci[i]));
-      fxacc a;
-      fx_first(a, basis.Dh[i], basis.Dl[i], vr[0].hi, vr[0].lo, C);
-      fx_fma(a, Dtjh[0], Dtjl[0], ls[0].hi, ls[0].lo);
-      fx_fma(a, Dtkh[0], Dtkl[0], lt[0].hi, lt[0].lo);
-#pragma unroll
-      for (int m = 1; m < N; ++m) {
-        fx_fma(a, basis.Dh[m * N + i], basis.Dl[m * N + i], vr[m].hi, vr[m].lo);
-        fx_fma(a, Dtjh[m], Dtjl[m], ls[m].hi, ls[m].lo);
-        fx_fma(a, Dtkh[m], Dtkl[m], lt[m].hi, lt[m].lo);
-      }
-      const df y = fx_finish(a, C);
-      if (cur[i] != MFGB_INVALID_DOF)
-        atomicAdd(dst + cur[i], fast_out ? fx_f2d_fast(y.hi, kout) + fx_f2d_fast(y.lo, kout)
-                                         : fx_f2d(y.hi, sc) + fx_f2d(y.lo, sc));
-    }
-    // the prefetched gather's largest exponent per cell, once its loads have
-    // landed (read after the next barrier A)
-    if (has_next) reduce_exp(slot ^ 1);
-  }
-}
-
-
-// BK6 (NC interleaved components per node sharing one G tile) with the offset
-// accumulation and per-cell scaling of the kernel above: per batch the scaled
-// G pairs arrive once, and the components run one after another, each with its
-// own exponent offset per cell (reduced while the previous component
-// integrates, read after one extra barrier).  The next component's gather is
-// prefetched during the current component's transpose, the next batch's first
-// component during the last one.
-template <int N, int E, int MB, bool MAPTMA, int NC>
-__global__ void __launch_bounds__(E * N * N, MB)
-    bk6fx_tma_kernel(const int64_t n_cells, const uint32_t *__restrict__ map,
-                     const float2 *__restrict__ G, const int *__restrict__ gexp,
-                     const double *__restrict__ src, double *__restrict__ dst,
-                     const BasisFX<N> basis, int *__restrict__ err_flag) {
-  using L = TmaLayout<N, E, ArithDF>;
-  constexpr int N2 = N * N, N3 = N * N * N;
-  extern __shared__ __align__(128) unsigned char smem[];
-  float2 *sG = reinterpret_cast<float2 *>(smem);
-  uint32_t *sMap = reinterpret_cast<uint32_t *>(smem + L::g_bytes);
-  df *s_u = reinterpret_cast<df *>(smem + L::g_bytes + L::map_bytes);
-  df *s_vs = s_u + E * N3;
-  df *s_vt = s_vs + E * N3;
-  uint64_t *mbar = reinterpret_cast<uint64_t *>(smem + L::g_bytes + L::map_bytes + L::work_bytes);
-  uint64_t *mbar_g = mbar, *mbar_m = mbar + 1;
-  __shared__ int s_emax[2][E];
-
-  const int tid = threadIdx.x;
-  const int el = tid / N2;
-  const int jk = tid - el * N2;
-  const int j = jk / N;
-  const int k = jk - j * N;
-  const int64_t n_batches = (n_cells + E - 1) / E;
-  int64_t batch = blockIdx.x;
-  if (batch >= n_batches) return;  // uniform across the CTA
-
-  __shared__ float2 s_D[N * N];
-  for (int t = tid; t < N * N; t += blockDim.x) s_D[t] = make_float2(basis.Dh[t], basis.Dl[t]);
-  const float cgj = basis.cg[j], cgk = basis.cg[k], cij = basis.ci[j], cik = basis.ci[k];
-
-  TmaTiles<N, E, ArithDF> T{n_cells, map, G, src, sG, sMap, mbar_g, mbar_m};
-  T.map_ok = MAPTMA;
-  auto fail = [&](uint32_t pg, uint32_t pm) {
-    if (tid == 0 && err_flag) atomicOr(err_flag, 1);
-    mbar_wait(mbar_g, pg);  // bounded waits for copies still in flight
-    mbar_wait(mbar_m, pm);
-  };
-
-  if (tid < 2 * E) (&s_emax[0][0])[tid] = 0;
-  if (tid == 0) {
-    mbar_init(mbar_g, 1);
-    mbar_init(mbar_m, 1);
-    fence_mbar_init();
-  }
-  __syncthreads();
-  if (tid == 0) {
-    T.issue_g(batch);
-    T.issue_map(batch);
+    if (!EVEC) issue_map(batch);
   }
   uint32_t ph_g = 0, ph_m = 0;
   uint32_t idx[N];
@@ -459,644 +320,217 @@ __global__ void __launch_bounds__(E * N * N, MB)
   int ge = 0;  // G exponent offset of this thread's cell in the prefetched batch
   // dof indices of column (el, jk) of batch b, from the map tile or global
   auto indices = [&](int64_t b) {
-    const int cells = T.cells_of(b);
-    const bool ok = el < cells;
-    const bool mt = T.map_by_tma(cells);
+    const bool ok = el < T.cells_of(b);
+    if (map_window(b)) {
+      const uint32_t *m = sMap + ((b * E * N3) & 3) + el * N3 + jk;
 #pragma unroll
-    for (int i = 0; i < N; ++i)
-      idx[i] = ok ? (mt ? sMap[el * N3 + i * N2 + jk] : __ldg(map + (b * E + el) * N3 + i * N2 + jk))
-                  : MFGB_INVALID_DOF;
-  };
-  auto gather = [&](int c) {
+      for (int i = 0; i < N; ++i) idx[i] = ok ? m[i * N2] : MFGB_INVALID_DOF;
+    } else {
+      const uint32_t *m = map + (b * E + el) * N3 + jk;
 #pragma unroll
-    for (int i = 0; i < N; ++i)
-      raw[i] = idx[i] != MFGB_INVALID_DOF ? __ldg(src + (size_t)NC * idx[i] + c) : 0.0;
+      for (int i = 0; i < N; ++i) idx[i] = ok ? __ldg(m + i * N2) : MFGB_INVALID_DOF;
+    }
   };
+  // component c of the column's values (EVEC: of batch b), and the cell's G exponent
+  auto gather = [&](int64_t b, int c) {
+    if constexpr (EVEC) {
+      const bool ok = el < T.cells_of(b);
+#pragma unroll
+      for (int i = 0; i < N; ++i)
+        raw[i] = ok ? __ldg(src + (b * E + el) * N3 + i * N2 + jk) : 0.0;
+    } else {
+#pragma unroll
+      for (int i = 0; i < N; ++i)
+        raw[i] = idx[i] != MFGB_INVALID_DOF ? __ldg(src + (size_t)NC * idx[i] + c) : 0.0;
+    }
+  };
+  // gathered column -> its largest exponent into the cell's slot
   auto reduce_exp = [&](int slot) {
-    int em = 0;
+    unsigned em = 0;
 #pragma unroll
-    for (int i = 0; i < N; ++i) em = max(em, idx[i] != MFGB_INVALID_DOF ? dexp(raw[i]) : 0);
-    if (em) atomicMax(&s_emax[slot][el], em);
+    for (int i = 0; i < N; ++i)
+      em = max(em, (unsigned)(__double_as_longlong(raw[i]) >> 32) & 0x7FFFFFFFu);
+    if (em >> 20) atomicMax(&s_emax[slot][el], (int)(em >> 20));
   };
   {
-    const bool ok = mbar_wait(mbar_m, ph_m);
-    if (__syncthreads_or(!ok)) { fail(ph_g, ph_m); return; }
-    ph_m ^= 1u;
-    indices(batch);
-    gather(0);
+    if constexpr (!EVEC) {
+      const bool ok = mbar_wait(mbar_m, ph_m, wlim);
+      if (__syncthreads_or(!ok)) { fail(ph_g, ph_m); return; }
+      ph_m ^= 1u;
+      indices(batch);
+    }
+    gather(batch, 0);
     reduce_exp(0);
-    if (el < T.cells_of(batch)) ge = __ldg(gexp + batch * E + el);
+    if (!G64 && el < T.cells_of(batch)) ge = __ldg(gexp + batch * E + el);
   }
 
   int cnt = 0;  // components run so far: the exponent slot alternates with it
   for (; batch < n_batches; batch += gridDim.x) {
     const int64_t next = batch + gridDim.x;
     const bool has_next = next < n_batches;
-    const bool okg = mbar_wait(mbar_g, ph_g);
+    const bool okg = mbar_wait(mbar_g, ph_g, wlim);
     if (__syncthreads_or(!okg)) { fail(ph_g, ph_m); return; }  // barrier A
     ph_g ^= 1u;
-    T.load_g_plain(batch, tid, blockDim.x);  // ordered before the metric phase by barrier B
+    T.load_g_plain(batch, tid, blockDim.x);  // ordered before the metric by barrier B
     const bool valid = el < T.cells_of(batch);
-    const float2 *Gc = sG + el * 6 * N3 + jk;
-    const int ge_batch = ge;
+    const GT *Gc = sG + el * 6 * N3 + jk;
+    if constexpr (G64) {  // the cell's largest G exponent (read after barrier B)
+      if (valid) {
+        int eg = 0;
+#pragma unroll 1
+        for (int c = 0; c < 6; ++c)
+#pragma unroll
+          for (int i = 0; i < N; ++i) eg = max(eg, dexp(Gc[c * N3 + i * N2]));
+        if (eg) atomicMax(&s_gmax[el], eg);
+      }
+    }
+    int sg = ge;  // G64: set after barrier B
 #pragma unroll 1
     for (int c = 0; c < NC; ++c, ++cnt) {
       const int slot = cnt & 1;
-      if (c > 0) __syncthreads();  // this component's exponents are in; s_u is free
-      const int su = fx_offset(s_emax[slot][el]);
-      const int sc = su + ge_batch;  // the cell's result scale for this component
-      const bool fast_out = (unsigned)(sc + 896) <= 1792u;
-      const unsigned kout = (unsigned)(896 + sc) << 20;
-      df u[N];
+      if (NC > 1 && c > 0) __syncthreads();  // this component's exponents are in; work arrays free
+      const int emax = s_emax[slot][el];
+      const int su = fx_offset(emax);
+      df x[N], qr[N];
+      if ((unsigned)(emax - 1) < 0x7FEu) {
 #pragma unroll
-      for (int i = 0; i < N; ++i) {
-        u[i] = idx[i] != MFGB_INVALID_DOF ? fx_from_double(raw[i], su) : df{0.f, 0.f};
-        s_u[el * N3 + i * N2 + jk] = u[i];
+        for (int i = 0; i < N; ++i) x[i] = fx_from_double_grid(raw[i], su);
+      } else {  // all zero or subnormal, or an inf or NaN among the values
+#pragma unroll
+        for (int i = 0; i < N; ++i) x[i] = fx_grid(fx_from_double(raw[i], su), 3.f);
       }
+#pragma unroll
+      for (int i = 0; i < N; ++i) s_u[col + i * S::i] = x[i];
+      fx_line_grid(basis.G, x, 1.f, qr);
       __syncthreads();  // barrier B: s_u ready, s_emax[slot] read (c = 0: the map tile is free)
       if (jk == 0) s_emax[slot][el] = 0;  // next written two components on
-      if (c == 0 && tid == 0 && has_next) {
+      if constexpr (G64)
+        if (c == 0) sg = fx_offset(s_gmax[el]);
+      if (!EVEC && c == 0 && tid == 0 && has_next) {
         fence_proxy_async_smem();
-        T.issue_map(next);
+        issue_map(next);
       }
-      float Djh[N], Djl[N], Dkh[N], Dkl[N];
+      // ---- gradient along the s- and t-lines
+      {
+        df y[N];
 #pragma unroll
-      for (int m = 0; m < N; ++m) {
-        const float2 a = lds_pair(s_D + j * N + m), b = lds_pair(s_D + k * N + m);
-        Djh[m] = a.x, Djl[m] = a.y, Dkh[m] = b.x, Dkl[m] = b.y;
+        for (int m = 0; m < N; ++m) x[m] = s_u[sline + m * S::j];
+        fx_line_grid(basis.G, x, 1.f, y);
+#pragma unroll
+        for (int m = 0; m < N; ++m) s_s[sline + m * S::j] = y[m];
+#pragma unroll
+        for (int m = 0; m < N; ++m) x[m] = s_u[tline + m];
+        fx_line_grid(basis.G, x, 1.f, y);
+        if (NB == 2) __syncthreads();  // every s-line has been read
+#pragma unroll
+        for (int m = 0; m < N; ++m) s_t[tline + m] = y[m];
       }
+      __syncthreads();
+      // ---- metric, bound per point: max |q| times the row sums of |G|
       df vr[N];
 #pragma unroll
       for (int i = 0; i < N; ++i) {
-        fxacc ar, as, at;
-        const float cr = basis.cg[i];
-        fx_first(ar, basis.Dh[i * N], basis.Dl[i * N], u[0].hi, u[0].lo, cr);
-        {
-          const df a = s_u[el * N3 + i * N2 + k], b = s_u[el * N3 + i * N2 + j * N];
-          fx_first(as, Djh[0], Djl[0], a.hi, a.lo, cgj);
-          fx_first(at, Dkh[0], Dkl[0], b.hi, b.lo, cgk);
-        }
-#pragma unroll
-        for (int m = 1; m < N; ++m) {
-          fx_fma(ar, basis.Dh[i * N + m], basis.Dl[i * N + m], u[m].hi, u[m].lo);
-          const df a = s_u[el * N3 + i * N2 + m * N + k], b = s_u[el * N3 + i * N2 + j * N + m];
-          fx_fma(as, Djh[m], Djl[m], a.hi, a.lo);
-          fx_fma(at, Dkh[m], Dkl[m], b.hi, b.lo);
-        }
-        const df qr = fx_finish(ar, cr), qs = fx_finish(as, cgj), qt = fx_finish(at, cgk);
-        float2 grr = make_float2(0.f, 0.f), grs = grr, grt = grr, gss = grr, gst = grr, gtt = grr;
-        if (valid) {
-          grr = Gc[0 * N3 + i * N2];
-          grs = Gc[1 * N3 + i * N2];
-          grt = Gc[2 * N3 + i * N2];
-          gss = Gc[3 * N3 + i * N2];
-          gst = Gc[4 * N3 + i * N2];
-          gtt = Gc[5 * N3 + i * N2];
-        }
-        const float kq = basis.K * fmaxf(fmaxf(fabsf(qr.hi), fabsf(qs.hi)), fabsf(qt.hi));
+        const df qs = s_s[col + i * S::i], qt = s_t[col + i * S::i];
+        auto g = [&](int q) {  // (a cell past the end reads a stale tile; nothing leaves it)
+          if constexpr (G64) {  // converted to pairs scaled by 2^-sg as it is read
+            const df d = fx_from_double(Gc[q * N3 + i * N2], sg);
+            return make_float2(d.hi, d.lo);
+          } else {
+            return Gc[q * N3 + i * N2];
+          }
+        };
+        const float2 grr = g(0), grs = g(1), grt = g(2), gss = g(3), gst = g(4), gtt = g(5);
+        const float kq = basis.K * fmaxf(fmaxf(fabsf(qr[i].hi), fabsf(qs.hi)), fabsf(qt.hi));
         const float Cr = (fabsf(grr.x) + fabsf(grs.x) + fabsf(grt.x)) * kq;
         const float Cs = (fabsf(grs.x) + fabsf(gss.x) + fabsf(gst.x)) * kq;
         const float Ct = (fabsf(grt.x) + fabsf(gst.x) + fabsf(gtt.x)) * kq;
         fxacc br, bs, bt;
-        fx_first(br, grr.x, grr.y, qr.hi, qr.lo, Cr);
+        fx_first(br, grr.x, grr.y, qr[i].hi, qr[i].lo, Cr);
         fx_fma(br, grs.x, grs.y, qs.hi, qs.lo);
         fx_fma(br, grt.x, grt.y, qt.hi, qt.lo);
-        fx_first(bs, grs.x, grs.y, qr.hi, qr.lo, Cs);
+        fx_first(bs, grs.x, grs.y, qr[i].hi, qr[i].lo, Cs);
         fx_fma(bs, gss.x, gss.y, qs.hi, qs.lo);
         fx_fma(bs, gst.x, gst.y, qt.hi, qt.lo);
-        fx_first(bt, grt.x, grt.y, qr.hi, qr.lo, Ct);
+        fx_first(bt, grt.x, grt.y, qr[i].hi, qr[i].lo, Ct);
         fx_fma(bt, gst.x, gst.y, qs.hi, qs.lo);
         fx_fma(bt, gtt.x, gtt.y, qt.hi, qt.lo);
         vr[i] = fx_finish(br, Cr);
-        s_vs[el * N3 + i * N2 + jk] = fx_finish(bs, Cs);
-        s_vt[el * N3 + i * N2 + jk] = fx_finish(bt, Ct);
+        s_s[col + i * S::i] = fx_finish(bs, Cs);
+        s_t[col + i * S::i] = fx_finish(bt, Ct);
       }
-      __syncthreads();  // barrier C: s_vs / s_vt ready (last component: G tile consumed)
-      if (c == NC - 1 && tid == 0 && has_next) {
-        fence_proxy_async_smem();
-        T.issue_g(next);
+      __syncthreads();  // barrier C: v_s, v_t ready (last component: G tile consumed)
+      if (c == NC - 1) {
+        if (G64 && jk == 0) s_gmax[el] = 0;
+        if (tid == 0 && has_next) {
+          fence_proxy_async_smem();
+          T.issue_g(next);
+        }
       }
       // this component's scatter targets; then prefetch the next component
       // (the next batch's first one after the last)
+      const int64_t out_cell = batch * E + el;
+      const int sc = su + sg;  // the cell's result scale
       uint32_t cur[N];
 #pragma unroll
-      for (int i = 0; i < N; ++i) cur[i] = idx[i];
+      for (int i = 0; i < N; ++i) cur[i] = EVEC ? 0u : idx[i];
       if (c + 1 < NC) {
-        gather(c + 1);
+        gather(batch, c + 1);
       } else if (has_next) {
-        const bool okm = mbar_wait(mbar_m, ph_m);
-        if (!okm && err_flag) atomicOr(err_flag, 1);  // the launch's result is void
-        ph_m ^= 1u;
-        if (okm) {
-          indices(next);
-          gather(0);
-        } else {
+        if constexpr (!EVEC) {
+          const bool okm = mbar_wait(mbar_m, ph_m, wlim);
+          if (!okm && err_flag) atomicOr(err_flag, 1);  // the launch's result is void
+          ph_m ^= 1u;
+          if (okm) {
+            indices(next);
+          } else {
 #pragma unroll
-          for (int i = 0; i < N; ++i) { idx[i] = MFGB_INVALID_DOF; raw[i] = 0.0; }
+            for (int i = 0; i < N; ++i) idx[i] = MFGB_INVALID_DOF;
+          }
         }
-        ge = el < T.cells_of(next) ? __ldg(gexp + next * E + el) : 0;
+        gather(next, 0);
+        if (!G64) ge = el < T.cells_of(next) ? __ldg(gexp + next * E + el) : 0;
       }
-      float Dtjh[N], Dtjl[N], Dtkh[N], Dtkl[N];
-#pragma unroll
-      for (int m = 0; m < N; ++m) {
-        const float2 a = lds_pair(s_D + m * N + j), b = lds_pair(s_D + m * N + k);
-        Dtjh[m] = a.x, Dtjl[m] = a.y, Dtkh[m] = b.x, Dtkl[m] = b.y;
-      }
-      float mr = 0.f;
-#pragma unroll
-      for (int m = 0; m < N; ++m) mr = fmaxf(mr, fabsf(vr[m].hi));
-#pragma unroll
-      for (int i = 0; i < N; ++i) {
-        df ls[N], lt[N];
-        float ms = 0.f, mt = 0.f;
-#pragma unroll
-        for (int m = 0; m < N; ++m) {
-          ls[m] = s_vs[el * N3 + i * N2 + m * N + k];
-          lt[m] = s_vt[el * N3 + i * N2 + j * N + m];
-          ms = fmaxf(ms, fabsf(ls[m].hi));
-          mt = fmaxf(mt, fabsf(lt[m].hi));
-        }
-        const float C = __fmaf_rn(mt, cik, __fmaf_rn(ms, cij, mr * basis.ci[i]));
-        fxacc a;
-        fx_first(a, basis.Dh[i], basis.Dl[i], vr[0].hi, vr[0].lo, C);
-        fx_fma(a, Dtjh[0], Dtjl[0], ls[0].hi, ls[0].lo);
-        fx_fma(a, Dtkh[0], Dtkl[0], lt[0].hi, lt[0].lo);
-#pragma unroll
-        for (int m = 1; m < N; ++m) {
-          fx_fma(a, basis.Dh[m * N + i], basis.Dl[m * N + i], vr[m].hi, vr[m].lo);
-          fx_fma(a, Dtjh[m], Dtjl[m], ls[m].hi, ls[m].lo);
-          fx_fma(a, Dtkh[m], Dtkl[m], lt[m].hi, lt[m].lo);
-        }
-        const df y = fx_finish(a, C);
-        if (cur[i] != MFGB_INVALID_DOF)
-          atomicAdd(dst + (size_t)NC * cur[i] + c,
-                    fast_out ? fx_f2d_fast(y.hi, kout) + fx_f2d_fast(y.lo, kout)
-                             : fx_f2d(y.hi, sc) + fx_f2d(y.lo, sc));
-      }
-      // the prefetched component's largest exponent per cell (read after the
-      // next component's first barrier, or the next batch's barrier A)
-      if (c + 1 < NC || has_next) reduce_exp(slot ^ 1);
-    }
-  }
-}
-
-// The same kernel on the caller's FP64 G (the BK5 L-vector seam, deal.II's
-// MatrixFree kernel, bakeoff_problems_dealii/include/bk3_kokkos_kernel.h):
-// G[cell][6][n^3] arrives by bulk copies, each cell's largest G exponent is
-// reduced in shared memory and the metric converts G to pairs scaled by it as
-// it reads them.  Any input range is carried.
-template <int N, int E, int MB, bool MAPTMA>
-__global__ void __launch_bounds__(E * N * N, MB)
-    bk5fx_g64_kernel(const int64_t n_cells, const uint32_t *__restrict__ map,
-                     const double *__restrict__ G, const double *__restrict__ src,
-                     double *__restrict__ dst, const BasisFX<N> basis,
-                     int *__restrict__ err_flag) {
-  using L = TmaLayout<N, E, ArithF64>;
-  constexpr int N2 = N * N, N3 = N * N * N;
-  extern __shared__ __align__(128) unsigned char smem[];
-  double *sG = reinterpret_cast<double *>(smem);
-  uint32_t *sMap = reinterpret_cast<uint32_t *>(smem + L::g_bytes);
-  df *s_u = reinterpret_cast<df *>(smem + L::g_bytes + L::map_bytes);
-  df *s_vs = s_u + E * N3;
-  df *s_vt = s_vs + E * N3;
-  uint64_t *mbar = reinterpret_cast<uint64_t *>(smem + L::g_bytes + L::map_bytes + L::work_bytes);
-  uint64_t *mbar_g = mbar, *mbar_m = mbar + 1;
-  __shared__ int s_emax[2][E];
-  __shared__ int s_gmax[E];  // largest biased exponent of the cell's G
-
-  const int tid = threadIdx.x;
-  const int el = tid / N2;
-  const int jk = tid - el * N2;
-  const int j = jk / N;
-  const int k = jk - j * N;
-  const int64_t n_batches = (n_cells + E - 1) / E;
-  int64_t batch = blockIdx.x;
-  if (batch >= n_batches) return;  // uniform across the CTA
-
-  // D as (hi, lo) pairs: the rows and columns this thread needs with a runtime
-  // index are read from here at the start of the phase that uses them, so only
-  // one phase's 4N of them are live at a time
-  __shared__ float2 s_D[N * N];
-  for (int t = tid; t < N * N; t += blockDim.x) s_D[t] = make_float2(basis.Dh[t], basis.Dl[t]);
-  const float cgj = basis.cg[j], cgk = basis.cg[k], cij = basis.ci[j], cik = basis.ci[k];
-
-  TmaTiles<N, E, ArithF64> T{n_cells, map, G, src, sG, sMap, mbar_g, mbar_m};
-  T.map_ok = MAPTMA;
-  constexpr uint64_t wlim = MFGB_WAIT_LIMIT_NS;
-  auto fail = [&](uint32_t pg, uint32_t pm) {
-    if (tid == 0 && err_flag) atomicOr(err_flag, 1);
-    mbar_wait(mbar_g, pg, wlim);  // bounded waits for copies still in flight
-    mbar_wait(mbar_m, pm, wlim);
-  };
-
-  if (tid < 2 * E) (&s_emax[0][0])[tid] = 0;
-  if (tid < E) s_gmax[tid] = 0;
-  if (tid == 0) {
-    mbar_init(mbar_g, 1);
-    mbar_init(mbar_m, 1);
-    fence_mbar_init();
-  }
-  __syncthreads();
-  if (tid == 0) {
-    T.issue_g(batch);
-    T.issue_map(batch);
-  }
-  uint32_t ph_g = 0, ph_m = 0;
-  uint32_t idx[N];
-  double raw[N];
-  // gathered column -> its largest exponent into the cell's slot
-  auto reduce_exp = [&](int slot) {
-    int em = 0;
-#pragma unroll
-    for (int i = 0; i < N; ++i) em = max(em, idx[i] != MFGB_INVALID_DOF ? dexp(raw[i]) : 0);
-    if (em) atomicMax(&s_emax[slot][el], em);
-  };
-  {
-    const bool ok = mbar_wait(mbar_m, ph_m, wlim);
-    if (__syncthreads_or(!ok)) { fail(ph_g, ph_m); return; }
-    ph_m ^= 1u;
-    T.gather(batch, el, jk, idx, raw);
-    reduce_exp(0);
-  }
-
-  for (int it = 0; batch < n_batches; batch += gridDim.x, ++it) {
-    const int slot = it & 1;
-    const int64_t next = batch + gridDim.x;
-    const bool has_next = next < n_batches;
-    const bool okg = mbar_wait(mbar_g, ph_g, wlim);
-    if (__syncthreads_or(!okg)) { fail(ph_g, ph_m); return; }  // barrier A
-    ph_g ^= 1u;
-    T.load_g_plain(batch, tid, blockDim.x);  // ordered before the metric phase by barrier B
-    const double *Gd = sG + el * 6 * N3 + jk;
-    if (el < T.cells_of(batch)) {  // the cell's largest G exponent (read after barrier B)
-      int eg = 0;
-#pragma unroll 1
-      for (int c = 0; c < 6; ++c)
-#pragma unroll
-        for (int i = 0; i < N; ++i) eg = max(eg, dexp(Gd[c * N3 + i * N2]));
-      if (eg) atomicMax(&s_gmax[el], eg);
-    }
-    const int su = fx_offset(s_emax[slot][el]);
-    df u[N];
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-      u[i] = idx[i] != MFGB_INVALID_DOF ? fx_from_double(raw[i], su) : df{0.f, 0.f};
-      s_u[el * N3 + i * N2 + jk] = u[i];
-    }
-    __syncthreads();  // barrier B: s_u and s_gmax ready, s_emax[slot] read; the map tile is free
-    if (jk == 0) s_emax[slot][el] = 0;  // next written after barrier C of the next batch
-    const int sg = fx_offset(s_gmax[el]);
-    const int sc = su + sg;  // the cell's result scale
-    const bool fast_out = (unsigned)(sc + 896) <= 1792u;
-    const unsigned kout = (unsigned)(896 + sc) << 20;
-    if (tid == 0 && has_next) {
-      fence_proxy_async_smem();
-      T.issue_map(next);
-    }
-
-    const bool valid = el < T.cells_of(batch);
-    float Djh[N], Djl[N], Dkh[N], Dkl[N];
-#pragma unroll
-    for (int m = 0; m < N; ++m) {
-      const float2 a = lds_pair(s_D + j * N + m), b = lds_pair(s_D + k * N + m);
-      Djh[m] = a.x, Djl[m] = a.y, Dkh[m] = b.x, Dkl[m] = b.y;
-    }
-    df vr[N];
-    // G converted to pairs scaled by 2^-sg as it is read
-    auto gpair = [&](int c, int i) {
-      const df d = fx_from_double(Gd[c * N3 + i * N2], sg);
-      return make_float2(d.hi, d.lo);
-    };
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-      // ---- gradient: q_r = D[i][.] u(., j, k), q_s = D[j][.] u(i, ., k), q_t = D[k][.] u(i, j, .)
-      fxacc ar, as, at;
-      const float cr = basis.cg[i];
-      fx_first(ar, basis.Dh[i * N], basis.Dl[i * N], u[0].hi, u[0].lo, cr);
+      // ---- transpose along the s- and t-lines, in place
       {
-        const df a = s_u[el * N3 + i * N2 + k], b = s_u[el * N3 + i * N2 + j * N];
-        fx_first(as, Djh[0], Djl[0], a.hi, a.lo, cgj);
-        fx_first(at, Dkh[0], Dkl[0], b.hi, b.lo, cgk);
-      }
+        df y[N];
 #pragma unroll
-      for (int m = 1; m < N; ++m) {
-        fx_fma(ar, basis.Dh[i * N + m], basis.Dl[i * N + m], u[m].hi, u[m].lo);
-        const df a = s_u[el * N3 + i * N2 + m * N + k], b = s_u[el * N3 + i * N2 + j * N + m];
-        fx_fma(as, Djh[m], Djl[m], a.hi, a.lo);
-        fx_fma(at, Dkh[m], Dkl[m], b.hi, b.lo);
-      }
-      const df qr = fx_finish(ar, cr), qs = fx_finish(as, cgj), qt = fx_finish(at, cgk);
-      // ---- metric, bound per point: max |q| times the row sums of |G|
-      float2 grr = make_float2(0.f, 0.f), grs = grr, grt = grr, gss = grr, gst = grr, gtt = grr;
-      if (valid) {
-        grr = gpair(0, i);
-        grs = gpair(1, i);
-        grt = gpair(2, i);
-        gss = gpair(3, i);
-        gst = gpair(4, i);
-        gtt = gpair(5, i);
-      }
-      const float kq = basis.K * fmaxf(fmaxf(fabsf(qr.hi), fabsf(qs.hi)), fabsf(qt.hi));
-      const float Cr = (fabsf(grr.x) + fabsf(grs.x) + fabsf(grt.x)) * kq;
-      const float Cs = (fabsf(grs.x) + fabsf(gss.x) + fabsf(gst.x)) * kq;
-      const float Ct = (fabsf(grt.x) + fabsf(gst.x) + fabsf(gtt.x)) * kq;
-      fxacc br, bs, bt;
-      fx_first(br, grr.x, grr.y, qr.hi, qr.lo, Cr);
-      fx_fma(br, grs.x, grs.y, qs.hi, qs.lo);
-      fx_fma(br, grt.x, grt.y, qt.hi, qt.lo);
-      fx_first(bs, grs.x, grs.y, qr.hi, qr.lo, Cs);
-      fx_fma(bs, gss.x, gss.y, qs.hi, qs.lo);
-      fx_fma(bs, gst.x, gst.y, qt.hi, qt.lo);
-      fx_first(bt, grt.x, grt.y, qr.hi, qr.lo, Ct);
-      fx_fma(bt, gst.x, gst.y, qs.hi, qs.lo);
-      fx_fma(bt, gtt.x, gtt.y, qt.hi, qt.lo);
-      vr[i] = fx_finish(br, Cr);
-      s_vs[el * N3 + i * N2 + jk] = fx_finish(bs, Cs);
-      s_vt[el * N3 + i * N2 + jk] = fx_finish(bt, Ct);
-    }
-    __syncthreads();  // barrier C: G tile consumed, s_vs / s_vt ready; s_gmax read
-    if (jk == 0) s_gmax[el] = 0;
-    if (tid == 0 && has_next) {
-      fence_proxy_async_smem();
-      T.issue_g(next);
-    }
-
-    // this batch's scatter targets; then prefetch the next batch's gather
-    uint32_t cur[N];
+        for (int m = 0; m < N; ++m) x[m] = s_s[sline + m * S::j];
+        fx_line(basis.T, x, y);
 #pragma unroll
-    for (int i = 0; i < N; ++i) cur[i] = idx[i];
-    if (has_next) {
-      const bool okm = mbar_wait(mbar_m, ph_m, wlim);
-      if (!okm && err_flag) atomicOr(err_flag, 1);  // the launch's result is void
-      ph_m ^= 1u;
-      if (okm) {
-        T.gather(next, el, jk, idx, raw);
+        for (int m = 0; m < N; ++m) s_s[sline + m * S::j] = y[m];
+#pragma unroll
+        for (int m = 0; m < N; ++m) x[m] = s_t[tline + m];
+        fx_line(basis.T, x, y);
+#pragma unroll
+        for (int m = 0; m < N; ++m) s_t[tline + m] = y[m];
+      }
+      fx_line(basis.T, vr, qr);  // the r-share of the own column
+      __syncthreads();
+      auto put = [&](int i, double v) {
+        if constexpr (EVEC) {
+          if (valid) dst[out_cell * N3 + i * N2 + jk] = v;
+        } else {
+          if (cur[i] != MFGB_INVALID_DOF) atomicAdd(dst + (size_t)NC * cur[i] + c, v);
+        }
+      };
+      if ((unsigned)(sc + 896) <= 1792u) {
+        const unsigned kout = (unsigned)(896 + sc) << 20;
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+          const df y = fx_sum3(qr[i], s_s[col + i * S::i], s_t[col + i * S::i]);
+          put(i, fx_f2d_fast(y.hi, kout) + fx_f2d_fast(y.lo, kout));
+        }
       } else {
 #pragma unroll
-        for (int i = 0; i < N; ++i) { idx[i] = MFGB_INVALID_DOF; raw[i] = 0.0; }
+        for (int i = 0; i < N; ++i) {
+          const df y = fx_sum3(qr[i], s_s[col + i * S::i], s_t[col + i * S::i]);
+          put(i, fx_f2d(y.hi, sc) + fx_f2d(y.lo, sc));
+        }
       }
+      // the prefetched gather's largest exponent per cell, once its loads have landed (read
+      // after the next component's first barrier, or the next batch's barrier A)
+      if (c + 1 < NC || has_next) reduce_exp(slot ^ 1);
     }
-
-    // ---- transpose: y = sum_m D[m][i] v_r(m,j,k) + D[m][j] v_s(i,m,k) + D[m][k] v_t(i,j,m);
-    // the bound of output i: max |v_r| of the own column and the maxima of the
-    // s- and t-lines it reads
-    float Dtjh[N], Dtjl[N], Dtkh[N], Dtkl[N];
-#pragma unroll
-    for (int m = 0; m < N; ++m) {
-      const float2 a = lds_pair(s_D + m * N + j), b = lds_pair(s_D + m * N + k);
-      Dtjh[m] = a.x, Dtjl[m] = a.y, Dtkh[m] = b.x, Dtkl[m] = b.y;
-    }
-    float mr = 0.f;
-#pragma unroll
-    for (int m = 0; m < N; ++m) mr = fmaxf(mr, fabsf(vr[m].hi));
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-      df ls[N], lt[N];
-      float ms = 0.f, mt = 0.f;
-#pragma unroll
-      for (int m = 0; m < N; ++m) {
-        ls[m] = s_vs[el * N3 + i * N2 + m * N + k];
-        lt[m] = s_vt[el * N3 + i * N2 + j * N + m];
-        ms = fmaxf(ms, fabsf(ls[m].hi));
-        mt = fmaxf(mt, fabsf(lt[m].hi));
-      }
-      const float C = __fmaf_rn(mt, cik, __fmaf_rn(ms, cij, mr * basis.ci[i]));
-      fxacc a;
-      fx_first(a, basis.Dh[i], basis.Dl[i], vr[0].hi, vr[0].lo, C);
-      fx_fma(a, Dtjh[0], Dtjl[0], ls[0].hi, ls[0].lo);
-      fx_fma(a, Dtkh[0], Dtkl[0], lt[0].hi, lt[0].lo);
-#pragma unroll
-      for (int m = 1; m < N; ++m) {
-        fx_fma(a, basis.Dh[m * N + i], basis.Dl[m * N + i], vr[m].hi, vr[m].lo);
-        fx_fma(a, Dtjh[m], Dtjl[m], ls[m].hi, ls[m].lo);
-        fx_fma(a, Dtkh[m], Dtkl[m], lt[m].hi, lt[m].lo);
-      }
-      const df y = fx_finish(a, C);
-      if (cur[i] != MFGB_INVALID_DOF)
-        atomicAdd(dst + cur[i], fast_out ? fx_f2d_fast(y.hi, kout) + fx_f2d_fast(y.lo, kout)
-                                         : fx_f2d(y.hi, sc) + fx_f2d(y.lo, sc));
-    }
-    // the prefetched gather's largest exponent per cell, once its loads have
-    // landed (read after the next barrier A)
-    if (has_next) reduce_exp(slot ^ 1);
-  }
-}
-
-
-// E-vector form of the kernel above (the CEED BK5 E-vector seam,
-// CEED_BK/include/kernels/BK5/templated_cuda_kernels.cuh:11-14): the caller's
-// FP64 G[e][6][n^3] arrives by bulk copies, each element's largest G exponent
-// is reduced in shared memory, and the metric converts G to pairs scaled by it
-// as it reads them; input and output are contiguous (plain loads prefetched a
-// batch ahead, plain stores).  Any input range is carried.
-template <int N, int E, int MB>
-__global__ void __launch_bounds__(E * N * N, MB)
-    bk5fx_evec_kernel(const int64_t n_cells, const double *__restrict__ G,
-                      const double *__restrict__ src, double *__restrict__ dst,
-                      const BasisFX<N> basis, int *__restrict__ err_flag) {
-  using L = TmaLayout<N, E, ArithF64>;
-  constexpr int N2 = N * N, N3 = N * N * N;
-  extern __shared__ __align__(128) unsigned char smem[];
-  double *sG = reinterpret_cast<double *>(smem);
-  df *s_u = reinterpret_cast<df *>(smem + L::g_bytes + L::map_bytes);
-  df *s_vs = s_u + E * N3;
-  df *s_vt = s_vs + E * N3;
-  uint64_t *mbar = reinterpret_cast<uint64_t *>(smem + L::g_bytes + L::map_bytes + L::work_bytes);
-  uint64_t *mbar_g = mbar;
-  __shared__ int s_emax[2][E];
-  __shared__ int s_gmax[E];  // largest biased exponent of the element's G
-
-  const int tid = threadIdx.x;
-  const int el = tid / N2;
-  const int jk = tid - el * N2;
-  const int j = jk / N;
-  const int k = jk - j * N;
-  const int64_t n_batches = (n_cells + E - 1) / E;
-  int64_t batch = blockIdx.x;
-  if (batch >= n_batches) return;  // uniform across the CTA
-
-  // D as (hi, lo) pairs: the rows and columns this thread needs with a runtime
-  // index are read from here at the start of the phase that uses them, so only
-  // one phase's 4N of them are live at a time
-  __shared__ float2 s_D[N * N];
-  for (int t = tid; t < N * N; t += blockDim.x) s_D[t] = make_float2(basis.Dh[t], basis.Dl[t]);
-  const float cgj = basis.cg[j], cgk = basis.cg[k], cij = basis.ci[j], cik = basis.ci[k];
-
-  // the G tiles (FP64, the caller's array) by bulk copies; no dof map
-  TmaTiles<N, E, ArithF64> T{n_cells, nullptr, G, src, sG, nullptr, mbar_g, nullptr};
-  auto fail = [&](uint32_t pg) {
-    if (tid == 0 && err_flag) atomicOr(err_flag, 1);
-    mbar_wait(mbar_g, pg);  // bounded wait for the copy still in flight
-  };
-
-  if (tid < 2 * E) (&s_emax[0][0])[tid] = 0;
-  if (tid < E) s_gmax[tid] = 0;
-  if (tid == 0) {
-    mbar_init(mbar_g, 1);
-    fence_mbar_init();
-  }
-  __syncthreads();
-  if (tid == 0) T.issue_g(batch);
-  uint32_t ph_g = 0;
-  double raw[N];
-  // this thread's column of element e of batch bt (E-vector: contiguous)
-  auto load = [&](int64_t bt) {
-    const int64_t e = bt * E + el;
-    const bool ok = e < n_cells;
-#pragma unroll
-    for (int i = 0; i < N; ++i) raw[i] = ok ? __ldg(src + e * N3 + i * N2 + jk) : 0.0;
-  };
-  auto reduce_exp = [&](int slot) {
-    int em = 0;
-#pragma unroll
-    for (int i = 0; i < N; ++i) em = max(em, dexp(raw[i]));
-    if (em) atomicMax(&s_emax[slot][el], em);
-  };
-  load(batch);
-  reduce_exp(0);
-
-  for (int it = 0; batch < n_batches; batch += gridDim.x, ++it) {
-    const int slot = it & 1;
-    const int64_t next = batch + gridDim.x;
-    const bool has_next = next < n_batches;
-    const bool okg = mbar_wait(mbar_g, ph_g);
-    if (__syncthreads_or(!okg)) { fail(ph_g); return; }  // barrier A
-    ph_g ^= 1u;
-    T.load_g_plain(batch, tid, blockDim.x);  // (every G tile arrives by bulk copy)
-    const bool valid = el < T.cells_of(batch);
-    const double *Gd = sG + el * 6 * N3 + jk;
-    if (valid) {  // the element's largest G exponent (read after barrier B)
-      int eg = 0;
-#pragma unroll 1
-      for (int c = 0; c < 6; ++c)
-#pragma unroll
-        for (int i = 0; i < N; ++i) eg = max(eg, dexp(Gd[c * N3 + i * N2]));
-      if (eg) atomicMax(&s_gmax[el], eg);
-    }
-    const int su = fx_offset(s_emax[slot][el]);
-    df u[N];
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-      u[i] = fx_from_double(raw[i], su);
-      s_u[el * N3 + i * N2 + jk] = u[i];
-    }
-    __syncthreads();  // barrier B: s_u and s_gmax ready, s_emax[slot] read
-    if (jk == 0) s_emax[slot][el] = 0;  // next written after barrier C of the next batch
-    const int sg = fx_offset(s_gmax[el]);
-    const int sc = su + sg;  // the element's result scale
-    const bool fast_out = (unsigned)(sc + 896) <= 1792u;
-    const unsigned kout = (unsigned)(896 + sc) << 20;
-
-    float Djh[N], Djl[N], Dkh[N], Dkl[N];
-#pragma unroll
-    for (int m = 0; m < N; ++m) {
-      const float2 a = lds_pair(s_D + j * N + m), b = lds_pair(s_D + k * N + m);
-      Djh[m] = a.x, Djl[m] = a.y, Dkh[m] = b.x, Dkl[m] = b.y;
-    }
-    df vr[N];
-    // G converted to pairs scaled by 2^-sg as it is read
-    auto gpair = [&](int c, int i) {
-      const df d = fx_from_double(Gd[c * N3 + i * N2], sg);
-      return make_float2(d.hi, d.lo);
-    };
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-      // ---- gradient: q_r = D[i][.] u(., j, k), q_s = D[j][.] u(i, ., k), q_t = D[k][.] u(i, j, .)
-      fxacc ar, as, at;
-      const float cr = basis.cg[i];
-      fx_first(ar, basis.Dh[i * N], basis.Dl[i * N], u[0].hi, u[0].lo, cr);
-      {
-        const df a = s_u[el * N3 + i * N2 + k], b = s_u[el * N3 + i * N2 + j * N];
-        fx_first(as, Djh[0], Djl[0], a.hi, a.lo, cgj);
-        fx_first(at, Dkh[0], Dkl[0], b.hi, b.lo, cgk);
-      }
-#pragma unroll
-      for (int m = 1; m < N; ++m) {
-        fx_fma(ar, basis.Dh[i * N + m], basis.Dl[i * N + m], u[m].hi, u[m].lo);
-        const df a = s_u[el * N3 + i * N2 + m * N + k], b = s_u[el * N3 + i * N2 + j * N + m];
-        fx_fma(as, Djh[m], Djl[m], a.hi, a.lo);
-        fx_fma(at, Dkh[m], Dkl[m], b.hi, b.lo);
-      }
-      const df qr = fx_finish(ar, cr), qs = fx_finish(as, cgj), qt = fx_finish(at, cgk);
-      // ---- metric, bound per point: max |q| times the row sums of |G|
-      float2 grr = make_float2(0.f, 0.f), grs = grr, grt = grr, gss = grr, gst = grr, gtt = grr;
-      if (valid) {
-        grr = gpair(0, i);
-        grs = gpair(1, i);
-        grt = gpair(2, i);
-        gss = gpair(3, i);
-        gst = gpair(4, i);
-        gtt = gpair(5, i);
-      }
-      const float kq = basis.K * fmaxf(fmaxf(fabsf(qr.hi), fabsf(qs.hi)), fabsf(qt.hi));
-      const float Cr = (fabsf(grr.x) + fabsf(grs.x) + fabsf(grt.x)) * kq;
-      const float Cs = (fabsf(grs.x) + fabsf(gss.x) + fabsf(gst.x)) * kq;
-      const float Ct = (fabsf(grt.x) + fabsf(gst.x) + fabsf(gtt.x)) * kq;
-      fxacc br, bs, bt;
-      fx_first(br, grr.x, grr.y, qr.hi, qr.lo, Cr);
-      fx_fma(br, grs.x, grs.y, qs.hi, qs.lo);
-      fx_fma(br, grt.x, grt.y, qt.hi, qt.lo);
-      fx_first(bs, grs.x, grs.y, qr.hi, qr.lo, Cs);
-      fx_fma(bs, gss.x, gss.y, qs.hi, qs.lo);
-      fx_fma(bs, gst.x, gst.y, qt.hi, qt.lo);
-      fx_first(bt, grt.x, grt.y, qr.hi, qr.lo, Ct);
-      fx_fma(bt, gst.x, gst.y, qs.hi, qs.lo);
-      fx_fma(bt, gtt.x, gtt.y, qt.hi, qt.lo);
-      vr[i] = fx_finish(br, Cr);
-      s_vs[el * N3 + i * N2 + jk] = fx_finish(bs, Cs);
-      s_vt[el * N3 + i * N2 + jk] = fx_finish(bt, Ct);
-    }
-    __syncthreads();  // barrier C: G tile consumed, s_vs / s_vt ready; s_gmax read
-    if (jk == 0) s_gmax[el] = 0;
-    if (tid == 0 && has_next) {
-      fence_proxy_async_smem();
-      T.issue_g(next);
-    }
-
-    const int64_t e_out = batch * E + el;  // this batch's element of the thread
-    if (has_next) load(next);  // the next batch's column, used after its barrier A
-
-    // ---- transpose: y = sum_m D[m][i] v_r(m,j,k) + D[m][j] v_s(i,m,k) + D[m][k] v_t(i,j,m);
-    // the bound of output i: max |v_r| of the own column and the maxima of the
-    // s- and t-lines it reads
-    float Dtjh[N], Dtjl[N], Dtkh[N], Dtkl[N];
-#pragma unroll
-    for (int m = 0; m < N; ++m) {
-      const float2 a = lds_pair(s_D + m * N + j), b = lds_pair(s_D + m * N + k);
-      Dtjh[m] = a.x, Dtjl[m] = a.y, Dtkh[m] = b.x, Dtkl[m] = b.y;
-    }
-    float mr = 0.f;
-#pragma unroll
-    for (int m = 0; m < N; ++m) mr = fmaxf(mr, fabsf(vr[m].hi));
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-      df ls[N], lt[N];
-      float ms = 0.f, mt = 0.f;
-#pragma unroll
-      for (int m = 0; m < N; ++m) {
-        ls[m] = s_vs[el * N3 + i * N2 + m * N + k];
-        lt[m] = s_vt[el * N3 + i * N2 + j * N + m];
-        ms = fmaxf(ms, fabsf(ls[m].hi));
-        mt = fmaxf(mt, fabsf(lt[m].hi));
-      }
-      const float C = __fmaf_rn(mt, cik, __fmaf_rn(ms, cij, mr * basis.ci[i]));
-      fxacc a;
-      fx_first(a, basis.Dh[i], basis.Dl[i], vr[0].hi, vr[0].lo, C);
-      fx_fma(a, Dtjh[0], Dtjl[0], ls[0].hi, ls[0].lo);
-      fx_fma(a, Dtkh[0], Dtkl[0], lt[0].hi, lt[0].lo);
-#pragma unroll
-      for (int m = 1; m < N; ++m) {
-        fx_fma(a, basis.Dh[m * N + i], basis.Dl[m * N + i], vr[m].hi, vr[m].lo);
-        fx_fma(a, Dtjh[m], Dtjl[m], ls[m].hi, ls[m].lo);
-        fx_fma(a, Dtkh[m], Dtkl[m], lt[m].hi, lt[m].lo);
-      }
-      const df y = fx_finish(a, C);
-      if (e_out < n_cells)
-        dst[e_out * N3 + i * N2 + jk] = fast_out ? fx_f2d_fast(y.hi, kout) + fx_f2d_fast(y.lo, kout)
-                                                 : fx_f2d(y.hi, sc) + fx_f2d(y.lo, sc);
-    }
-    // the next batch's largest exponent per element (read after its barrier A)
-    if (has_next) reduce_exp(slot ^ 1);
   }
 }
 

@@ -68,7 +68,7 @@ template <> struct ElemsPerCtaPt<9> { static constexpr int value = 1; };
 // 2 = column with TMA-prefetched geometric factors.  Default per
 // (arithmetic, N); overridable at run time (autotuner).
 // 5 and 6 (double-float only, GLL operators): the offset-accumulation kernel of
-// mfgb_bk5fx.cuh at the shape-2 and shape-4 cells per CTA; elsewhere they run as 2 / 4.
+// mfgb_bk5fx.cuh at its two cells per CTA (FxDefault, FxAlt); elsewhere they run as 2 / 4.
 enum { SHAPE_COLUMN = 0, SHAPE_POINT = 1, SHAPE_TMA = 2, SHAPE_COLUMN_ALT = 3, SHAPE_TMA_ALT = 4,
        SHAPE_FX = 5, SHAPE_FX_ALT = 6 };
 int kernel_shape(int arith_class, int N);  // mfgb_api.cu

@@ -95,8 +95,8 @@ typedef struct {
    with the geometric factors prefetched by bulk TMA copies, 3 / 4 = shapes 0 /
    2 at an alternative number of cells per thread block (the autotuner's
    elements-per-block choice); for MFGB_ARITH_FP64_DF also 5 / 6 = the
-   offset-accumulation kernel with per-cell scaling at the cells per block of
-   shapes 2 / 4 (GLL operators; elsewhere they run as 2 / 4).  The library
+   offset-accumulation kernel with per-cell scaling at two cells per block of
+   its own (GLL operators; elsewhere they run as 2 / 4).  The library
    starts from a built-in table; the autotuner overrides it.  No
    counterpart in the reference (its launch shape is a compile-time choice,
    CEED_BK/src/BK5/templated_cuda_benchmark.cc:114-124). */
@@ -245,8 +245,8 @@ mfgb_status mfgb_bk3_evector(int degree, int64_t nelmt, const double *d_basis,
    keeps two device vectors for this call after the first use. */
 mfgb_status mfgb_vmult_host(const mfgb_operator *op, double *h_dst, const double *h_src, int arith,
                             void *stream);
-/* number of z-slabs of that pipeline (1..64; 0 = automatic: 16, each slab at
-   least two cell layers) */
+/* number of z-slabs of that pipeline (1..64; 0 = automatic: 2 to 24 with the
+   square root of the vector's size, each slab at least two cell layers) */
 mfgb_status mfgb_set_host_pipeline(int slabs);
 
 /* ---- diagonal -------------------------------------------------------------

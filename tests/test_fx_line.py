@@ -1,0 +1,128 @@
+"""The line contractions of the double-float kernels (benchmarks_gb300/csrc/
+mfgb_fxline.cuh: fx_grid, fx_line, fx_sum3 in even-odd form) restated with numpy
+float32 operations.
+
+Claims checked: rounding a line to the grid of 3 max|x| leaves the sums and
+differences of mirrored values exact; with the offset 3 max(bound A, bound B) the
+high parts of A +- B add exactly; the result is as accurate as the plain offset sum
+(2^-42 of the bound at most, near 2^-46 in the mean); and on the GPU a caller's
+general derivative matrix takes the plain form, a mirror-antisymmetric one the
+even-odd form, both to 1e-12 of the oracle."""
+import numpy as np
+import pytest
+
+from test_fx_arith import Acc, EXT, ext, f32, gll_derivative, split
+
+extended = pytest.mark.skipif(np.finfo(np.longdouble).nmant < 60, reason="needs an extended long double")
+
+
+def grid(x, C):
+    t = (C + x[0]).astype(f32)
+    h = (t - C).astype(f32)
+    return h, ((x[0] - h).astype(f32) + x[1]).astype(f32)
+
+
+def add(a, b, sign=1):
+    """(sum of the parts, whether the high parts' sum is exact)"""
+    h = (a[0] + f32(sign) * b[0]).astype(f32)
+    exact = np.all(h.astype(EXT) == a[0].astype(EXT) + sign * b[0].astype(EXT))
+    return (h, (a[1] + f32(sign) * b[1]).astype(f32)), bool(exact)
+
+
+def line(M, x, sym):
+    """fx_line for mirror-symmetric (sym = 1) or antisymmetric (-1) M; x: pairs per input"""
+    no, ni = M.shape
+    hi, ok = ni // 2, True
+    mx = (np.max([np.abs(v[0]) for v in x], axis=0) * f32(1 + 2.0 ** -20)).astype(f32)
+    C = (mx * f32(3)).astype(f32)
+    x = [v if ni % 2 and i == hi else grid(v, C) for i, v in enumerate(x)]
+    e, f = [], []
+    for i in range(hi):
+        s, k1 = add(x[i], x[ni - 1 - i])
+        d, k2 = add(x[i], x[ni - 1 - i], -1)
+        e.append(s), f.append(d)
+        ok &= k1 and k2
+    y, bound = [None] * no, []
+    for o in range((no + 1) // 2):
+        P = [split(0.5 * (M[o, i] + M[o, ni - 1 - i])) for i in range(hi)]
+        Q = [split(0.5 * (M[o, i] - M[o, ni - 1 - i])) for i in range(hi)]
+        xs = list(e)
+        if ni % 2:
+            P.append(split(M[o, hi])), xs.append(x[hi])
+        bp = sum((2 if i < hi else 1) * abs(float(p[0])) for i, p in enumerate(P))
+        bq = sum(2 * abs(float(q[0])) for q in Q)
+        Co = (f32(3 * (1 + 2.0 ** -18) * max(bp, bq)) * mx).astype(f32)
+        bound.append(Co)
+        A, B = Acc(Co), Acc(Co)
+        for p, v in zip(P, xs):
+            A.add((np.full_like(mx, p[0]), np.full_like(mx, p[1])), v)
+        for q, v in zip(Q, f):
+            B.add((np.full_like(mx, q[0]), np.full_like(mx, q[1])), v)
+        a, b = A.finish(), B.finish()
+        ok &= A.exact_ok and B.exact_ok
+        if no % 2 and o == no // 2:
+            y[o] = b if sym < 0 else a
+        else:
+            y[o], k1 = add(a, b)
+            y[no - 1 - o], k2 = add(b, a, -1) if sym < 0 else add(a, b, -1)
+            ok &= k1 and k2
+    return y, np.max(bound, axis=0), ok
+
+
+@extended
+@pytest.mark.parametrize("n", range(2, 10))
+@pytest.mark.parametrize("spread", [0, 12])  # binades between a line's values
+def test_line_in_even_odd_form(n, spread):
+    D = gll_derivative(n)[1]
+    D = 0.5 * (D - D[::-1, ::-1])
+    rng = np.random.default_rng(n)
+    x = [split(rng.uniform(-1, 1, 3000) * 2.0 ** -rng.integers(0, spread + 1, 3000)) for _ in range(n)]
+    for M in (D, D.T.copy()):
+        y, C, ok = line(M, x, -1)
+        assert ok
+        Mp = [[split(M[o, i]) for i in range(n)] for o in range(n)]
+        err = np.array([np.abs(ext(y[o]) - sum(ext(Mp[o][i]) * ext(x[i]) for i in range(n))) / C.astype(EXT)
+                        for o in range(n)])
+        assert float(err.max()) < 2.0 ** -42
+        assert float(np.sqrt(np.mean(err ** 2))) < 2.0 ** -45
+
+
+@extended
+def test_sum_of_three_shares():
+    rng = np.random.default_rng(3)
+    v = [split(rng.uniform(-1, 1, 20000) * 2.0 ** rng.integers(-20, 20, 20000)) for _ in range(3)]
+    (a, al), (b, bl), (c, cl) = v
+    s = a + b
+    bb = s - a
+    e = (a - (s - bb)) + (b - bb)
+    t = s + c
+    cc = t - s
+    g = (s - (t - cc)) + (c - cc)
+    lo = ((al + bl) + (e + g)) + cl
+    big = np.max([np.abs(x[0]) for x in v], axis=0).astype(EXT)
+    assert float(np.max(np.abs(ext((t, lo)) - sum(map(ext, v))) / big)) < 2.0 ** -45
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("p", range(1, 9))
+def test_seam_matrices_of_both_kinds(p):
+    """Cell counts around the cells per thread block and the dof-map windows' ends."""
+    import torch
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import benchmarks_gb300 as mf
+    from oracle import oracle
+    n = p + 1
+    rng = np.random.default_rng(p)
+    general = rng.uniform(-1, 1, (n, n))
+    for D in (general, 0.5 * (general - general[::-1, ::-1])):
+        for cells in (1, 2, 7, 37):
+            G = rng.uniform(-1, 1, cells * 6 * n ** 3)
+            u = rng.uniform(-1, 1, cells * n ** 3)
+            want = oracle.evector(n, D, G, u)
+            dev = [torch.from_numpy(np.ascontiguousarray(a).reshape(-1)).cuda() for a in (D, G, u)]
+            got = mf.bk5_evector(p, *dev, torch.zeros_like(dev[2]), arith="df").cpu().numpy()
+            assert np.linalg.norm(got - want) <= 1e-12 * np.linalg.norm(want)
+            index = torch.arange(cells * n ** 3, dtype=torch.int32, device="cuda")
+            got = mf.bk5_lvector(p, *dev, torch.zeros_like(dev[2]), index, arith="df").cpu().numpy()
+            assert np.linalg.norm(got - want) <= 1e-12 * np.linalg.norm(want)
