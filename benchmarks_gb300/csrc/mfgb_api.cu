@@ -98,7 +98,8 @@ mfgb_status ensure_fx(mfgb_operator *op) {
       (op->d_JxW && (st = dev_alloc((void **)&op->d_JxWfx, sizeof(float2) * op->n_cells * n3,
                                     "JxW (scaled double-float)"))) ||
       (st = cuda_status(g_to_fx(op->n_cells, (int)(6 * n3), op->d_G, op->d_Gfx, op->d_Gexp, nullptr,
-                                op->d_JxW ? (int)n3 : 0, op->d_JxW, op->d_JxWfx),
+                                op->d_JxW ? (int)n3 : 0, op->d_JxW, op->d_JxWfx,
+                                op->quadrature ? (int)nq : 0),
                         "G -> scaled double-float")) ||
       (st = cuda_status(cudaDeviceSynchronize(), "G -> scaled double-float"))) {
     // all or nothing: the arrays exist only complete

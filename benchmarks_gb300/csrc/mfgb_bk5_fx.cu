@@ -104,8 +104,9 @@ static cudaError_t fx_pairs(int64_t n_cells, const uint32_t *map, const float2 *
 template <int N, int SYM>
 static cudaError_t fx_seam(int64_t n_cells, const uint32_t *map, const double *G, const double *src,
                            double *dst, const FxBasis<N, SYM> &b, cudaStream_t s) {
-  // FP64 tiles take twice the shared memory of pairs: fewer resident CTAs
-  using Sh = FxShape<FxDefault<N>::E, (FxDefault<N>::MB + 1) / 2, FxDefault<N>::NB>;
+  // (the general form keeps N^2 matrix entries live: its register cap is the wider one)
+  using Sh = FxShape<FxDefault<N>::E, SYM == 0 ? (FxDefault<N>::MB + 1) / 2 : FxDefault<N>::MB,
+                     FxDefault<N>::NB>;
   if (map == nullptr)
     return fx_run<N, Sh, double, true, 1, SYM, false>(n_cells, nullptr, G, nullptr, src, dst, b, s, nullptr);
   if (reinterpret_cast<uintptr_t>(map) & 15u)
@@ -180,10 +181,18 @@ cudaError_t bk5_fx(int N, int64_t n_cells, const uint32_t *map, const float2 *G,
 // (hi = nearest float, lo = nearest float of the remainder); gexp[cell] =
 // e - 1022 (0 for an all-zero cell).  Values more than 2^126 below the cell's
 // largest lose their low digits or flush to zero, far below the operator's
-// accuracy bar relative to the cell's largest term.
+// accuracy bar relative to the cell's largest term.  nt > 0: the nt^3 points of
+// every component are written with their first and last index exchanged (the
+// order the Gauss-point kernel reads).
 __global__ void g_to_fx_kernel(int64_t n_cells, int per_cell, const double *__restrict__ G,
                                float2 *__restrict__ out, int *__restrict__ gexp, int per_j,
-                               const double *__restrict__ J, float2 *__restrict__ jout) {
+                               const double *__restrict__ J, float2 *__restrict__ jout, int nt) {
+  auto from = [=](int t) {
+    if (nt == 0) return t;
+    const int n2 = nt * nt, c = t / (n2 * nt), r = t - c * n2 * nt;
+    const int a = r / n2, b = (r - a * n2) / nt, d = r - a * n2 - b * nt;
+    return (c * nt + d) * n2 + b * nt + a;
+  };
   const int lane = threadIdx.x & 31;
   const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int64_t n_warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -207,19 +216,19 @@ __global__ void g_to_fx_kernel(int64_t n_cells, int per_cell, const double *__re
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) em = max(em, __shfl_xor_sync(0xFFFFFFFFu, em, o));
     const int off = fx_offset(em);
-    for (int t = lane; t < per_cell; t += 32) out[c * per_cell + t] = split(g[t], off);
-    for (int t = lane; t < per_j; t += 32) jout[c * per_j + t] = split(j[t], off);
+    for (int t = lane; t < per_cell; t += 32) out[c * per_cell + t] = split(g[from(t)], off);
+    for (int t = lane; t < per_j; t += 32) jout[c * per_j + t] = split(j[from(t)], off);
     if (lane == 0) gexp[c] = off;
   }
 }
 
 cudaError_t g_to_fx(int64_t n_cells, int per_cell, const double *G, float2 *Gfx, int *gexp,
-                    cudaStream_t s, int per_cell_j, const double *J, float2 *Jfx) {
+                    cudaStream_t s, int per_cell_j, const double *J, float2 *Jfx, int nt) {
   if (n_cells <= 0) return cudaSuccess;
   if (per_cell_j > 0 && (!J || !Jfx)) return cudaErrorInvalidValue;
   const int64_t blocks = std::min<int64_t>((n_cells + 7) / 8, 152 * 32);
   g_to_fx_kernel<<<(int)blocks, 256, 0, s>>>(n_cells, per_cell, G, Gfx, gexp,
-                                             per_cell_j > 0 ? per_cell_j : 0, J, Jfx);
+                                             per_cell_j > 0 ? per_cell_j : 0, J, Jfx, nt);
   return cudaGetLastError();
 }
 

@@ -161,34 +161,6 @@ struct FxLines {
   unsigned short s[E * N * N], t[E * N * N];
 };
 
-// deals the lines a[0..T) over half-warps: each takes lines from the banks (offset mod 16) that
-// have most left, a bank twice only when every other one is used up
-template <int T>
-constexpr void fx_deal(const int (&a)[T], unsigned short (&out)[T]) {
-  bool used[T] = {};
-  int left[16] = {};
-  for (int v : a) ++left[v % 16];
-  for (int h = 0; h < T; h += 16) {
-    bool bank[16] = {};
-    for (int t = h; t < T && t < h + 16; ++t) {
-      int best = -1;
-      for (int b = 0; b < 16; ++b)
-        if (left[b] > 0 && !bank[b] && (best < 0 || left[b] > left[best])) best = b;
-      if (best < 0)
-        for (int b = 0; b < 16; ++b)
-          if (left[b] > 0 && (best < 0 || left[b] > left[best])) best = b;
-      bank[best] = true;
-      --left[best];
-      for (int q = 0; q < T; ++q)
-        if (!used[q] && a[q] % 16 == best) {
-          used[q] = true;
-          out[t] = (unsigned short)a[q];
-          break;
-        }
-    }
-  }
-}
-
 template <int N, int E>
 constexpr FxLines<N, E> fx_lines() {
   using S = FxStride<N>;

@@ -82,10 +82,11 @@ cudaError_t bk5_fx_g64(int N, int64_t n_cells, const uint32_t *map, const double
 // contiguous src / dst (dst overwritten)
 cudaError_t bk5_fx_evec(int N, int64_t nelmt, const double *G, const double *src, double *dst,
                         const double *D, cudaStream_t s);
-// per-cell scaled float pairs of G (and of JxW, with the same per-cell offset)
+// per-cell scaled float pairs of G (and of JxW, with the same per-cell offset); nt > 0: the nt^3
+// points of every component with the first and last index exchanged (the Gauss-point kernel's order)
 cudaError_t g_to_fx(int64_t n_cells, int per_cell, const double *G, float2 *Gfx, int *gexp,
                     cudaStream_t s, int per_cell_j = 0, const double *J = nullptr,
-                    float2 *Jfx = nullptr);
+                    float2 *Jfx = nullptr, int nt = 0);
 cudaError_t bk5_df_g64(int N, int64_t n_cells, const uint32_t *map, const double *G,
                        const double *src, double *dst, const double *D, cudaStream_t s,
                        const int *done = nullptr);

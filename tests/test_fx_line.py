@@ -3,8 +3,8 @@ mfgb_fxline.cuh: fx_grid, fx_line, fx_sum3 in even-odd form) restated with numpy
 float32 operations.
 
 Claims checked: rounding a line to the grid of 3 max|x| leaves the sums and
-differences of mirrored values exact; with the offset 3 max(bound A, bound B) the
-high parts of A +- B add exactly; the result is as accurate as the plain offset sum
+differences of mirrored values exact; with the offset max(bound A, bound B) + bound(A +- B)
+the high parts of A +- B add exactly; the result is as accurate as the plain offset sum
 (2^-42 of the bound at most, near 2^-46 in the mean); and on the GPU a caller's
 general derivative matrix takes the plain form, a mirror-antisymmetric one the
 even-odd form, both to 1e-12 of the oracle."""
@@ -51,7 +51,9 @@ def line(M, x, sym):
             P.append(split(M[o, hi])), xs.append(x[hi])
         bp = sum((2 if i < hi else 1) * abs(float(p[0])) for i, p in enumerate(P))
         bq = sum(2 * abs(float(q[0])) for q in Q)
-        Co = (f32(3 * (1 + 2.0 ** -18) * max(bp, bq)) * mx).astype(f32)
+        row = sum(2 * max(abs(float(p[0])), abs(float(q[0]))) for p, q in zip(P, Q)) + \
+            (abs(float(P[hi][0])) if ni % 2 else 0)
+        Co = (f32((1 + 2.0 ** -18) * (max(bp, bq) + row)) * mx).astype(f32)
         bound.append(Co)
         A, B = Acc(Co), Acc(Co)
         for p, v in zip(P, xs):
@@ -125,4 +127,31 @@ def test_seam_matrices_of_both_kinds(p):
             assert np.linalg.norm(got - want) <= 1e-12 * np.linalg.norm(want)
             index = torch.arange(cells * n ** 3, dtype=torch.int32, device="cuda")
             got = mf.bk5_lvector(p, *dev, torch.zeros_like(dev[2]), index, arith="df").cpu().numpy()
+            assert np.linalg.norm(got - want) <= 1e-12 * np.linalg.norm(want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("p", range(1, 9))
+def test_interpolation_seams_of_both_kinds(p):
+    """BK1 and BK3 with mirror-symmetric and general matrices, element counts around the cells per
+    thread block."""
+    import torch
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import benchmarks_gb300 as mf
+    from oracle import oracle
+    n, q = p + 1, p + 2
+    rng = np.random.default_rng(p)
+    B, D = rng.uniform(-1, 1, (q, n)), rng.uniform(-1, 1, (q, q))
+    for b, d in ((B, D), (0.5 * (B + B[::-1, ::-1]), 0.5 * (D - D[::-1, ::-1]))):
+        for cells in (1, 5, 29):
+            G, J = rng.uniform(-1, 1, cells * 6 * q ** 3), rng.uniform(0.5, 1.5, cells * q ** 3)
+            u = rng.uniform(-1, 1, cells * n ** 3)
+            db, dd, dG, dJ, du = (torch.from_numpy(np.ascontiguousarray(a).reshape(-1)).cuda()
+                                  for a in (b, d, G, J, u))
+            got = mf.bk3_evector(p, db, dd, dG, du, torch.zeros_like(du), arith="df").cpu().numpy()
+            want = oracle.bk3_evector(n, q, b, d, G, u)
+            assert np.linalg.norm(got - want) <= 1e-12 * np.linalg.norm(want)
+            got = mf.bk1_evector(p, db, dJ, du, torch.zeros_like(du), arith="df").cpu().numpy()
+            want = oracle.bk1_evector(n, q, b, J, u)
             assert np.linalg.norm(got - want) <= 1e-12 * np.linalg.norm(want)
