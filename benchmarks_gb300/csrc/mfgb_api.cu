@@ -190,13 +190,14 @@ mfgb_status vmult_impl(mfgb_operator *op, double *dst, const double *src, int ar
 }
 
 // kernel shape per (arithmetic class, N): 0 column, 1 point-per-thread,
-// 2 column with TMA-prefetched geometric factors, 3 / 4 the column / TMA
-// kernels at the alternative cells per CTA (AltElems).  Defaults are the fastest
+// 2 column with TMA-prefetched geometric factors (FP32, and FP64 from N = 6: the
+// line kernel), 3 / 4 the column / TMA kernels at the alternative cells per CTA
+// (AltElems, LineAlt).  Defaults are the fastest
 // shape per degree measured on a GB300 at ~3e7 DoFs (autotune.py re-measures).
 static int g_shape[3][10] = {
-    {0, 0, 4, 3, 2, 4, 2, 1, 2, 1},  // FP64
+    {0, 0, 4, 3, 2, 4, 2, 2, 2, 2},  // FP64
     {2, 2, 5, 5, 5, 5, 5, 5, 5, 5},  // double-float (5, 6: offset accumulation)
-    {0, 0, 3, 3, 0, 3, 2, 4, 4, 2},  // FP32
+    {0, 0, 3, 2, 2, 2, 2, 2, 2, 2},  // FP32
 };
 
 // device-side error word, one per device: bit 0 a TMA wait that ran out of

@@ -289,26 +289,27 @@ __device__ __forceinline__ void fx_line_joint(const FxMat<NI, NO, SP> &P, const 
   }
 }
 
-// deals the lines a[0..T) over half-warps: each takes lines from the banks (offset mod 16) that
-// have most left, a bank twice only when every other one is used up
-template <int T>
+// deals the lines a[0..T) over groups of W lanes that access shared memory together (16 for 8-byte
+// values, 32 for 4-byte ones): each takes lines from the banks (offset mod W) that have most left, a
+// bank twice only when every other one is used up
+template <int W = 16, int T>
 constexpr void fx_deal(const int (&a)[T], unsigned short (&out)[T]) {
   bool used[T] = {};
-  int left[16] = {};
-  for (int v : a) ++left[v % 16];
-  for (int h = 0; h < T; h += 16) {
-    bool bank[16] = {};
-    for (int t = h; t < T && t < h + 16; ++t) {
+  int left[W] = {};
+  for (int v : a) ++left[v % W];
+  for (int h = 0; h < T; h += W) {
+    bool bank[W] = {};
+    for (int t = h; t < T && t < h + W; ++t) {
       int best = -1;
-      for (int b = 0; b < 16; ++b)
+      for (int b = 0; b < W; ++b)
         if (left[b] > 0 && !bank[b] && (best < 0 || left[b] > left[best])) best = b;
       if (best < 0)
-        for (int b = 0; b < 16; ++b)
+        for (int b = 0; b < W; ++b)
           if (left[b] > 0 && (best < 0 || left[b] > left[best])) best = b;
       bank[best] = true;
       --left[best];
       for (int q = 0; q < T; ++q)
-        if (!used[q] && a[q] % 16 == best) {
+        if (!used[q] && a[q] % W == best) {
           used[q] = true;
           out[t] = (unsigned short)a[q];
           break;

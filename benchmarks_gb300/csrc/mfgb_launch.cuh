@@ -2,6 +2,7 @@
 #pragma once
 #include <algorithm>
 #include "mfgb_bk5.cuh"
+#include "mfgb_bk5line.cuh"
 
 namespace mfgb {
 
@@ -19,7 +20,6 @@ template <> struct ElemsPerCta<9> { static constexpr int value = 2; };
 // bulk-TMA column kernel: elements per CTA, per arithmetic (default: as the
 // column kernel)
 template <int N, class A> struct ElemsPerCtaTma { static constexpr int value = ElemsPerCta<N>::value; };
-template <> struct ElemsPerCtaTma<5, ArithF32> { static constexpr int value = 6; };
 template <> struct ElemsPerCtaTma<5, ArithDF> { static constexpr int value = 5; };
 
 // Alternative cells per CTA for the autotuner's shapes 3 (column) and 4 (bulk
@@ -103,6 +103,58 @@ int ctas_per_sm(K kernel, int threads, size_t smem) {
   return ps;
 }
 
+// Shapes 2 and 4 of the plain arithmetics as the line kernel (mfgb_bk5line.cuh): cells per CTA,
+// resident CTAs and work arrays.  FP32 at every degree, FP64 from N = 6 (below, the column kernel's
+// 4.05 / 3.82 ms at N = 4, 5 are not beaten: 4.62 / 3.86; the FP64 pipe is the bound and the even-odd
+// additions cost as much as the multiply-adds they save).  Kernel ms at 3e7 DoFs, FP32, N = 3..9: 0.67,
+// 0.40, 0.32, 0.28, 0.26, 0.23, 0.24 (vmult with the best earlier shape: 0.75, 0.44, 0.43, 0.36, 0.51,
+// 0.28, 0.42); FP64, N = 6..9: 4.24, 4.16, 3.87, 4.67 (4.48, 4.63, 4.18, 4.99).
+template <int E_, int MB_, int NB_> struct LineShapeIs {
+  static constexpr int E = E_, MB = MB_, NB = NB_;
+};
+template <int N, class A> struct LineShape : LineShapeIs<0, 0, 0> {};
+template <> struct LineShape<2, ArithF32> : LineShapeIs<64, 6, 2> {};
+template <> struct LineShape<3, ArithF32> : LineShapeIs<28, 5, 2> {};
+template <> struct LineShape<4, ArithF32> : LineShapeIs<16, 4, 3> {};
+template <> struct LineShape<5, ArithF32> : LineShapeIs<10, 4, 2> {};
+template <> struct LineShape<6, ArithF32> : LineShapeIs<7, 4, 3> {};
+template <> struct LineShape<7, ArithF32> : LineShapeIs<5, 4, 2> {};
+template <> struct LineShape<8, ArithF32> : LineShapeIs<3, 4, 3> {};
+template <> struct LineShape<9, ArithF32> : LineShapeIs<3, 3, 3> {};
+template <> struct LineShape<6, ArithF64> : LineShapeIs<5, 3, 2> {};
+template <> struct LineShape<7, ArithF64> : LineShapeIs<3, 3, 2> {};
+template <> struct LineShape<8, ArithF64> : LineShapeIs<2, 3, 2> {};
+template <> struct LineShape<9, ArithF64> : LineShapeIs<1, 4, 2> {};
+// fewer cells per CTA: shape 4, and shape 2 on meshes too small for one batch per resident CTA
+template <int N, class A> struct LineAlt : LineShape<N, A> {};
+template <> struct LineAlt<2, ArithF32> : LineShapeIs<32, 8, 3> {};
+template <> struct LineAlt<3, ArithF32> : LineShapeIs<14, 8, 3> {};
+template <> struct LineAlt<4, ArithF32> : LineShapeIs<8, 8, 3> {};
+template <> struct LineAlt<5, ArithF32> : LineShapeIs<5, 8, 3> {};
+template <> struct LineAlt<6, ArithF32> : LineShapeIs<3, 8, 3> {};
+template <> struct LineAlt<7, ArithF32> : LineShapeIs<3, 6, 2> {};
+template <> struct LineAlt<8, ArithF32> : LineShapeIs<1, 12, 3> {};
+template <> struct LineAlt<9, ArithF32> : LineShapeIs<1, 8, 3> {};
+template <> struct LineAlt<6, ArithF64> : LineShapeIs<3, 5, 2> {};
+
+// one launch of the line kernel
+template <int N, class A, class Sh>
+cudaError_t line_run(int64_t n_cells, const uint32_t *map, const typename A::GType *G,
+                     const typename A::VecT *src, typename A::VecT *dst, const Basis<N, A> &basis,
+                     int *grid_used, cudaStream_t stream, const int *done) {
+  constexpr int E = Sh::E, T = E * N * N;
+  constexpr size_t smem = LineLayout<N, E, typename A::VecT, Sh::NB>::total;
+  const auto kernel = bk5_line_kernel<N, E, Sh::MB, Sh::NB, A>;
+  static int per_sm = -1;
+  if (per_sm < 0) per_sm = std::max(1, ctas_per_sm(kernel, T, smem));
+  const int64_t nb = (n_cells + E - 1) / E;
+  const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(nb, (int64_t)per_sm * num_sms()));
+  if (grid_used) *grid_used = grid;
+  if (n_cells <= 0) return cudaSuccess;
+  kernel<<<grid, T, smem, stream>>>(n_cells, map, G, src, dst, basis, done, device_error_flag());
+  return cudaGetLastError();
+}
+
 // grid for a persistent launch: all resident CTAs, capped by the work
 template <int N, class A, bool EVEC, bool EN>
 int bk5_grid(int64_t n_cells, int shape) {
@@ -118,7 +170,7 @@ int bk5_grid(int64_t n_cells, int shape) {
                          EA * N * N, 0);
     }
   } else if (shape == SHAPE_TMA_ALT) {
-    if constexpr (EA > 0 && !EVEC) {
+    if constexpr (EA > 0 && !EVEC && LineShape<N, A>::E == 0) {
       E = EA;
       if (ps < 0)
         ps = ctas_per_sm(bk5_tma_kernel<N, EA, A, EN, AltMinBlocks<N, EA, A>::value>, EA * N * N,
@@ -128,10 +180,12 @@ int bk5_grid(int64_t n_cells, int shape) {
     E = ElemsPerCtaPt<N>::value;
     if (ps < 0) ps = ctas_per_sm(bk5_pt_kernel<N, ElemsPerCtaPt<N>::value, A, EVEC, EN>, E * N * N * N, 0);
   } else if (shape == SHAPE_TMA) {
-    constexpr int ET = ElemsPerCtaTma<N, A>::value;
-    E = ET;
-    if (ps < 0)
-      ps = ctas_per_sm(bk5_tma_kernel<N, ET, A, EN>, ET * N * N, TmaLayout<N, ET, A>::total);
+    if constexpr (!EVEC && LineShape<N, A>::E == 0) {
+      constexpr int ET = ElemsPerCtaTma<N, A>::value;
+      E = ET;
+      if (ps < 0)
+        ps = ctas_per_sm(bk5_tma_kernel<N, ET, A, EN>, ET * N * N, TmaLayout<N, ET, A>::total);
+    }
   } else {
     E = ElemsPerCta<N>::value;
     if (ps < 0) {
@@ -155,6 +209,19 @@ cudaError_t bk5_launch(int64_t n_cells, const uint32_t *map, const typename A::G
   int shape = kernel_shape(ArithClass<A>::value, N);
   if (shape == SHAPE_FX) shape = SHAPE_TMA;
   if (shape == SHAPE_FX_ALT) shape = SHAPE_TMA_ALT;
+  // the line kernel (even-odd bases: the operators' own, not every caller's matrix)
+  if constexpr (!EVEC && LineShape<N, A>::E > 0) {
+    if (shape == SHAPE_TMA || shape == SHAPE_TMA_ALT) {
+      if (basis.eo && !((reinterpret_cast<uintptr_t>(G) | reinterpret_cast<uintptr_t>(map)) & 15u)) {
+        using Sh = LineShape<N, A>;
+        using Alt = LineAlt<N, A>;
+        if (shape == SHAPE_TMA_ALT || n_cells <= (int64_t)Sh::E * Sh::MB * num_sms())
+          return line_run<N, A, Alt>(n_cells, map, G, src, dst, basis, grid_used, stream, done_flag);
+        return line_run<N, A, Sh>(n_cells, map, G, src, dst, basis, grid_used, stream, done_flag);
+      }
+      shape = SHAPE_COLUMN;
+    }
+  }
   // without an alternative cells-per-CTA instantiation (E-vector mode, other
   // arithmetic, large N) shapes 3 / 4 run as 0 / 2; bulk copies need 16-byte
   // aligned tiles: caller arrays that are not 16-byte aligned use the column
@@ -171,12 +238,13 @@ cudaError_t bk5_launch(int64_t n_cells, const uint32_t *map, const typename A::G
   if (n_cells <= 0) return cudaSuccess;
   constexpr int EA = AltElems<N, A>::value;
   constexpr int MBA = AltMinBlocks<N, EA, A>::value;
+  constexpr bool TMA = !EVEC && LineShape<N, A>::E == 0;  // the column kernel with bulk copies
   if (shape == SHAPE_COLUMN_ALT) {
     if constexpr (EA > 0 && !EVEC)
       bk5_kernel_mb<N, EA, A, EVEC, EN, MBA><<<grid, EA * N * N, 0, stream>>>(
           n_cells, map, G, src, dst, basis, partials, done_flag);
   } else if (shape == SHAPE_TMA_ALT) {
-    if constexpr (EA > 0 && !EVEC)
+    if constexpr (EA > 0 && TMA)
       bk5_tma_kernel<N, EA, A, EN, MBA><<<grid, EA * N * N, TmaLayout<N, EA, A>::total, stream>>>(
           n_cells, map, G, src, dst, basis, partials, done_flag, device_error_flag());
   } else if (shape == SHAPE_POINT) {
@@ -184,7 +252,7 @@ cudaError_t bk5_launch(int64_t n_cells, const uint32_t *map, const typename A::G
     bk5_pt_kernel<N, E, A, EVEC, EN><<<grid, E * N * N * N, 0, stream>>>(
         n_cells, map, G, src, dst, basis, partials, done_flag);
   } else if (shape == SHAPE_TMA) {
-    if constexpr (!EVEC) {
+    if constexpr (TMA) {
       constexpr int E = ElemsPerCtaTma<N, A>::value;
       bk5_tma_kernel<N, E, A, EN><<<grid, E * N * N, TmaLayout<N, E, A>::total, stream>>>(
           n_cells, map, G, src, dst, basis, partials, done_flag, device_error_flag());

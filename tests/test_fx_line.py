@@ -155,3 +155,45 @@ def test_interpolation_seams_of_both_kinds(p):
             got = mf.bk1_evector(p, db, dJ, du, torch.zeros_like(du), arith="df").cpu().numpy()
             want = oracle.bk1_evector(n, q, b, J, u)
             assert np.linalg.norm(got - want) <= 1e-12 * np.linalg.norm(want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("p", range(1, 9))
+def test_plain_line_kernels(p):
+    """FP32 (shapes 2 and 4) and FP64 operators on meshes of one cell, of odd cell counts that leave
+    partial batches and unaligned tiles, and of several batches a thread block."""
+    import ctypes
+
+    import torch
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import benchmarks_gb300 as mf
+    from benchmarks_gb300 import _abi
+    from oracle import oracle
+    L = mf.lib()
+    old = {a: ctypes.c_int() for a in (0, 2)}
+    for a in old:
+        L.mfgb_get_kernel_shape(a, p, ctypes.byref(old[a]))
+    big = {1: 60, 2: 44, 3: 34, 4: 30, 5: 26, 6: 22, 7: 20, 8: 18}[p]
+    try:
+        for cells in ((1, 1, 1), (3, 5, 3), (big, big - 1, big + 1)):
+            A = mf.LaplaceOperator(mf.BoxMesh(*cells, degree=p))
+            ref = oracle.BoxProblem(*cells, p, amplitude=0.05)
+            src = np.random.default_rng(p).uniform(-1, 1, ref.n_dofs)
+            want = ref.apply(src)
+            u64 = torch.from_numpy(src).cuda()
+            for shape in (2, 4):
+                for a, dt, bound in ((0, torch.float64, 1e-12), (2, torch.float32, 1e-5)):
+                    _abi.check(L.mfgb_set_kernel_shape(a, p, shape))
+                    u = u64.to(dt)
+                    y = torch.zeros_like(u)
+                    ptr = [ctypes.c_void_p(t.data_ptr()) for t in (y, u)]
+                    _abi.check(L.mfgb_vmult_f32(A.handle, *ptr, None) if a == 2 else
+                               L.mfgb_vmult(A.handle, *ptr, 0, None))
+                    torch.cuda.synchronize()
+                    mf.check_device_errors()
+                    got = y.double().cpu().numpy()
+                    assert np.linalg.norm(got - want) <= bound * np.linalg.norm(want), (cells, shape, a)
+    finally:
+        for a, v in old.items():
+            L.mfgb_set_kernel_shape(a, p, v.value)
