@@ -83,10 +83,13 @@ __global__ void kb_offset_i64(int64_t n, const int64_t *__restrict__ src, int64_
 }
 
 // ---- batched Chebyshev (FP32), coefficients per part: [1/theta, c1_1, c2_1, ...]
+// (every consumer of an operator result zeroes it for the next application and takes the
+// constrained rows from the operator's input, mfgb_mg_kernels.cuh)
 __global__ void __launch_bounds__(T256)
     kb_cheb_first_zero(const Chunk *__restrict__ ch, const float *__restrict__ b,
                        const float *__restrict__ dinv, float *__restrict__ x, float *__restrict__ d,
-                       float *__restrict__ r, const float *__restrict__ coef, int cs) {
+                       float *__restrict__ r, float *__restrict__ tz, const float *__restrict__ coef,
+                       int cs) {
   const float it = coef[(int64_t)ch[blockIdx.x].part * cs];
   CHUNK_LOOP(c, t) {
     const float bt = b[t];
@@ -94,48 +97,59 @@ __global__ void __launch_bounds__(T256)
     r[t] = bt;
     d[t] = dt;
     x[t] = dt;
+    tz[t] = 0.f;
   }
 }
 
 __global__ void __launch_bounds__(T256)
-    kb_cheb_first(const Chunk *__restrict__ ch, const float *__restrict__ b,
-                  const float *__restrict__ ax, const float *__restrict__ dinv, float *__restrict__ x,
-                  float *__restrict__ d, float *__restrict__ r, const float *__restrict__ coef,
-                  int cs) {
+    kb_cheb_first(const Chunk *__restrict__ ch, const float *__restrict__ b, float *__restrict__ ax,
+                  const float *__restrict__ dinv, float *__restrict__ x, float *__restrict__ d,
+                  float *__restrict__ r, const uint32_t *__restrict__ bits,
+                  const float *__restrict__ coef, int cs) {
   const float it = coef[(int64_t)ch[blockIdx.x].part * cs];
   CHUNK_LOOP(c, t) {
-    const float rt = b[t] - ax[t];
+    const float xt = x[t], rt = b[t] - (bit_at(bits, t) ? xt : ax[t]);
     const float dt = it * dinv[t] * rt;
     r[t] = rt;
     d[t] = dt;
-    x[t] += dt;
+    x[t] = xt + dt;
+    ax[t] = 0.f;
   }
 }
 
 __global__ void __launch_bounds__(T256)
-    kb_cheb_step(const Chunk *__restrict__ ch, const float *__restrict__ ad,
+    kb_cheb_step(const Chunk *__restrict__ ch, float *__restrict__ ad,
                  const float *__restrict__ dinv, float *__restrict__ x, float *__restrict__ d,
-                 float *__restrict__ r, const float *__restrict__ coef, int cs, int j) {
+                 float *__restrict__ r, const uint32_t *__restrict__ bits,
+                 const float *__restrict__ coef, int cs, int j) {
   const float *cf = coef + (int64_t)ch[blockIdx.x].part * cs;
   const float c1 = cf[2 * j - 1], c2 = cf[2 * j];
   CHUNK_LOOP(c, t) {
-    const float rt = r[t] - ad[t];
-    const float dt = c1 * d[t] + c2 * dinv[t] * rt;
+    const float dv = d[t], rt = r[t] - (bit_at(bits, t) ? dv : ad[t]);
+    const float dt = c1 * dv + c2 * dinv[t] * rt;
     r[t] = rt;
     d[t] = dt;
     x[t] += dt;
+    ad[t] = 0.f;
   }
 }
 
 __global__ void __launch_bounds__(T256)
-    kb_residual(const Chunk *__restrict__ ch, const float *__restrict__ b,
-                const float *__restrict__ ax, float *__restrict__ r) {
-  CHUNK_LOOP(c, t) r[t] = b[t] - ax[t];
+    kb_residual(const Chunk *__restrict__ ch, const float *__restrict__ b, float *__restrict__ ax,
+                const float *__restrict__ x, const uint32_t *__restrict__ bits,
+                float *__restrict__ r) {
+  CHUNK_LOOP(c, t) {
+    r[t] = b[t] - (bit_at(bits, t) ? x[t] : ax[t]);
+    ax[t] = 0.f;
+  }
 }
 
 __global__ void __launch_bounds__(T256)
-    kb_add(const Chunk *__restrict__ ch, const float *__restrict__ t_, float *__restrict__ x) {
-  CHUNK_LOOP(c, t) x[t] += t_[t];
+    kb_add_clear(const Chunk *__restrict__ ch, float *__restrict__ t_, float *__restrict__ x) {
+  CHUNK_LOOP(c, t) {
+    x[t] += t_[t];
+    t_[t] = 0.f;
+  }
 }
 
 __global__ void __launch_bounds__(T256)
@@ -235,20 +249,18 @@ __device__ __forceinline__ double problem_sum(const int *__restrict__ cbeg,
   return cta_sum(s, sh);
 }
 
-__global__ void __launch_bounds__(T256)
-    kb_sum_pap(const int *__restrict__ cbeg, const int *__restrict__ pid,
-               const double *__restrict__ part, BScal *__restrict__ sc) {
-  __shared__ double sh[T256 / 32];
-  const double s = problem_sum(cbeg, part, sh);
-  if (threadIdx.x == 0) sc[pid[blockIdx.x]].pap = s;
-}
-
-__global__ void __launch_bounds__(T256)
-    kb_sum_rz(const int *__restrict__ cbeg, const int *__restrict__ pid,
-              const double *__restrict__ part, BScal *__restrict__ sc) {
-  __shared__ double sh[T256 / 32];
-  const double s = problem_sum(cbeg, part, sh);
-  if (threadIdx.x == 0) sc[pid[blockIdx.x]].rz_new = s;
+// the same in every CTA of a chunk kernel, for the chunk's own problem (range: its chunks)
+__device__ __forceinline__ double chunk_problem_sum(const int2 range, const double *__restrict__ part,
+                                                    double *sh) {
+  double s = 0;
+  for (int i = range.x + threadIdx.x; i < range.y; i += blockDim.x) s += part[i];
+  s = cta_sum(s, sh);
+  __syncthreads();
+  if (threadIdx.x == 0) sh[0] = s;
+  __syncthreads();
+  s = sh[0];
+  __syncthreads();
+  return s;
 }
 
 // initial residual norms: tol_eff = max(tol, reduce |r0|)
@@ -263,31 +275,80 @@ __global__ void __launch_bounds__(T256)
     q.res0 = q.res = res;
     q.tol_eff = fmax(tol, reduce * res);
     q.its = 0;
+    q.rz = INFINITY;  // no previous direction: beta = 0
     q.done = isnan(res) ? 2 : (res <= q.tol_eff ? 1 : 0);
   }
 }
 
-__global__ void kb_init_rz(int n, BScal *__restrict__ sc) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p < n) sc[p].rz = sc[p].rz_new;
+// The outer iteration: each chunk's CTA sums the partials of its problem from the pass before, so no
+// launch is spent on sums; the V-cycle's z stays in FP32 and r is stored for it by the update.
+__global__ void __launch_bounds__(T256)
+    kb_rz(const Chunk *__restrict__ ch, const double *__restrict__ r, const float *__restrict__ z,
+          double *__restrict__ part) {
+  __shared__ double sh[T256 / 32];
+  double s = 0;
+  CHUNK_LOOP(c, t) s = fma(r[t], (double)z[t], s);
+  s = cta_sum(s, sh);
+  if (threadIdx.x == 0) part[blockIdx.x] = s;
 }
 
-// x += alpha p; r -= alpha v (alpha = rz / pAp); per-chunk |r|^2
+// p = z + beta p (beta = r.z / previous r.z) for running problems; v = 0 with p on the constrained
+// rows, ready for v += A p
 __global__ void __launch_bounds__(T256)
-    kb_update(const Chunk *__restrict__ ch, double *__restrict__ x, double *__restrict__ r,
-              const double *__restrict__ p, const double *__restrict__ v,
-              const BScal *__restrict__ sc, double *__restrict__ part) {
+    kb_direction(const Chunk *__restrict__ ch, const int2 *__restrict__ range,
+                 const float *__restrict__ z, double *__restrict__ p, double *__restrict__ v,
+                 const uint32_t *__restrict__ bits, const double *__restrict__ part,
+                 BScal *__restrict__ sc) {
   __shared__ double sh[T256 / 32];
-  const BScal &q = sc[ch[blockIdx.x].part];
+  const int pr = ch[blockIdx.x].part;
+  BScal &q = sc[pr];
+  const int2 rg = range[pr];
+  const bool run = !q.done;
+  double beta = 0.0;
+  if (run) {
+    const double rz = chunk_problem_sum(rg, part, sh);
+    beta = rz / q.rz;
+    if ((int)blockIdx.x == rg.x && threadIdx.x == 0) q.rz_new = rz;
+  }
+  CHUNK_LOOP(c, t) {
+    double pt = p[t];
+    if (run) p[t] = pt = fma(beta, pt, (double)z[t]);
+    v[t] = bit_at(bits, t) ? pt : 0.0;
+  }
+}
+
+// per-chunk p.v; the new r.z becomes the current one
+__global__ void __launch_bounds__(T256)
+    kb_pv(const Chunk *__restrict__ ch, const int2 *__restrict__ range, const double *__restrict__ p,
+          const double *__restrict__ v, double *__restrict__ part, BScal *__restrict__ sc) {
+  __shared__ double sh[T256 / 32];
+  const int pr = ch[blockIdx.x].part;
+  if (sc[pr].done) return;
+  if ((int)blockIdx.x == range[pr].x && threadIdx.x == 0) sc[pr].rz = sc[pr].rz_new;
   double s = 0;
-  if (!q.done) {
-    const double alpha = q.rz / q.pap;
-    CHUNK_LOOP(c, t) {
-      x[t] = fma(alpha, p[t], x[t]);
-      const double rt = fma(-alpha, v[t], r[t]);
-      r[t] = rt;
-      s = fma(rt, rt, s);
-    }
+  CHUNK_LOOP(c, t) s = fma(p[t], v[t], s);
+  s = cta_sum(s, sh);
+  if (threadIdx.x == 0) part[blockIdx.x] = s;
+}
+
+// x += alpha p; r -= alpha v (alpha = r.z / p.v); b = r in FP32; per-chunk |r|^2
+__global__ void __launch_bounds__(T256)
+    kb_update(const Chunk *__restrict__ ch, const int2 *__restrict__ range, double *__restrict__ x,
+              double *__restrict__ r, const double *__restrict__ p, const double *__restrict__ v,
+              float *__restrict__ b, const double *__restrict__ pv, const BScal *__restrict__ sc,
+              double *__restrict__ part) {
+  __shared__ double sh[T256 / 32];
+  const int pr = ch[blockIdx.x].part;
+  const BScal &q = sc[pr];
+  if (q.done) return;
+  const double alpha = q.rz / chunk_problem_sum(range[pr], pv, sh);
+  double s = 0;
+  CHUNK_LOOP(c, t) {
+    x[t] = fma(alpha, p[t], x[t]);
+    const double rt = fma(-alpha, v[t], r[t]);
+    r[t] = rt;
+    b[t] = (float)rt;
+    s = fma(rt, rt, s);
   }
   s = cta_sum(s, sh);
   if (threadIdx.x == 0) part[blockIdx.x] = s;
@@ -337,30 +398,10 @@ __global__ void kb_continue(cudaGraphConditionalHandle h, const int *active,
   cudaGraphSetConditional(h, (*active > 0 && *active_dofs > threshold && it < max_iter) ? 1u : 0u);
 }
 
-// p = z + beta p (beta = rz_new / rz) for running problems
-__global__ void __launch_bounds__(T256)
-    kb_direction(const Chunk *__restrict__ ch, const double *__restrict__ z, double *__restrict__ p,
-                 const BScal *__restrict__ sc) {
-  const BScal &q = sc[ch[blockIdx.x].part];
-  if (q.done) return;
-  const double beta = q.rz_new / q.rz;
-  CHUNK_LOOP(c, t) p[t] = fma(beta, p[t], z[t]);
-}
-
-__global__ void kb_roll(int n, BScal *__restrict__ sc) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p < n && !sc[p].done) sc[p].rz = sc[p].rz_new;
-}
-
 __global__ void __launch_bounds__(T256)
     kb_residual64(const Chunk *__restrict__ ch, const double *__restrict__ b,
                   const double *__restrict__ v, double *__restrict__ r) {
   CHUNK_LOOP(c, t) r[t] = b[t] - v[t];
-}
-
-__global__ void __launch_bounds__(T256)
-    kb_copy64(const Chunk *__restrict__ ch, const double *__restrict__ a, double *__restrict__ b) {
-  CHUNK_LOOP(c, t) b[t] = a[t];
 }
 
 // ---- host-side structures -------------------------------------------------
@@ -405,6 +446,7 @@ struct Plan {
   const Chunk *d_all = nullptr;  // outer CG chunks (depth 0)
   int n_all = 0;
   const int *d_cbeg = nullptr, *d_pid = nullptr;
+  const int2 *d_range = nullptr;  // per problem: its chunks in d_all
   int n_prob = 0;
   int64_t dofs = 0;              // depth-0 DoFs of its problems
   bool owns = false;             // a gathered plan owns what it points to
@@ -424,6 +466,7 @@ struct Depth {
   Chunk *d_pch = nullptr;    // parts with a p-transfer to depth+1
   int n_pch = 0;
   float *d_coef = nullptr;   // [parts][cs]
+  uint32_t *bits = nullptr;  // one bit per DoF: constrained
   std::vector<PGroup> pgroups;
   HPart *d_hp = nullptr;
   Chunk *d_hfine = nullptr;  // fine nodes of h-transfer parts (this depth)
@@ -512,6 +555,7 @@ struct mfgb_batch {
   mfgb::Chunk *d_all = nullptr;
   int n_all = 0;
   int *d_cbeg = nullptr, *d_pid = nullptr;
+  int2 *d_range = nullptr;
   mfgb::Plan full;
   double *r = nullptr, *z = nullptr, *p = nullptr, *v = nullptr, *part = nullptr;
   mfgb::BScal *d_scal = nullptr;
@@ -536,10 +580,11 @@ void free_batch(mfgb_batch *B) {
     for (auto &pg : D.pgroups) cudaFree(pg.map_c);
     cudaFree(D.d_cons); cudaFree(D.x); cudaFree(D.b); cudaFree(D.r); cudaFree(D.d); cudaFree(D.t);
     cudaFree(D.inv_diag); cudaFree(D.inv_val); cudaFree(D.d_cheb); cudaFree(D.d_pch);
-    cudaFree(D.d_coef); cudaFree(D.d_hp); cudaFree(D.d_hfine); cudaFree(D.d_hcoarse);
+    cudaFree(D.d_coef); cudaFree(D.bits); cudaFree(D.d_hp); cudaFree(D.d_hfine); cudaFree(D.d_hcoarse);
   }
   cudaFree(B->d_coarse); cudaFree(B->d_Ainv); cudaFree(B->d_cids);
   cudaFree(B->d_all); cudaFree(B->d_cbeg); cudaFree(B->d_pid);
+  cudaFree(B->d_range);
   cudaFree(B->r); cudaFree(B->z); cudaFree(B->p); cudaFree(B->v); cudaFree(B->part);
   cudaFree(B->d_scal); cudaFree(B->d_active);
   cudaFree(B->d_pdofs); cudaFree(B->d_active_dofs); cudaFree(B->d_iter);
@@ -583,6 +628,60 @@ mfgb_status apply32(const Depth &V, const DepthPlan &D, const float *src, float 
   return cuda_status(cudaGetLastError(), "batch A32 constrained");
 }
 
+// Streams that run the degrees of one depth side by side: their kernels touch different problems,
+// and on small batches one alone leaves most of the GPU idle.  Used while a solve's iteration is
+// captured; elsewhere (br == nullptr) the degrees run one after another on the caller's stream.
+struct Branches {
+  static constexpr int MAX = 7;
+  cudaStream_t aux[MAX] = {};
+  cudaEvent_t fork = nullptr, done[MAX] = {};
+  mfgb_status init() {
+    cudaError_t e = cudaEventCreateWithFlags(&fork, cudaEventDisableTiming);
+    for (int k = 0; k < MAX && e == cudaSuccess; ++k) {
+      e = cudaStreamCreateWithFlags(&aux[k], cudaStreamNonBlocking);
+      if (e == cudaSuccess) e = cudaEventCreateWithFlags(&done[k], cudaEventDisableTiming);
+    }
+    return cuda_status(e, "batch streams");
+  }
+  ~Branches() {
+    for (int k = 0; k < MAX; ++k) {
+      if (done[k]) cudaEventDestroy(done[k]);
+      if (aux[k]) cudaStreamDestroy(aux[k]);
+    }
+    if (fork) cudaEventDestroy(fork);
+  }
+};
+
+// f(k, stream) for k = 0..n-1, side by side where br is given; s continues after all of them
+template <class F>
+mfgb_status side_by_side(Branches *br, size_t n, cudaStream_t s, F f) {
+  mfgb_status st = MFGB_OK;
+  const size_t side = br && n > 1 ? std::min<size_t>(n - 1, Branches::MAX) : 0;
+  if (side) cudaEventRecord(br->fork, s);
+  for (size_t k = 0; k < n && !st; ++k) {
+    const size_t b = side ? k % (side + 1) : 0;  // branch 0 is s itself
+    const cudaStream_t q = b ? br->aux[b - 1] : s;
+    if (b && k < side + 1) cudaStreamWaitEvent(q, br->fork, 0);
+    st = f(k, q);
+  }
+  for (size_t b = 0; b < side; ++b) {
+    cudaEventRecord(br->done[b], br->aux[b]);
+    cudaStreamWaitEvent(s, br->done[b], 0);
+  }
+  return st;
+}
+
+// t += A src on the unconstrained rows of one depth (FP32); t enters zero
+mfgb_status level_apply(const Depth &V, const DepthPlan &D, const float *src, cudaStream_t s,
+                        Branches *br) {
+  return side_by_side(br, D.groups.size(), s, [&](size_t k, cudaStream_t q) {
+    const mfgb_operator *op = D.groups[k];
+    return cuda_status(bk5_f32(op->n, op->n_cells, op->d_map, op->d_G32, src, V.t, op->D, nullptr,
+                               nullptr, q),
+                       "batch A32 kernel");
+  });
+}
+
 // dst = A src on depth 0 in FP64 (double-float union operators)
 mfgb_status apply64(const mfgb_batch *B, const Plan &P, const double *src, double *dst,
                     cudaStream_t s) {
@@ -597,27 +696,27 @@ mfgb_status apply64(const mfgb_batch *B, const Plan &P, const double *src, doubl
 }
 
 mfgb_status chebyshev_b(const mfgb_batch *B, const Depth &V, const DepthPlan &D, bool zero_start,
-                        cudaStream_t s) {
+                        cudaStream_t s, Branches *br) {
   mfgb_status st;
   if (zero_start) {
-    kb_cheb_first_zero<<<D.n_cheb, T256, 0, s>>>(D.d_cheb, V.b, V.inv_diag, V.x, V.d, V.r,
+    kb_cheb_first_zero<<<D.n_cheb, T256, 0, s>>>(D.d_cheb, V.b, V.inv_diag, V.x, V.d, V.r, V.t,
                                                  V.d_coef, B->cs);
   } else {
-    if ((st = apply32(V, D, V.x, V.t, s))) return st;
-    kb_cheb_first<<<D.n_cheb, T256, 0, s>>>(D.d_cheb, V.b, V.t, V.inv_diag, V.x, V.d, V.r,
+    if ((st = level_apply(V, D, V.x, s, br))) return st;
+    kb_cheb_first<<<D.n_cheb, T256, 0, s>>>(D.d_cheb, V.b, V.t, V.inv_diag, V.x, V.d, V.r, V.bits,
                                             V.d_coef, B->cs);
   }
   for (int j = 1; j < B->cheb_degree; ++j) {
-    if ((st = apply32(V, D, V.d, V.t, s))) return st;
-    kb_cheb_step<<<D.n_cheb, T256, 0, s>>>(D.d_cheb, V.t, V.inv_diag, V.x, V.d, V.r, V.d_coef,
-                                           B->cs, j);
+    if ((st = level_apply(V, D, V.d, s, br))) return st;
+    kb_cheb_step<<<D.n_cheb, T256, 0, s>>>(D.d_cheb, V.t, V.inv_diag, V.x, V.d, V.r, V.bits,
+                                           V.d_coef, B->cs, j);
   }
   return cuda_status(cudaGetLastError(), "batch chebyshev");
 }
 
 // depth-0 x = V(b): descend every depth the plan's problems reach, all coarse
 // solves, ascend
-mfgb_status vcycle_b(const mfgb_batch *B, const Plan &P, cudaStream_t s) {
+mfgb_status vcycle_b(const mfgb_batch *B, const Plan &P, cudaStream_t s, Branches *br = nullptr) {
   size_t nd = 1;
   for (size_t l = 0; l < P.depth.size(); ++l)
     if (P.depth[l].n_cheb) nd = l + 2;  // depth l smooths, so depth l + 1 exists
@@ -627,18 +726,24 @@ mfgb_status vcycle_b(const mfgb_batch *B, const Plan &P, cudaStream_t s) {
     const Depth &V = B->depth[l], &C = B->depth[l + 1];
     const DepthPlan &D = P.depth[l];
     if (!D.n_cheb) continue;
-    if ((st = chebyshev_b(B, V, D, true, s))) return st;
-    if ((st = apply32(V, D, V.x, V.t, s))) return st;
-    kb_residual<<<D.n_cheb, T256, 0, s>>>(D.d_cheb, V.b, V.t, V.r);
+    if ((st = chebyshev_b(B, V, D, true, s, br))) return st;
+    if ((st = level_apply(V, D, V.x, s, br))) return st;
+    kb_residual<<<D.n_cheb, T256, 0, s>>>(D.d_cheb, V.b, V.t, V.x, V.bits, V.r);
     if ((st = cuda_status(cudaMemsetAsync(C.b, 0, sizeof(float) * C.n, s), "batch coarse b = 0")))
       return st;
-    for (const PGroup &pg : D.pgroups) {
-      const mfgb_operator *op = D.groups[pg.g];
-      p_transfer<float>(true, op->n_cells, op->d_map, pg.map_c, V.r, V.inv_val, C.b, pg.P, s);
-    }
-    if (D.n_hcoarse)
-      kb_h_restrict<<<D.n_hcoarse, T256, 0, s>>>(D.d_hcoarse, D.d_hp, V.r, C.b);
-    if ((st = cuda_status(cudaGetLastError(), "batch restrict"))) return st;
+    // the p-transfers of each degree and the h-transfers
+    const size_t np = D.pgroups.size();
+    if ((st = side_by_side(br, np + (D.n_hcoarse > 0), s, [&](size_t k, cudaStream_t q) {
+           if (k < np) {
+             const PGroup &pg = D.pgroups[k];
+             const mfgb_operator *op = D.groups[pg.g];
+             p_transfer<float>(true, op->n_cells, op->d_map, pg.map_c, V.r, V.inv_val, C.b, pg.P, q);
+           } else {
+             kb_h_restrict<<<D.n_hcoarse, T256, 0, q>>>(D.d_hcoarse, D.d_hp, V.r, C.b);
+           }
+           return cuda_status(cudaGetLastError(), "batch restrict");
+         })))
+      return st;
   }
   if (P.n_coarse)
     kb_coarse<<<P.n_coarse, T256, P.coarse_smem, s>>>(P.d_coarse);
@@ -647,18 +752,21 @@ mfgb_status vcycle_b(const mfgb_batch *B, const Plan &P, cudaStream_t s) {
     const Depth &V = B->depth[l], &C = B->depth[l + 1];
     const DepthPlan &D = P.depth[l];
     if (!D.n_cheb) continue;
-    if (!D.pgroups.empty()) {
-      if ((st = cuda_status(cudaMemsetAsync(V.t, 0, sizeof(float) * V.n, s), "batch t = 0")))
-        return st;
-      for (const PGroup &pg : D.pgroups) {
-        const mfgb_operator *op = D.groups[pg.g];
-        p_transfer<float>(false, op->n_cells, op->d_map, pg.map_c, C.x, nullptr, V.t, pg.P, s);
-      }
-      kb_add<<<D.n_pch, T256, 0, s>>>(D.d_pch, V.t, V.x);
-    }
-    if (D.n_hfine) kb_h_prolongate_add<<<D.n_hfine, T256, 0, s>>>(D.d_hfine, D.d_hp, C.x, V.x);
-    if ((st = cuda_status(cudaGetLastError(), "batch prolongate"))) return st;
-    if ((st = chebyshev_b(B, V, D, false, s))) return st;
+    // V.t is zero (its last consumer cleared it)
+    const size_t np = D.pgroups.size();
+    if ((st = side_by_side(br, np + (D.n_hfine > 0), s, [&](size_t k, cudaStream_t q) {
+           if (k < np) {
+             const PGroup &pg = D.pgroups[k];
+             const mfgb_operator *op = D.groups[pg.g];
+             p_transfer<float>(false, op->n_cells, op->d_map, pg.map_c, C.x, nullptr, V.t, pg.P, q);
+           } else {
+             kb_h_prolongate_add<<<D.n_hfine, T256, 0, q>>>(D.d_hfine, D.d_hp, C.x, V.x);
+           }
+           return cuda_status(cudaGetLastError(), "batch prolongate");
+         })))
+      return st;
+    if (np) kb_add_clear<<<D.n_pch, T256, 0, s>>>(D.d_pch, V.t, V.x);
+    if ((st = chebyshev_b(B, V, D, false, s, br))) return st;
   }
   return MFGB_OK;
 }
@@ -801,6 +909,7 @@ mfgb_status gather_plan(const mfgb_batch *B, const std::vector<char> &active, Pl
   std::vector<CoarseDesc> cd;
   std::vector<Chunk> all;
   std::vector<int> cbeg, pid;
+  std::vector<int2> range(B->n_problems, int2{0, 0});
   for (int i = 0; i < B->n_problems; ++i) {
     if (!active[i]) continue;
     cd.push_back(B->coarse_host[i]);
@@ -808,16 +917,19 @@ mfgb_status gather_plan(const mfgb_batch *B, const std::vector<char> &active, Pl
     cbeg.push_back((int)all.size());
     pid.push_back(i);
     append_chunks(all, Q.off, Q.n, part_at[i][0]);
+    range[i] = int2{cbeg.back(), (int)all.size()};
     P.dofs += Q.n;
   }
   cbeg.push_back((int)all.size());
   CoarseDesc *dcd = nullptr;
   Chunk *dall = nullptr;
   int *dcb = nullptr, *dpid = nullptr;
-  if ((st = upload(&dcd, cd)) || (st = upload(&dall, all)) || (st = upload(&dcb, cbeg)) ||
-      (st = upload(&dpid, pid)))
-    return fail(st);
-  track(dcd); track(dall); track(dcb); track(dpid);
+  int2 *drange = nullptr;
+  (st = upload(&dcd, cd)) || (st = upload(&dall, all)) || (st = upload(&dcb, cbeg)) ||
+      (st = upload(&dpid, pid)) || (st = upload(&drange, range));
+  track(dcd); track(dall); track(dcb); track(dpid); track(drange);
+  if (st) return fail(st);
+  P.d_range = drange;
   P.d_coarse = dcd;
   P.n_coarse = (int)cd.size();
   P.coarse_smem = B->full.coarse_smem;
@@ -969,18 +1081,22 @@ mfgb_status build_batch(mfgb_batch *B, const mfgb_box_desc *boxes, int n,
     const Depth &D = B->depth[0];
     std::vector<Chunk> all;
     std::vector<int> cbeg;
+    std::vector<int2> range;  // (depth 0: part k is problem k)
     for (size_t k = 0; k < D.parts.size(); ++k) {
       cbeg.push_back((int)all.size());
       append_chunks(all, D.parts[k].off, D.parts[k].n, (int)k);
+      range.push_back(int2{cbeg.back(), (int)all.size()});
     }
     cbeg.push_back((int)all.size());
     B->n_all = (int)all.size();
-    if ((st = upload(&B->d_all, all)) || (st = upload(&B->d_cbeg, cbeg))) return st;
+    if ((st = upload(&B->d_all, all)) || (st = upload(&B->d_cbeg, cbeg)) ||
+        (st = upload(&B->d_range, range)))
+      return st;
     if ((st = dalloc((void **)&B->r, sizeof(double) * D.n)) ||
         (st = dalloc((void **)&B->z, sizeof(double) * D.n)) ||
         (st = dalloc((void **)&B->p, sizeof(double) * D.n)) ||
         (st = dalloc((void **)&B->v, sizeof(double) * D.n)) ||
-        (st = dalloc((void **)&B->part, sizeof(double) * std::max(1, B->n_all))) ||
+        (st = dalloc((void **)&B->part, sizeof(double) * 3 * std::max(1, B->n_all))) ||
         (st = dalloc((void **)&B->d_scal, sizeof(BScal) * n)) ||
         (st = dalloc((void **)&B->d_active, sizeof(int))) ||
         (st = dalloc((void **)&B->d_active_dofs, sizeof(unsigned long long))) ||
@@ -1092,6 +1208,14 @@ mfgb_status build_batch(mfgb_batch *B, const mfgb_box_desc *boxes, int n,
     }
     if ((st = cuda_status(cudaDeviceSynchronize(), "batch copy"))) return st;
   }
+  // ---- constrained bits of every depth ---------------------------------------
+  for (Depth &D : B->depth) {
+    const size_t bytes = sizeof(uint32_t) * ((D.n + 31) / 32);
+    if ((st = dalloc((void **)&D.bits, bytes)) ||
+        (st = cuda_status(cudaMemset(D.bits, 0, bytes), "batch bits")))
+      return st;
+    if (D.n_cons) k_set_bits<<<grid1d(D.n_cons), T256>>>(D.n_cons, D.d_cons, D.bits);
+  }
   // ---- lambda_max of every smoothed part: one power iteration per depth -----
   // over all its parts (the start, normalisation, FP32 operator, constrained
   // rows and Jacobi scaling of the single-problem estimate)
@@ -1199,6 +1323,7 @@ mfgb_status build_batch(mfgb_batch *B, const mfgb_box_desc *boxes, int n,
   F.d_all = B->d_all;
   F.n_all = B->n_all;
   F.d_cbeg = B->d_cbeg;
+  F.d_range = B->d_range;
   F.d_pid = B->d_pid;
   F.n_prob = n;
   F.dofs = B->depth[0].n;
@@ -1363,19 +1488,20 @@ mfgb_status mfgb_batch_cg_solve(mfgb_batch *B, const double *d_b, double *d_x,
   if (st) return st;
   struct J { cudaStream_t s; void *o; ~J() { join_stream(s, o); } } join{s, stream};
   const int np = B->n_problems;
-  const unsigned gp = (unsigned)((np + 127) / 128);
   const Plan &F = B->full;
-  // r = b - A x; |r0|; z = M r; p = z; rz
+  // r = b - A x; |r0|; the V-cycle's right-hand side; p = 0 and an infinite previous r.z (kb_init)
+  // before the first direction
   if ((st = apply64(B, F, d_x, B->v, s))) return st;
   kb_residual64<<<F.n_all, T256, 0, s>>>(F.d_all, d_b, B->v, B->r);
   kb_dot<<<F.n_all, T256, 0, s>>>(F.d_all, B->r, B->r, B->part);
   kb_init<<<np, T256, 0, s>>>(F.d_cbeg, F.d_pid, B->part, B->d_scal, ctl->tol, ctl->reduce);
-  if ((st = precondition_b(B, F, B->z, B->r, s))) return st;
-  kb_copy64<<<F.n_all, T256, 0, s>>>(F.d_all, B->z, B->p);
-  kb_dot<<<F.n_all, T256, 0, s>>>(F.d_all, B->r, B->z, B->part);
-  kb_sum_rz<<<np, T256, 0, s>>>(F.d_cbeg, F.d_pid, B->part, B->d_scal);
-  kb_init_rz<<<gp, 128, 0, s>>>(np, B->d_scal);
-  if ((st = cuda_status(cudaGetLastError(), "batch cg init"))) return st;
+  const Depth &V0 = B->depth[0];
+  k_convert<float, double><<<grid1d(V0.n), T256, 0, s>>>(V0.n, B->r, V0.b);
+  if ((st = cuda_status(cudaMemsetAsync(B->p, 0, sizeof(double) * V0.n, s), "batch p = 0")) ||
+      (st = cuda_status(cudaGetLastError(), "batch cg init")))
+    return st;
+  Branches br;
+  if ((st = br.init())) return st;
   std::vector<BScal> hs(np);
   auto read_scalars = [&]() {
     mfgb_status e = cuda_status(cudaMemcpyAsync(hs.data(), B->d_scal, sizeof(BScal) * np,
@@ -1388,26 +1514,27 @@ mfgb_status mfgb_batch_cg_solve(mfgb_batch *B, const double *d_b, double *d_x,
   int running = 0;
   for (const BScal &q : hs) running += q.done == 0;
 
-  // one CG iteration of the plan's problems, issued on s (in capture)
+  // one CG iteration of the plan's problems, issued on s (in capture): V-cycle, direction, operator,
+  // update.  The V-cycle comes first, so none is spent on residuals that end a solve.
+  double *part_rz = B->part, *part_pv = part_rz + B->n_all, *part_rr = part_pv + B->n_all;
   auto iteration = [&](const Plan &P) -> mfgb_status {
-    const int nb = P.n_prob;
-    mfgb_status cap = apply64(B, P, B->p, B->v, s);
-    if (!cap) {
-      kb_dot<<<P.n_all, T256, 0, s>>>(P.d_all, B->p, B->v, B->part);
-      kb_sum_pap<<<nb, T256, 0, s>>>(P.d_cbeg, P.d_pid, B->part, B->d_scal);
-      kb_update<<<P.n_all, T256, 0, s>>>(P.d_all, d_x, B->r, B->p, B->v, B->d_scal, B->part);
-      kb_zero_active<<<1, 1, 0, s>>>(B->d_active, B->d_active_dofs);
-      kb_sum_check<<<nb, T256, 0, s>>>(P.d_cbeg, P.d_pid, B->part, B->d_scal, ctl->max_steps,
-                                       B->d_active, B->d_pdofs, B->d_active_dofs);
-      cap = precondition_b(B, P, B->z, B->r, s);
-    }
-    if (!cap) {
-      kb_dot<<<P.n_all, T256, 0, s>>>(P.d_all, B->r, B->z, B->part);
-      kb_sum_rz<<<nb, T256, 0, s>>>(P.d_cbeg, P.d_pid, B->part, B->d_scal);
-      kb_direction<<<P.n_all, T256, 0, s>>>(P.d_all, B->z, B->p, B->d_scal);
-      kb_roll<<<gp, 128, 0, s>>>(np, B->d_scal);
-    }
-    return cap;
+    mfgb_status e = vcycle_b(B, P, s, &br);
+    if (e) return e;
+    kb_rz<<<P.n_all, T256, 0, s>>>(P.d_all, B->r, V0.x, part_rz);
+    kb_direction<<<P.n_all, T256, 0, s>>>(P.d_all, P.d_range, V0.x, B->p, B->v, V0.bits, part_rz,
+                                          B->d_scal);
+    const DepthPlan &D = P.depth[0];
+    e = side_by_side(&br, D.groups.size(), s, [&](size_t k, cudaStream_t q) {
+      return apply_add_impl(D.groups[k], B->v, B->p, MFGB_ARITH_FP64_DF, q, nullptr);
+    });
+    if (e) return e;
+    kb_pv<<<P.n_all, T256, 0, s>>>(P.d_all, P.d_range, B->p, B->v, part_pv, B->d_scal);
+    kb_update<<<P.n_all, T256, 0, s>>>(P.d_all, P.d_range, d_x, B->r, B->p, B->v, V0.b, part_pv,
+                                       B->d_scal, part_rr);
+    kb_zero_active<<<1, 1, 0, s>>>(B->d_active, B->d_active_dofs);
+    kb_sum_check<<<P.n_prob, T256, 0, s>>>(P.d_cbeg, P.d_pid, part_rr, B->d_scal, ctl->max_steps,
+                                           B->d_active, B->d_pdofs, B->d_active_dofs);
+    return cuda_status(cudaGetLastError(), "batch cg iteration");
   };
   // The plan's iterations as one graph: a conditional while node whose body is
   // one iteration plus the condition kernel (kb_continue), so one launch runs

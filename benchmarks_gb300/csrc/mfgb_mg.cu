@@ -142,35 +142,119 @@ __global__ void __launch_bounds__(T256)
   if (threadIdx.x == 0) *out = s;
 }
 
-// x += alpha p; r -= alpha v; alpha = scal[0] / scal[1]; partial |r|^2
-__global__ void __launch_bounds__(T256)
-    k_pcg_update(int64_t n, double *__restrict__ x, double *__restrict__ r,
-                 const double *__restrict__ p, const double *__restrict__ v,
-                 const double *__restrict__ scal, double *__restrict__ part) {
-  __shared__ double sh[T256 / 32];
-  const double alpha = scal[0] / scal[1];
+// The outer iteration in four passes over the FP64 vectors besides the operator and the V-cycle.
+// Every CTA of a pass sums the partials of the pass before it in the same order, so no launch is
+// spent on sums; the V-cycle's result z stays in its own precision, and the residual is stored in
+// it by the pass that updates r: 13.5 words of 8 bytes a DoF and iteration (FP32 V-cycle) instead of
+// the 17 of one kernel per vector operation with FP64 copies of z, in 5 launches instead of 13.
+// sc: [0] r.z of the current direction, [1] r.z new, [3] |r|^2.
+constexpr int PCG_BLOCKS = 152 * 6;
+
+__device__ __forceinline__ double all_partials(const double *__restrict__ part, double *sh) {
   double s = 0;
-  GRID_STRIDE(t, n) {
-    x[t] = fma(alpha, p[t], x[t]);
-    const double rt = fma(-alpha, v[t], r[t]);
-    r[t] = rt;
-    s = fma(rt, rt, s);
+  for (int i = threadIdx.x; i < PCG_BLOCKS; i += T256) s += part[i];
+  s = warp_block_sum(s, sh);
+  __syncthreads();
+  if (threadIdx.x == 0) sh[0] = s;
+  __syncthreads();
+  s = sh[0];
+  __syncthreads();
+  return s;
+}
+
+// partials of r.z
+template <class T>
+__global__ void __launch_bounds__(T256)
+    k_pcg_rz(int64_t n, const double *__restrict__ r, const T *__restrict__ z,
+             double *__restrict__ part) {
+  __shared__ double sh[T256 / 32];
+  double s = 0;
+  constexpr int W = Pack<T>::W;
+  GRID_STRIDE(q, n / W) {
+    const int64_t t = q * W;
+    const Pack<T> pz = pack_at(z, t);
+#pragma unroll
+    for (int k = 0; k < W; k += 2) {
+      const Pack<double> pr = pack_at(r, t + k);
+      s = fma(pr.v[0], (double)pz.v[k], s);
+      s = fma(pr.v[1], (double)pz.v[k + 1], s);
+    }
   }
+  GRID_STRIDE(q, n % W) s = fma(r[n / W * W + q], (double)z[n / W * W + q], s);
   s = warp_block_sum(s, sh);
   if (threadIdx.x == 0) part[blockIdx.x] = s;
 }
 
-// p = z + beta p, beta = scal[2] / scal[0]; then scal[0] = scal[2]  (one CTA
-// updates the scalar after every CTA has read it: done by a separate kernel)
+// p = z + beta p, beta = r.z / previous r.z (infinite before the first direction: beta = 0);
+// v = 0 with p on the constrained rows, ready for v += A p
+template <class T>
 __global__ void __launch_bounds__(T256)
-    k_pcg_direction(int64_t n, const double *__restrict__ z, double *__restrict__ p,
-                    const double *__restrict__ scal) {
-  const double beta = scal[2] / scal[0];
-  GRID_STRIDE(t, n) p[t] = fma(beta, p[t], z[t]);
+    k_pcg_direction(int64_t n, const T *__restrict__ z, double *__restrict__ p,
+                    double *__restrict__ v, const uint32_t *__restrict__ bits,
+                    const double *__restrict__ part, double *__restrict__ sc) {
+  __shared__ double sh[T256 / 32];
+  const double rz = all_partials(part, sh), beta = rz / sc[0];
+  if (blockIdx.x == 0 && threadIdx.x == 0) sc[1] = rz;
+  constexpr int W = Pack<T>::W;
+  GRID_STRIDE(q, n / W) {
+    const int64_t t = q * W;
+    const Pack<T> pz = pack_at(z, t);
+    const uint32_t m = __ldg(bits + (t >> 5)) >> (t & 31);
+#pragma unroll
+    for (int k = 0; k < W; k += 2) {
+      Pack<double> pp = pack_at(p, t + k), pv;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        pp.v[h] = fma(beta, pp.v[h], (double)pz.v[k + h]);
+        pv.v[h] = (m >> (k + h)) & 1u ? pp.v[h] : 0.0;
+      }
+      put_pack(p, t + k, pp);
+      put_pack(v, t + k, pv);
+    }
+  }
+  GRID_STRIDE(q, n % W) {
+    const int64_t t = n / W * W + q;
+    p[t] = fma(beta, p[t], (double)z[t]);
+    v[t] = bit_at(bits, t) ? p[t] : 0.0;
+  }
 }
 
-__global__ void k_copy_scalar(double *__restrict__ scal, int from, int to) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) scal[to] = scal[from];
+// partials of p.v; the new r.z becomes the current one
+__global__ void __launch_bounds__(T256)
+    k_pcg_pv(int64_t n, const double *__restrict__ p, const double *__restrict__ v,
+             double *__restrict__ part, double *__restrict__ sc) {
+  __shared__ double sh[T256 / 32];
+  if (blockIdx.x == 0 && threadIdx.x == 0) sc[0] = sc[1];
+  double s = 0;
+  GRID_STRIDE(q, n / 2) {
+    const Pack<double> a = pack_at(p, q * 2), b = pack_at(v, q * 2);
+    s = fma(a.v[0], b.v[0], s);
+    s = fma(a.v[1], b.v[1], s);
+  }
+  if (n % 2 && blockIdx.x == 0 && threadIdx.x == 0) s = fma(p[n - 1], v[n - 1], s);
+  s = warp_block_sum(s, sh);
+  if (threadIdx.x == 0) part[blockIdx.x] = s;
+}
+
+// x += alpha p; r -= alpha v, alpha = r.z / p.v; b = r in the V-cycle's precision; partials of |r|^2
+template <class T>
+__global__ void __launch_bounds__(T256)
+    k_pcg_update(int64_t n, double *__restrict__ x, double *__restrict__ r,
+                 const double *__restrict__ p, const double *__restrict__ v, T *__restrict__ b,
+                 const double *__restrict__ pv_part, const double *__restrict__ sc,
+                 double *__restrict__ part) {
+  __shared__ double sh[T256 / 32];
+  const double alpha = sc[0] / all_partials(pv_part, sh);
+  double s = 0;
+  GRID_STRIDE(t, n) {  // (x is the caller's: no alignment beyond its own)
+    x[t] = fma(alpha, p[t], x[t]);
+    const double rt = fma(-alpha, v[t], r[t]);
+    r[t] = rt;
+    b[t] = (T)rt;
+    s = fma(rt, rt, s);
+  }
+  s = warp_block_sum(s, sh);
+  if (threadIdx.x == 0) part[blockIdx.x] = s;
 }
 
 }  // namespace
@@ -254,6 +338,16 @@ mfgb_status level_vmult(mfgb_operator *op, int prec, void *dst, const void *src,
   return cuda_status(cudaGetLastError(), "A32 constrained");
 }
 
+// t += A src on the unconstrained rows of one level in the V-cycle precision; t enters zero and its
+// consumer takes the constrained rows from src (MgLevel::bits)
+mfgb_status level_apply(const MgLevel &L, int prec, const void *src, cudaStream_t s) {
+  if (prec == 64)
+    return apply_add_impl(L.op, (double *)L.t, (const double *)src, MFGB_ARITH_FP64_DF, s, nullptr);
+  return cuda_status(bk5_f32(L.op->n, L.op->n_cells, L.op->d_map, L.op->d_G32, (const float *)src,
+                             (float *)L.t, L.op->D, nullptr, nullptr, s),
+                     "A32 kernel");
+}
+
 template <class T>
 mfgb_status chebyshev(const MgLevel &L, int degree, double range, bool zero_start, int prec,
                       cudaStream_t s) {
@@ -264,19 +358,19 @@ mfgb_status chebyshev(const MgLevel &L, int degree, double range, bool zero_star
   double rho = 1.0 / sigma;
   T *x = (T *)L.x, *b = (T *)L.b, *r = (T *)L.r, *d = (T *)L.d, *t = (T *)L.t;
   const T *dinv = (const T *)L.inv_diag;
-  const unsigned g = grid1d(L.n);
+  const unsigned g = grid1d(L.n / Pack<T>::W);
   mfgb_status st;
   if (zero_start) {
-    k_cheb_first_zero<T><<<g, T256, 0, s>>>(L.n, b, dinv, x, d, r, (T)(1.0 / theta));
+    k_cheb_first_zero<T><<<g, T256, 0, s>>>(L.n, b, dinv, x, d, r, t, (T)(1.0 / theta));
   } else {
-    if ((st = level_vmult(L.op, prec, t, x, s))) return st;
-    k_cheb_first<T><<<g, T256, 0, s>>>(L.n, b, t, dinv, x, d, r, (T)(1.0 / theta));
+    if ((st = level_apply(L, prec, x, s))) return st;
+    k_cheb_first<T><<<g, T256, 0, s>>>(L.n, b, t, dinv, x, d, r, L.bits, (T)(1.0 / theta));
   }
   for (int k = 1; k < degree; ++k) {
-    if ((st = level_vmult(L.op, prec, t, d, s))) return st;
+    if ((st = level_apply(L, prec, d, s))) return st;
     const double rho_new = 1.0 / (2.0 * sigma - rho);
     const double c1 = rho_new * rho, c2 = 2.0 * rho_new / delta;
-    k_cheb_step<T><<<g, T256, 0, s>>>(L.n, t, dinv, x, d, r, (T)c1, (T)c2);
+    k_cheb_step<T><<<g, T256, 0, s>>>(L.n, t, dinv, x, d, r, L.bits, (T)c1, (T)c2);
     rho = rho_new;
   }
   return cuda_status(cudaGetLastError(), "chebyshev");
@@ -297,8 +391,9 @@ mfgb_status vcycle(mfgb_mg *mg, size_t l, cudaStream_t s) {
   }
   MgLevel &C = mg->levels[l + 1];
   if ((st = chebyshev<T>(L, mg->degree, mg->range, true, prec, s))) return st;
-  if ((st = level_vmult(L.op, prec, L.t, L.x, s))) return st;
-  k_residual<T><<<grid1d(L.n), T256, 0, s>>>(L.n, (const T *)L.b, (const T *)L.t, (T *)L.r);
+  if ((st = level_apply(L, prec, L.x, s))) return st;
+  const unsigned g = grid1d(L.n / Pack<T>::W);
+  k_level_residual<T><<<g, T256, 0, s>>>(L.n, (const T *)L.b, (T *)L.t, (const T *)L.x, L.bits, (T *)L.r);
   if (L.to_coarse == 1) {
     const PTransferParams P = ptransfer(L.op, C.op);
     if ((st = cuda_status(cudaMemsetAsync(C.b, 0, sizeof(T) * C.n, s), "coarse b = 0"))) return st;
@@ -311,10 +406,9 @@ mfgb_status vcycle(mfgb_mg *mg, size_t l, cudaStream_t s) {
   if ((st = vcycle<T>(mg, l + 1, s))) return st;
   if (L.to_coarse == 1) {
     const PTransferParams P = ptransfer(L.op, C.op);
-    if ((st = cuda_status(cudaMemsetAsync(L.t, 0, sizeof(T) * L.n, s), "t = 0"))) return st;
     p_transfer<T>(false, L.op->n_cells, L.op->d_map, C.op->d_map, (const T *)C.x, nullptr,
                   (T *)L.t, P, s);
-    k_axpy<T><<<grid1d(L.n), T256, 0, s>>>(L.n, (T)1, (const T *)L.t, (T *)L.x);
+    k_add_clear<T><<<g, T256, 0, s>>>(L.n, (T *)L.t, (T *)L.x);
   } else {
     k_h_prolongate_add<T><<<grid1d(L.n), T256, 0, s>>>(hgrid(L.box, L.bs, C.box), (const T *)C.x,
                                                         (T *)L.x);
@@ -460,12 +554,12 @@ void free_mg(mfgb_mg *mg) {
   if (!mg) return;
   for (auto &L : mg->levels) {
     cudaFree(L.x); cudaFree(L.b); cudaFree(L.r); cudaFree(L.d); cudaFree(L.t);
-    cudaFree(L.inv_diag); cudaFree(L.inv_val);
+    cudaFree(L.inv_diag); cudaFree(L.inv_val); cudaFree(L.bits);
     if (L.op && !L.borrowed) mfgb_operator_destroy(L.op);
   }
   cudaFree(mg->coarse.A); cudaFree(mg->coarse.dinv); cudaFree(mg->coarse.work);
   cudaFree(mg->coarse.ids);
-  cudaFree(mg->r); cudaFree(mg->z); cudaFree(mg->p); cudaFree(mg->v); cudaFree(mg->part);
+  cudaFree(mg->r); cudaFree(mg->p); cudaFree(mg->v); cudaFree(mg->part);
   cudaFree(mg->scal);
   delete mg;
 }
@@ -544,8 +638,12 @@ static mfgb_status mg_setup_impl(const mfgb_box_desc *fine, const mfgb_mg_params
     MgLevel &M = mg->levels.back();
     if ((st = dalloc(&M.x, ts * M.n)) || (st = dalloc(&M.b, ts * M.n)) ||
         (st = dalloc(&M.r, ts * M.n)) || (st = dalloc(&M.d, ts * M.n)) ||
-        (st = dalloc(&M.t, ts * M.n)) || (st = dalloc(&M.inv_diag, ts * M.n)))
+        (st = dalloc(&M.t, ts * M.n)) || (st = dalloc(&M.inv_diag, ts * M.n)) ||
+        (st = dalloc((void **)&M.bits, sizeof(uint32_t) * ((M.n + 31) / 32))))
       break;
+    cudaMemset(M.bits, 0, sizeof(uint32_t) * ((M.n + 31) / 32));
+    if (M.op->n_constrained)
+      k_set_bits<<<grid1d(M.op->n_constrained), T256>>>(M.op->n_constrained, M.op->d_constrained, M.bits);
     if (prm->precision == 32 && (st = ensure_g32(M.op))) break;
     if (prm->precision == 64 && (st = ensure_arith(M.op, MFGB_ARITH_FP64_DF))) break;
     // Jacobi in the V-cycle precision
@@ -727,14 +825,13 @@ extern "C" mfgb_status mfgb_mg_cg_solve(const mfgb_operator *cop, mfgb_mg *mg, c
   const int64_t n = op->n_dofs;
   mfgb_status st;
   if (mg->outer_n != n) {
-    cudaFree(mg->r); cudaFree(mg->z); cudaFree(mg->p); cudaFree(mg->v); cudaFree(mg->part);
-    cudaFree(mg->scal);
-    mg->r = mg->z = mg->p = mg->v = mg->part = mg->scal = nullptr;
+    cudaFree(mg->r); cudaFree(mg->p); cudaFree(mg->v); cudaFree(mg->part); cudaFree(mg->scal);
+    mg->r = mg->p = mg->v = mg->part = mg->scal = nullptr;
+    mg->outer_n = -1;
     if ((st = dalloc((void **)&mg->r, sizeof(double) * n)) ||
-        (st = dalloc((void **)&mg->z, sizeof(double) * n)) ||
         (st = dalloc((void **)&mg->p, sizeof(double) * n)) ||
         (st = dalloc((void **)&mg->v, sizeof(double) * n)) ||
-        (st = dalloc((void **)&mg->part, sizeof(double) * (152 * 32 + 8))) ||
+        (st = dalloc((void **)&mg->part, sizeof(double) * 3 * PCG_BLOCKS)) ||
         (st = dalloc((void **)&mg->scal, sizeof(double) * 8)))
       return st;
     mg->outer_n = n;
@@ -750,17 +847,15 @@ extern "C" mfgb_status mfgb_mg_cg_solve(const mfgb_operator *cop, mfgb_mg *mg, c
   cudaEventDestroy(ev);
   const int arith = ctl->arith;
   if ((st = ensure_arith(op, arith))) return st;
-  const unsigned g = grid1d(n);
-  double *r = mg->r, *z = mg->z, *p = mg->p, *v = mg->v, *part = mg->part, *scal = mg->scal;
-  // scal: [0] r.z (current), [1] p.v, [2] r.z (new), [3] |r|^2
-  auto dot_into = [&](const double *a, const double *b, int slot) {
-    k_dot_partials<<<g, T256, 0, s>>>(n, a, b, part);
-    k_sum_partials<<<1, T256, 0, s>>>(part, (int)g, scal + slot);
-  };
-  // r = b - A x ; z = M r ; p = z ; rz
+  double *r = mg->r, *p = mg->p, *v = mg->v, *scal = mg->scal;
+  double *part_rz = mg->part, *part_pv = part_rz + PCG_BLOCKS, *part_rr = part_pv + PCG_BLOCKS;
+  const MgLevel &L = mg->levels[0];
+  constexpr unsigned g = PCG_BLOCKS;
+  // r = b - A x
   if ((st = vmult_impl(op, v, d_x, arith, nullptr, nullptr, s))) return st;
-  k_residual<double><<<g, T256, 0, s>>>(n, d_b, v, r);
-  dot_into(r, r, 3);
+  k_residual<double><<<grid1d(n), T256, 0, s>>>(n, d_b, v, r);
+  k_dot_partials<<<g, T256, 0, s>>>(n, r, r, part_rr);
+  k_sum_partials<<<1, T256, 0, s>>>(part_rr, (int)g, scal + 3);
   double h[4];
   if ((st = cuda_status(cudaMemcpyAsync(h, scal, sizeof(h), cudaMemcpyDeviceToHost, s), "pcg init")) ||
       (st = cuda_status(cudaStreamSynchronize(s), "pcg init")))
@@ -772,27 +867,36 @@ extern "C" mfgb_status mfgb_mg_cg_solve(const mfgb_operator *cop, mfgb_mg *mg, c
   const double tol_eff = std::fmax(ctl->tol, ctl->reduce * res0);
   if (res0 <= tol_eff) { info->converged = 1; return MFGB_OK; }
   if (std::isnan(res0)) { set_error("mfgb_mg_cg_solve: NaN residual"); return MFGB_ERR_NONFINITE; }
-  if ((st = mg_apply(mg, z, r, s))) return st;
-  cudaMemcpyAsync(p, z, sizeof(double) * n, cudaMemcpyDeviceToDevice, s);
-  dot_into(r, z, 0);
+  // before the first direction: p = 0, an infinite previous r.z, and the residual as the V-cycle's
+  // right-hand side
+  const double inf = INFINITY;
+  if (mg->precision == 32)
+    k_convert<float, double><<<grid1d(n), T256, 0, s>>>(n, r, (float *)L.b);
+  else
+    cudaMemcpyAsync(L.b, r, sizeof(double) * n, cudaMemcpyDeviceToDevice, s);
+  cudaMemsetAsync(p, 0, sizeof(double) * n, s);
+  if ((st = cuda_status(cudaMemcpyAsync(scal, &inf, sizeof(inf), cudaMemcpyHostToDevice, s), "pcg start")))
+    return st;
 
-  // one iteration as a graph
+  // one iteration as a graph: V-cycle, direction, operator, update.  The V-cycle comes first, so
+  // none is spent on the residual that ends the solve.
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   if ((st = cuda_status(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal), "capture")))
     return st;
-  mfgb_status cap = vmult_impl(op, v, p, arith, nullptr, nullptr, s);
-  if (!cap) {
-    dot_into(p, v, 1);
-    k_pcg_update<<<g, T256, 0, s>>>(n, d_x, r, p, v, scal, part);
-    k_sum_partials<<<1, T256, 0, s>>>(part, (int)g, scal + 3);
-    cap = mg_apply(mg, z, r, s);
-  }
-  if (!cap) {
-    dot_into(r, z, 2);
-    k_pcg_direction<<<g, T256, 0, s>>>(n, z, p, scal);
-    k_copy_scalar<<<1, 32, 0, s>>>(scal, 2, 0);
-  }
+  auto iteration = [&](auto zero) -> mfgb_status {
+    using T = decltype(zero);
+    mfgb_status e = vcycle<T>(mg, 0, s);
+    if (e) return e;
+    k_pcg_rz<T><<<g, T256, 0, s>>>(n, r, (const T *)L.x, part_rz);
+    k_pcg_direction<T><<<g, T256, 0, s>>>(n, (const T *)L.x, p, v, L.bits, part_rz, scal);
+    if ((e = apply_add_impl(op, v, p, arith, s, nullptr))) return e;
+    k_pcg_pv<<<g, T256, 0, s>>>(n, p, v, part_pv, scal);
+    k_pcg_update<T><<<g, T256, 0, s>>>(n, d_x, r, p, v, (T *)L.b, part_pv, scal, part_rr);
+    k_sum_partials<<<1, T256, 0, s>>>(part_rr, (int)g, scal + 3);
+    return cuda_status(cudaGetLastError(), "pcg iteration");
+  };
+  const mfgb_status cap = mg->precision == 32 ? iteration(0.f) : iteration(0.0);
   const cudaError_t ce = cudaStreamEndCapture(s, &graph);
   if (cap) { if (graph) cudaGraphDestroy(graph); return cap; }
   if ((st = cuda_status(ce, "end capture"))) return st;

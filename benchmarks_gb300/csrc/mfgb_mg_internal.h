@@ -14,6 +14,7 @@ struct MgLevel {
   int64_t n = 0;
   void *x = nullptr, *b = nullptr, *r = nullptr, *d = nullptr, *t = nullptr;
   void *inv_diag = nullptr;  // Jacobi (precision T)
+  uint32_t *bits = nullptr;  // one bit per DoF: constrained
   void *inv_val = nullptr;   // 1/valence (precision T), for p-restriction from this level
   double lmax = 0;
   int to_coarse = 0;  // 1 = p-transfer, 2 = h-transfer, 0 = coarsest
@@ -50,7 +51,6 @@ struct mfgb_mg {
   std::vector<mfgb::MgLevel> levels;
   mfgb::MgCoarse coarse;
   // outer PCG buffers (FP64)
-  double *r = nullptr, *z = nullptr, *p = nullptr, *v = nullptr, *part = nullptr,
-         *scal = nullptr;
+  double *r = nullptr, *p = nullptr, *v = nullptr, *part = nullptr, *scal = nullptr;
   int64_t outer_n = 0;
 };

@@ -59,44 +59,166 @@ __global__ void k_convert(int64_t n, const TI *__restrict__ a, TO *__restrict__ 
   GRID_STRIDE(t, n) b[t] = (TO)a[t];
 }
 
-// Chebyshev first step from x0 = 0: x = d = (1/theta) Dinv b ; r = b
+// Smoothing works on an operator result t that every consumer zeroes again after reading it, so
+// that the next application can accumulate into it: no clearing pass and launch of its own.  The
+// identity rows of the constrained DoFs are taken from the operator's input instead of being copied
+// into its result: `bits` has one bit per DoF, set where it is constrained.
+__global__ void k_set_bits(int64_t nc, const int64_t *__restrict__ c, uint32_t *__restrict__ bits) {
+  GRID_STRIDE(t, nc) atomicOr(bits + (c[t] >> 5), 1u << (c[t] & 31));
+}
+__device__ __forceinline__ bool bit_at(const uint32_t *__restrict__ bits, int64_t t) {
+  return (__ldg(bits + (t >> 5)) >> (t & 31)) & 1u;
+}
+
+// 16-byte packs: the level vectors are whole allocations, so every pack of W values is aligned and
+// lies in one word of bits; the last n % W values go one at a time
+template <class T> struct alignas(16) Pack {
+  static constexpr int W = 16 / sizeof(T);
+  T v[W];
+};
+template <class T> __device__ __forceinline__ Pack<T> pack_at(const T *p, int64_t t) {
+  return *reinterpret_cast<const Pack<T> *>(p + t);
+}
+template <class T> __device__ __forceinline__ void put_pack(T *p, int64_t t, const Pack<T> &v) {
+  *reinterpret_cast<Pack<T> *>(p + t) = v;
+}
+
+// Chebyshev first step from x0 = 0: x = d = (1/theta) Dinv b ; r = b ; t = 0
 template <class T>
 __global__ void k_cheb_first_zero(int64_t n, const T *__restrict__ b, const T *__restrict__ dinv,
                                   T *__restrict__ x, T *__restrict__ d, T *__restrict__ r,
-                                  T inv_theta) {
-  GRID_STRIDE(t, n) {
-    const T bt = b[t];
-    const T dt = inv_theta * dinv[t] * bt;
-    r[t] = bt;
-    d[t] = dt;
-    x[t] = dt;
+                                  T *__restrict__ tz, T inv_theta) {
+  constexpr int W = Pack<T>::W;
+  GRID_STRIDE(q, n / W) {
+    const int64_t t = q * W;
+    const Pack<T> pb = pack_at(b, t), pd = pack_at(dinv, t);
+    Pack<T> o, z;
+#pragma unroll
+    for (int k = 0; k < W; ++k) o.v[k] = inv_theta * pd.v[k] * pb.v[k], z.v[k] = T(0);
+    put_pack(r, t, pb);
+    put_pack(d, t, o);
+    put_pack(x, t, o);
+    put_pack(tz, t, z);
+  }
+  GRID_STRIDE(q, n % W) {
+    const int64_t t = n / W * W + q;
+    r[t] = b[t];
+    d[t] = x[t] = inv_theta * dinv[t] * b[t];
+    tz[t] = T(0);
   }
 }
 
-// Chebyshev first step from x0: r = b - Ax (Ax in ax); d = (1/theta) Dinv r; x += d
+// Chebyshev first step from x0: r = b - A x (A x in ax, zeroed); d = (1/theta) Dinv r; x += d
 template <class T>
-__global__ void k_cheb_first(int64_t n, const T *__restrict__ b, const T *__restrict__ ax,
+__global__ void k_cheb_first(int64_t n, const T *__restrict__ b, T *__restrict__ ax,
                              const T *__restrict__ dinv, T *__restrict__ x, T *__restrict__ d,
-                             T *__restrict__ r, T inv_theta) {
-  GRID_STRIDE(t, n) {
-    const T rt = b[t] - ax[t];
+                             T *__restrict__ r, const uint32_t *__restrict__ bits, T inv_theta) {
+  constexpr int W = Pack<T>::W;
+  GRID_STRIDE(q, n / W) {
+    const int64_t t = q * W;
+    const Pack<T> pb = pack_at(b, t), pa = pack_at(ax, t), pd = pack_at(dinv, t);
+    Pack<T> px = pack_at(x, t), od, orr, z;
+    const uint32_t m = __ldg(bits + (t >> 5)) >> (t & 31);
+#pragma unroll
+    for (int k = 0; k < W; ++k) {
+      orr.v[k] = pb.v[k] - ((m >> k) & 1u ? px.v[k] : pa.v[k]);
+      od.v[k] = inv_theta * pd.v[k] * orr.v[k];
+      px.v[k] += od.v[k];
+      z.v[k] = T(0);
+    }
+    put_pack(r, t, orr);
+    put_pack(d, t, od);
+    put_pack(x, t, px);
+    put_pack(ax, t, z);
+  }
+  GRID_STRIDE(q, n % W) {
+    const int64_t t = n / W * W + q;
+    const T rt = b[t] - (bit_at(bits, t) ? x[t] : ax[t]);
     const T dt = inv_theta * dinv[t] * rt;
     r[t] = rt;
     d[t] = dt;
     x[t] += dt;
+    ax[t] = T(0);
   }
 }
 
-// r -= A d (in ad); d = c1 d + c2 Dinv r; x += d
+// r -= A d (A d in ad, zeroed); d = c1 d + c2 Dinv r; x += d
 template <class T>
-__global__ void k_cheb_step(int64_t n, const T *__restrict__ ad, const T *__restrict__ dinv,
-                            T *__restrict__ x, T *__restrict__ d, T *__restrict__ r, T c1, T c2) {
-  GRID_STRIDE(t, n) {
-    const T rt = r[t] - ad[t];
+__global__ void k_cheb_step(int64_t n, T *__restrict__ ad, const T *__restrict__ dinv,
+                            T *__restrict__ x, T *__restrict__ d, T *__restrict__ r,
+                            const uint32_t *__restrict__ bits, T c1, T c2) {
+  constexpr int W = Pack<T>::W;
+  GRID_STRIDE(q, n / W) {
+    const int64_t t = q * W;
+    const Pack<T> pa = pack_at(ad, t), pi = pack_at(dinv, t);
+    Pack<T> px = pack_at(x, t), pd = pack_at(d, t), pr = pack_at(r, t), z;
+    const uint32_t m = __ldg(bits + (t >> 5)) >> (t & 31);
+#pragma unroll
+    for (int k = 0; k < W; ++k) {
+      pr.v[k] -= (m >> k) & 1u ? pd.v[k] : pa.v[k];
+      pd.v[k] = c1 * pd.v[k] + c2 * pi.v[k] * pr.v[k];
+      px.v[k] += pd.v[k];
+      z.v[k] = T(0);
+    }
+    put_pack(r, t, pr);
+    put_pack(d, t, pd);
+    put_pack(x, t, px);
+    put_pack(ad, t, z);
+  }
+  GRID_STRIDE(q, n % W) {
+    const int64_t t = n / W * W + q;
+    const T rt = r[t] - (bit_at(bits, t) ? d[t] : ad[t]);
     const T dt = c1 * d[t] + c2 * dinv[t] * rt;
     r[t] = rt;
     d[t] = dt;
     x[t] += dt;
+    ad[t] = T(0);
+  }
+}
+
+// r = b - A x (A x in ax, zeroed)
+template <class T>
+__global__ void k_level_residual(int64_t n, const T *__restrict__ b, T *__restrict__ ax,
+                                 const T *__restrict__ x, const uint32_t *__restrict__ bits,
+                                 T *__restrict__ r) {
+  constexpr int W = Pack<T>::W;
+  GRID_STRIDE(q, n / W) {
+    const int64_t t = q * W;
+    const Pack<T> pb = pack_at(b, t), pa = pack_at(ax, t);
+    Pack<T> o, z;
+    const uint32_t m = __ldg(bits + (t >> 5)) >> (t & 31);
+#pragma unroll
+    for (int k = 0; k < W; ++k) {
+      o.v[k] = pb.v[k] - ((m >> k) & 1u ? x[t + k] : pa.v[k]);
+      z.v[k] = T(0);
+    }
+    put_pack(r, t, o);
+    put_pack(ax, t, z);
+  }
+  GRID_STRIDE(q, n % W) {
+    const int64_t t = n / W * W + q;
+    r[t] = b[t] - (bit_at(bits, t) ? x[t] : ax[t]);
+    ax[t] = T(0);
+  }
+}
+
+// x += t ; t = 0
+template <class T>
+__global__ void k_add_clear(int64_t n, T *__restrict__ tv, T *__restrict__ x) {
+  constexpr int W = Pack<T>::W;
+  GRID_STRIDE(q, n / W) {
+    const int64_t t = q * W;
+    Pack<T> px = pack_at(x, t), z;
+    const Pack<T> pt = pack_at(tv, t);
+#pragma unroll
+    for (int k = 0; k < W; ++k) px.v[k] += pt.v[k], z.v[k] = T(0);
+    put_pack(x, t, px);
+    put_pack(tv, t, z);
+  }
+  GRID_STRIDE(q, n % W) {
+    const int64_t t = n / W * W + q;
+    x[t] += tv[t];
+    tv[t] = T(0);
   }
 }
 
@@ -105,11 +227,6 @@ template <class T>
 __global__ void k_residual(int64_t n, const T *__restrict__ b, const T *__restrict__ ax,
                            T *__restrict__ r) {
   GRID_STRIDE(t, n) r[t] = b[t] - ax[t];
-}
-
-template <class T>
-__global__ void k_axpy(int64_t n, T a, const T *__restrict__ x, T *__restrict__ y) {
-  GRID_STRIDE(t, n) y[t] += a * x[t];
 }
 
 template <class T>
