@@ -133,7 +133,7 @@ mfgb_status ensure_arith(mfgb_operator *op, int arith) {
 // partials/grid (the energy form) are supported by the GLL and Gauss p+1 kernels
 static cudaError_t apply_range(mfgb_operator *op, int64_t cell0, int64_t n, double *dst,
                                const double *src, int arith, double *partials, int *grid,
-                               cudaStream_t s, const int *done) {
+                               cudaStream_t s, const int *done, bool after_start = false) {
   const int64_t n3 = (int64_t)op->n * op->n * op->n;
   const int64_t q3 = (int64_t)op->nq * op->nq * op->nq;
   const uint32_t *map = op->d_map + cell0 * n3;
@@ -142,7 +142,8 @@ static cudaError_t apply_range(mfgb_operator *op, int64_t cell0, int64_t n, doub
   if (op->quadrature >= 1 && arith == MFGB_ARITH_FP64_DF && op->d_Gfx && !partials &&
       (!op->d_JxW || op->d_JxWfx))
     return bp3_fx(op->degree, op->nq, n, map, op->d_Gfx + cell0 * 6 * q3, op->d_Gexp + cell0, src,
-                  dst, op->Bq, op->DG, s, done, op->d_JxWfx ? op->d_JxWfx + cell0 * q3 : nullptr);
+                  dst, op->Bq, op->DG, s, done, op->d_JxWfx ? op->d_JxWfx + cell0 * q3 : nullptr,
+                  after_start);
   if (op->quadrature == 2) {
     if (partials || done) return cudaErrorNotSupported;
     return bp3_apply(op->degree, n, map, op->d_Bq, op->d_DGq, op->Bq, op->DG,
@@ -161,10 +162,16 @@ static cudaError_t apply_range(mfgb_operator *op, int64_t cell0, int64_t n, doub
   // GLL collocation: the offset-accumulation kernel (no energy partials)
   if (op->d_Gfx && !partials && (kernel_shape(1, op->n) >= kShapeFx || !op->d_Gdf))
     return bk5_fx(op->n, n, map, op->d_Gfx + cell0 * 6 * n3, op->d_Gexp + cell0, src, dst, op->D, s,
-                  done);
+                  done, after_start);
   return bk5_df(op->n, n, map, op->d_Gdf + cell0 * 6 * n3, src, dst, op->D, partials, grid, s,
                 done);
 }
+
+// Whether a result of n values gets its start values from start_vmult: up to 160 MB.  Above, a
+// clearing memset writes faster than the kernel, by more than the two launches it takes with the
+// identity rows (p = 4, us with memset / start_vmult: 0.27M DoFs 27 / 16, 4.2M 114 / 107, 17M 412 /
+// 410, 33M 788 / 797, 67.6M 1588 / 1635).
+bool starts_in_one(const mfgb_operator *op, int64_t n) { return op->masked && n <= 20000000; }
 
 mfgb_status vmult_impl(mfgb_operator *op, double *dst, const double *src, int arith,
                        double *partials, int *grid, cudaStream_t s, const int *done) {
@@ -177,13 +184,16 @@ mfgb_status vmult_impl(mfgb_operator *op, double *dst, const double *src, int ar
   if ((st = ensure_arith(op, arith))) return st;
   if (arith == MFGB_ARITH_FP64_DF && !uses_fx(op) && (st = range_check_async(op, op->n_dofs, src, s)))
     return st;
-  if (full && (st = cuda_status(cudaMemsetAsync(dst, 0, sizeof(double) * op->n_dofs, s),
-                                "vmult: dst = 0")))
+  // the start values and the identity rows in one launch, which the operator kernel's prologue
+  // overlaps, unless the map leaves constrained DoFs in (their rows are then overwritten afterwards)
+  const bool start = full && starts_in_one(op, op->n_dofs);
+  if (start) st = cuda_status(start_vmult(op->n_dofs, 1, op->d_cbits, src, dst, s), "vmult: start");
+  else if (full) st = cuda_status(cudaMemsetAsync(dst, 0, sizeof(double) * op->n_dofs, s), "vmult: dst = 0");
+  if (st || (st = cuda_status(apply_range(op, 0, op->n_cells, dst, src, arith, partials, grid, s, done,
+                                          start),
+                              "vmult: operator kernel")))
     return st;
-  if ((st = cuda_status(apply_range(op, 0, op->n_cells, dst, src, arith, partials, grid, s, done),
-                        "vmult: operator kernel")))
-    return st;
-  if (full)
+  if (full && !start)
     return cuda_status(copy_constrained(op->n_constrained, op->d_constrained, src, dst, s),
                        "vmult: constrained rows");
   return MFGB_OK;
@@ -390,6 +400,7 @@ static void free_operator(mfgb_operator *op) {
   cudaFree(op->d_Gexp);
   cudaFree(op->d_range);
   cudaFree(op->d_constrained);
+  cudaFree(op->d_cbits);
   cudaFree(op->d_partials);
   cudaFree(op->d_JxW);
   cudaFree(op->d_JxWdf);
@@ -562,10 +573,13 @@ static mfgb_status create_box_impl(const mfgb_box_desc *box, int quadrature, mfg
     }
   op->n_constrained = (int64_t)cons.size();
   op->h_constrained = cons;
+  op->masked = true;
   mfgb_status st;
   if ((st = dev_alloc((void **)&op->d_map, sizeof(uint32_t) * op->n_cells * n3, "dof map")) ||
       (st = dev_alloc((void **)&op->d_G, sizeof(double) * op->n_cells * 6 * q3, "G")) ||
       (st = dev_alloc((void **)&op->d_constrained, sizeof(int64_t) * cons.size(), "constraints")) ||
+      (st = dev_alloc((void **)&op->d_cbits, sizeof(uint32_t) * ((n_dofs + 31) / 32),
+                      "constrained bits")) ||
       (mass && (st = dev_alloc((void **)&op->d_JxW, sizeof(double) * op->n_cells * n3, "JxW"))) ||
       (quadrature == 2 &&
        ((st = dev_alloc((void **)&op->d_Bq, sizeof(double) * op->nq * op->n, "BP3 basis")) ||
@@ -576,6 +590,8 @@ static mfgb_status create_box_impl(const mfgb_box_desc *box, int quadrature, mfg
   if ((st = cuda_status(cudaMemcpy(op->d_constrained, cons.data(), sizeof(int64_t) * cons.size(),
                                    cudaMemcpyHostToDevice),
                         "constraints copy")) ||
+      (st = cuda_status(set_cbits(n_dofs, op->n_constrained, op->d_constrained, op->d_cbits, nullptr),
+                        "constrained bits")) ||
       (st = cuda_status(box_map(*box, op->d_map, nullptr), "box map")) ||
       (st = cuda_status(box_geometry(*box, op->gll_x, op->gll_w, op->D, op->d_G, nullptr,
                                      quadrature != 0, bs, op->d_JxW, op->nq),
@@ -610,21 +626,30 @@ mfgb_status mfgb_operator_create(int degree, int64_t n_dofs, int64_t n_cells,
       set_error("mfgb_operator_create: dof map entry out of range");
       return MFGB_ERR_INVALID_ARG;
     }
-  for (int64_t c = 0; c < n_constrained; ++c)
+  std::vector<bool> fixed(n_dofs, false);
+  for (int64_t c = 0; c < n_constrained; ++c) {
     if (h_constrained[c] < 0 || h_constrained[c] >= n_dofs) {
       set_error("mfgb_operator_create: constrained index out of range");
       return MFGB_ERR_INVALID_ARG;
     }
+    fixed[h_constrained[c]] = true;
+  }
+  bool masked = true;
+  for (int64_t t = 0; t < n_cells * n3; ++t)
+    if (h_dof_map[t] != MFGB_INVALID_DOF && fixed[h_dof_map[t]]) masked = false;
   mfgb_operator *op = new mfgb_operator();
   init_basis(op, degree);
   op->n_dofs = n_dofs;
   op->n_cells = n_cells;
   op->n_constrained = n_constrained;
+  op->masked = masked;
   mfgb_status st;
   if ((st = dev_alloc((void **)&op->d_map, sizeof(uint32_t) * n_cells * n3, "dof map")) ||
       (st = dev_alloc((void **)&op->d_G, sizeof(double) * n_cells * 6 * n3, "G")) ||
       (st = dev_alloc((void **)&op->d_constrained, sizeof(int64_t) * n_constrained,
-                      "constraints"))) {
+                      "constraints")) ||
+      (st = dev_alloc((void **)&op->d_cbits, sizeof(uint32_t) * ((n_dofs + 31) / 32),
+                      "constrained bits"))) {
     free_operator(op);
     return st;
   }
@@ -638,7 +663,10 @@ mfgb_status mfgb_operator_create(int degree, int64_t n_dofs, int64_t n_cells,
       (n_constrained > 0 &&
        (st = cuda_status(cudaMemcpy(op->d_constrained, h_constrained,
                                     sizeof(int64_t) * n_constrained, cudaMemcpyHostToDevice),
-                         "constraints copy")))) {
+                         "constraints copy"))) ||
+      (n_dofs > 0 &&
+       (st = cuda_status(set_cbits(n_dofs, n_constrained, op->d_constrained, op->d_cbits, nullptr),
+                         "constrained bits")))) {
     free_operator(op);
     return st;
   }

@@ -1212,9 +1212,8 @@ mfgb_status build_batch(mfgb_batch *B, const mfgb_box_desc *boxes, int n,
   for (Depth &D : B->depth) {
     const size_t bytes = sizeof(uint32_t) * ((D.n + 31) / 32);
     if ((st = dalloc((void **)&D.bits, bytes)) ||
-        (st = cuda_status(cudaMemset(D.bits, 0, bytes), "batch bits")))
+        (st = cuda_status(set_cbits(D.n, D.n_cons, D.d_cons, D.bits, nullptr), "batch bits")))
       return st;
-    if (D.n_cons) k_set_bits<<<grid1d(D.n_cons), T256>>>(D.n_cons, D.d_cons, D.bits);
   }
   // ---- lambda_max of every smoothed part: one power iteration per depth -----
   // over all its parts (the start, normalisation, FP32 operator, constrained

@@ -63,7 +63,7 @@ static bool fx_basis(const double *D, FxBasis<N, SYM> &b) {
 template <int N, class Sh, class GT, bool EVEC, int NC, int SYM, bool MT, bool EXPIRE = false>
 static cudaError_t fx_run(int64_t n_cells, const uint32_t *map, const GT *G, const int *gexp,
                           const double *src, double *dst, const FxBasis<N, SYM> &b, cudaStream_t s,
-                          const int *done) {
+                          const int *done, bool after = false) {
   constexpr int E = Sh::E, T = E * N * N;
   constexpr size_t smem = FxLayout<N, E, GT, EVEC, Sh::NB>::total;
   const auto kernel = bk5fx_kernel<N, E, Sh::MB, Sh::NB, GT, EVEC, NC, SYM, MT, EXPIRE>;
@@ -71,8 +71,8 @@ static cudaError_t fx_run(int64_t n_cells, const uint32_t *map, const GT *G, con
   if (per_sm < 0) per_sm = std::max(1, ctas_per_sm(kernel, T, smem));
   const int64_t nb = (n_cells + E - 1) / E;
   const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(nb, (int64_t)per_sm * num_sms()));
-  kernel<<<grid, T, smem, s>>>(n_cells, map, G, gexp, src, dst, b, done, device_error_flag());
-  return cudaGetLastError();
+  return launch_after(after, kernel, grid, T, smem, s, n_cells, map, G, gexp, src, dst, b, done,
+                      device_error_flag());
 }
 
 // The kernel on the library's own scaled pairs.  Bulk copies of the dof-map tiles need a 16-byte
@@ -80,22 +80,22 @@ static cudaError_t fx_run(int64_t n_cells, const uint32_t *map, const GT *G, con
 template <int N, int NC>
 static cudaError_t fx_pairs(int64_t n_cells, const uint32_t *map, const float2 *G, const int *gexp,
                             const double *src, double *dst, const double *D, cudaStream_t s,
-                            const int *done) {
+                            const int *done, bool after) {
   FxBasis<N, -1> b;
   if (!fx_basis<N, -1>(D, b)) return cudaErrorInvalidValue;  // the GLL derivative has the symmetry
   using Sh = FxDefault<N>;
   const bool mt = (reinterpret_cast<uintptr_t>(map) & 15u) == 0;
   if (NC == 1 && take_expire())
     return fx_run<N, Sh, float2, false, 1, -1, false, true>(n_cells, map, G, gexp, src, dst, b, s,
-                                                            done);
+                                                            done, after);
   if constexpr (NC == 1) {
     using Alt = FxAlt<N>;
     if (kernel_shape(ArithClass<ArithDF>::value, N) == SHAPE_FX_ALT)
-      return mt ? fx_run<N, Alt, float2, false, 1, -1, true>(n_cells, map, G, gexp, src, dst, b, s, done)
-                : fx_run<N, Alt, float2, false, 1, -1, false>(n_cells, map, G, gexp, src, dst, b, s, done);
+      return mt ? fx_run<N, Alt, float2, false, 1, -1, true>(n_cells, map, G, gexp, src, dst, b, s, done, after)
+                : fx_run<N, Alt, float2, false, 1, -1, false>(n_cells, map, G, gexp, src, dst, b, s, done, after);
   }
-  return mt ? fx_run<N, Sh, float2, false, NC, -1, true>(n_cells, map, G, gexp, src, dst, b, s, done)
-            : fx_run<N, Sh, float2, false, NC, -1, false>(n_cells, map, G, gexp, src, dst, b, s, done);
+  return mt ? fx_run<N, Sh, float2, false, NC, -1, true>(n_cells, map, G, gexp, src, dst, b, s, done, after)
+            : fx_run<N, Sh, float2, false, NC, -1, false>(n_cells, map, G, gexp, src, dst, b, s, done, after);
 }
 
 // The kernel on the caller's FP64 G (16-byte aligned): L-vectors through map, or element vectors
@@ -157,20 +157,21 @@ cudaError_t bk5_fx_evec(int N, int64_t nelmt, const double *G, const double *src
 
 // the BK6 vector Laplacian: 3 interleaved components per DoF on one scaled G
 cudaError_t bk6_fx(int N, int64_t n_cells, const uint32_t *map, const float2 *G, const int *gexp,
-                   const double *src, double *dst, const double *D, cudaStream_t s) {
+                   const double *src, double *dst, const double *D, cudaStream_t s,
+                   bool after_start) {
   if (n_cells <= 0) return cudaSuccess;
   if (map == nullptr || (reinterpret_cast<uintptr_t>(G) & 15u)) return cudaErrorInvalidValue;
-#define MFGB_CALL(NN) (fx_pairs<NN, 3>(n_cells, map, G, gexp, src, dst, D, s, nullptr))
+#define MFGB_CALL(NN) (fx_pairs<NN, 3>(n_cells, map, G, gexp, src, dst, D, s, nullptr, after_start))
   MFGB_FX_DEGREES(MFGB_CALL)
 #undef MFGB_CALL
 }
 
 cudaError_t bk5_fx(int N, int64_t n_cells, const uint32_t *map, const float2 *G, const int *gexp,
                    const double *src, double *dst, const double *D, cudaStream_t s,
-                   const int *done) {
+                   const int *done, bool after_start) {
   if (n_cells <= 0) return cudaSuccess;
   if (map == nullptr || (reinterpret_cast<uintptr_t>(G) & 15u)) return cudaErrorInvalidValue;
-#define MFGB_CALL(NN) (fx_pairs<NN, 1>(n_cells, map, G, gexp, src, dst, D, s, done))
+#define MFGB_CALL(NN) (fx_pairs<NN, 1>(n_cells, map, G, gexp, src, dst, D, s, done, after_start))
   MFGB_FX_DEGREES(MFGB_CALL)
 #undef MFGB_CALL
 }

@@ -478,6 +478,7 @@ __global__ void __launch_bounds__(E * N * N, MB)
       }
       fx_line(basis.T, vr, qr);  // the r-share of the own column
       __syncthreads();
+      if (!EVEC) cudaGridDependencySynchronize();  // dst has its start values
       auto put = [&](int i, double v) {
         if constexpr (EVEC) {
           if (valid) dst[out_cell * N3 + i * N2 + jk] = v;

@@ -36,15 +36,18 @@ extern "C" mfgb_status mfgb_vmult_vector(const mfgb_operator *cop, double *d_dst
   mfgb_operator *op = const_cast<mfgb_operator *>(cop);
   cudaStream_t s = (cudaStream_t)stream;
   mfgb_status st;
-  if ((st = cuda_status(cudaMemsetAsync(d_dst, 0, sizeof(double) * 3 * op->n_dofs, s), "dst = 0")))
-    return st;
+  if (arith == MFGB_ARITH_FP64_DF && (op->d_Gfx || op->d_G) && (st = ensure_fx(op))) return st;
+  // the start values and identity rows in one launch, as vmult_impl
+  const bool start = starts_in_one(op, 3 * op->n_dofs);
+  st = start ? cuda_status(start_vmult(op->n_dofs, 3, op->d_cbits, d_src, d_dst, s), "start")
+                  : cuda_status(cudaMemsetAsync(d_dst, 0, sizeof(double) * 3 * op->n_dofs, s), "dst = 0");
+  if (st) return st;
   cudaError_t e;
   if (arith == MFGB_ARITH_FP64) {
     e = bk6_f64(op->n, op->n_cells, op->d_map, op->d_G, d_src, d_dst, op->D, s);
   } else if (arith == MFGB_ARITH_FP64_DF && (op->d_Gfx || op->d_G)) {
     // offset double-float, every component scaled per cell: any input range
-    if ((st = ensure_fx(op))) return st;
-    e = bk6_fx(op->n, op->n_cells, op->d_map, op->d_Gfx, op->d_Gexp, d_src, d_dst, op->D, s);
+    e = bk6_fx(op->n, op->n_cells, op->d_map, op->d_Gfx, op->d_Gexp, d_src, d_dst, op->D, s, start);
   } else if (arith == MFGB_ARITH_FP64_DF) {
     if ((st = ensure_df(op)) || (st = range_check_async(op, 3 * op->n_dofs, d_src, s))) return st;
     e = bk6_df(op->n, op->n_cells, op->d_map, op->d_Gdf, d_src, d_dst, op->D, s);
@@ -53,7 +56,7 @@ extern "C" mfgb_status mfgb_vmult_vector(const mfgb_operator *cop, double *d_dst
     return MFGB_ERR_INVALID_ARG;
   }
   if ((st = cuda_status(e, "bk6 kernel"))) return st;
-  if (op->n_constrained)
+  if (op->n_constrained && !start)
     copy_constrained_vec_kernel<<<152 * 8, 256, 0, s>>>(op->n_constrained, op->d_constrained, 3,
                                                         d_src, d_dst);
   return cuda_status(cudaGetLastError(), "bk6 constrained rows");

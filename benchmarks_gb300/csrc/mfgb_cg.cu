@@ -9,14 +9,18 @@
 //
 // GB300 layout of one iteration (all on the device, no host round trip):
 //   1. bk5 apply  v += A p (cell loop)
-//   2. constrained rows v_c = p_c
-//   3. p.v        per-CTA partials (one read of p and v)
-//   4. update     alpha = rz / pAp; x += alpha p; r -= alpha v;
+//   2. p.v        per-CTA partials (one read of p and v)
+//   3. update     alpha = rz / pAp; x += alpha p; r -= alpha v;
 //                 partials of r.r and r.z (z = Dinv r, never stored)
-//   5. direction  |r| test -> done flag; beta; p = z + beta p; v = 0
+//   4. direction  |r| test -> done flag; beta; p = z + beta p; v = 0 with p on the
+//                 constrained rows (operators whose map leaves constrained DoFs in
+//                 copy those rows after 1 instead)
+// The vector passes take one CTA per 1,024 entries, up to 8 CTAs an SM: with the
+// full grid at 1e5 DoFs every CTA summed 1,216 partials for 97 entries of its own.
 // Each kernel returns at once when the done flag is set, so a CUDA graph of
 // K iterations can be replayed until the host sees the flag.  All reductions
 // are two-stage with a fixed order (deterministic).
+#include <algorithm>
 #include <cmath>
 #include <vector>
 
@@ -47,7 +51,10 @@ __global__ void cg_continue_kernel(cudaGraphConditionalHandle h, CgScalars *sc, 
 }
 
 constexpr int VEC_THREADS = 256;
-constexpr int VEC_BLOCKS = 152 * 8;
+constexpr int VEC_BLOCKS = 152 * 8;  // at most
+static int vec_blocks(int64_t n) {
+  return (int)std::max<int64_t>(1, std::min<int64_t>((n + 1023) / 1024, VEC_BLOCKS));
+}
 
 template <int T>
 __device__ __forceinline__ double block_sum(double v, double *sh) {
@@ -132,8 +139,8 @@ __global__ void __launch_bounds__(VEC_THREADS)
 __global__ void __launch_bounds__(VEC_THREADS)
     cg_direction_kernel(int64_t n, const double *__restrict__ r, double *__restrict__ p,
                         double *__restrict__ v, const double *__restrict__ dinv,
-                        const double *__restrict__ partials, int n_part,
-                        CgScalars *__restrict__ sc, int parity) {
+                        const uint32_t *__restrict__ bits, const double *__restrict__ partials,
+                        int n_part, CgScalars *__restrict__ sc, int parity) {
   if (sc->done) return;
   __shared__ double sh[40];
   const double rr = sum_partials(partials, n_part, 2, sh);
@@ -155,8 +162,9 @@ __global__ void __launch_bounds__(VEC_THREADS)
        t += (int64_t)gridDim.x * blockDim.x) {
     const double rt = r[t];
     const double zt = dinv ? dinv[t] * rt : rt;
-    p[t] = __fma_rn(beta, p[t], zt);
-    v[t] = 0.0;
+    const double pt = __fma_rn(beta, p[t], zt);
+    p[t] = pt;
+    v[t] = bits && ((__ldg(bits + (t >> 5)) >> (t & 31)) & 1u) ? pt : 0.0;
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     sc->rz[parity ^ 1] = rz_new;
@@ -215,8 +223,9 @@ int dot_partials_count() { return VEC_BLOCKS; }
 // partials holds dot_partials_count() doubles
 cudaError_t dot_to_device(int64_t n, const double *a, const double *b, double *partials,
                           double *out, cudaStream_t s) {
-  dot_kernel<<<VEC_BLOCKS, VEC_THREADS, 0, s>>>(n, a, b, partials);
-  finish_sum_kernel<<<1, VEC_THREADS, 0, s>>>(partials, VEC_BLOCKS, 1, out);
+  const int nb = vec_blocks(n);
+  dot_kernel<<<nb, VEC_THREADS, 0, s>>>(n, a, b, partials);
+  finish_sum_kernel<<<1, VEC_THREADS, 0, s>>>(partials, nb, 1, out);
   return cudaGetLastError();
 }
 
@@ -257,8 +266,9 @@ extern "C" mfgb_status mfgb_dot(int64_t n, const double *d_a, const double *d_b,
   mfgb_status st = alloc(part, sizeof(double) * (VEC_BLOCKS + 1));
   if (st) return st;
   double *pp = (double *)part.p;
-  dot_kernel<<<VEC_BLOCKS, VEC_THREADS, 0, s>>>(n, d_a, d_b, pp);
-  finish_sum_kernel<<<1, VEC_THREADS, 0, s>>>(pp, VEC_BLOCKS, 1, pp + VEC_BLOCKS);
+  const int nb = vec_blocks(n);
+  dot_kernel<<<nb, VEC_THREADS, 0, s>>>(n, d_a, d_b, pp);
+  finish_sum_kernel<<<1, VEC_THREADS, 0, s>>>(pp, nb, 1, pp + VEC_BLOCKS);
   st = cuda_status(cudaMemcpyAsync(h_result, pp + VEC_BLOCKS, sizeof(double),
                                    cudaMemcpyDeviceToHost, s),
                    "dot copy");
@@ -314,10 +324,10 @@ extern "C" mfgb_status mfgb_cg_solve(const mfgb_operator *cop, const double *d_b
 
   // r0 = b - A x0, p0 = z0
   if ((st = vmult_impl(op, v, d_x, ctl->arith, nullptr, nullptr, s))) return st;
-  cg_init_kernel<<<VEC_BLOCKS, VEC_THREADS, 0, s>>>(n, d_b, v, r, p, dinv, vec_part);
-  finish_sum_kernel<<<1, VEC_THREADS, 0, s>>>(vec_part, VEC_BLOCKS, 2, vec_part + 2 * VEC_BLOCKS);
-  finish_sum_kernel<<<1, VEC_THREADS, 0, s>>>(vec_part + 1, VEC_BLOCKS, 2,
-                                              vec_part + 2 * VEC_BLOCKS + 1);
+  const int nb = vec_blocks(n);
+  cg_init_kernel<<<nb, VEC_THREADS, 0, s>>>(n, d_b, v, r, p, dinv, vec_part);
+  finish_sum_kernel<<<1, VEC_THREADS, 0, s>>>(vec_part, nb, 2, vec_part + 2 * VEC_BLOCKS);
+  finish_sum_kernel<<<1, VEC_THREADS, 0, s>>>(vec_part + 1, nb, 2, vec_part + 2 * VEC_BLOCKS + 1);
   double h2[2];
   if ((st = cuda_status(cudaMemcpyAsync(h2, vec_part + 2 * VEC_BLOCKS, 2 * sizeof(double),
                                         cudaMemcpyDeviceToHost, s),
@@ -350,7 +360,12 @@ extern "C" mfgb_status mfgb_cg_solve(const mfgb_operator *cop, const double *d_b
   if ((st = cuda_status(cudaMemcpyAsync(sc, &hsc, sizeof(hsc), cudaMemcpyHostToDevice, s),
                         "cg scalars")))
     return st;
-  if ((st = cuda_status(cudaMemsetAsync(v, 0, sizeof(double) * n, s), "v = 0"))) return st;
+  // v before the first application: 0, and p on the constrained rows where the map is masked
+  const uint32_t *bits = op->masked ? op->d_cbits : nullptr;
+  if ((st = cuda_status(bits ? start_vmult(n, 1, bits, p, v, s)
+                             : cudaMemsetAsync(v, 0, sizeof(double) * n, s),
+                        "v = 0")))
+    return st;
 
   // K iterations (parity alternates, K even) captured as the body of a
   // conditional while node: one graph launch runs the whole solve on the device
@@ -399,14 +414,13 @@ extern "C" mfgb_status mfgb_cg_solve(const mfgb_operator *cop, const double *d_b
       const int parity = k & 1;
       cap_st = apply_add_impl(op, v, p, ctl->arith, s, &sc->done);
       if (cap_st) break;
-      if (op->n_constrained)
+      if (op->n_constrained && !op->masked)
         cg_constrained_copy_kernel<<<VEC_BLOCKS, VEC_THREADS, 0, s>>>(op->n_constrained,
                                                                       op->d_constrained, p, v, sc);
-      cg_dot_pv_kernel<<<VEC_BLOCKS, VEC_THREADS, 0, s>>>(n, p, v, pap_part, sc);
-      cg_update_kernel<<<VEC_BLOCKS, VEC_THREADS, 0, s>>>(n, d_x, r, p, v, dinv, pap_part,
-                                                          VEC_BLOCKS, vec_part, sc, parity);
-      cg_direction_kernel<<<VEC_BLOCKS, VEC_THREADS, 0, s>>>(n, r, p, v, dinv, vec_part,
-                                                             VEC_BLOCKS, sc, parity);
+      cg_dot_pv_kernel<<<nb, VEC_THREADS, 0, s>>>(n, p, v, pap_part, sc);
+      cg_update_kernel<<<nb, VEC_THREADS, 0, s>>>(n, d_x, r, p, v, dinv, pap_part, nb, vec_part, sc,
+                                                  parity);
+      cg_direction_kernel<<<nb, VEC_THREADS, 0, s>>>(n, r, p, v, dinv, bits, vec_part, nb, sc, parity);
     }
     if (looped && !cap_st)
       cg_continue_kernel<<<1, 1, 0, s>>>(cond_h, sc, ctl->max_steps / K + 2);
@@ -587,10 +601,10 @@ extern "C" mfgb_status mfgb_cg_solve_noalloc(const mfgb_operator *op, const doub
   // r0 = b - A x0, p0 = z0
   if ((st = noalloc_apply(op, v, d_x, ctl->arith, nullptr, nullptr, s, nullptr, range_slot)))
     return st;
-  cg_init_kernel<<<VEC_BLOCKS, VEC_THREADS, 0, s>>>(n, d_b, v, r, p, dinv, vec_part);
-  finish_sum_kernel<<<1, VEC_THREADS, 0, s>>>(vec_part, VEC_BLOCKS, 2, vec_part + 2 * VEC_BLOCKS);
-  finish_sum_kernel<<<1, VEC_THREADS, 0, s>>>(vec_part + 1, VEC_BLOCKS, 2,
-                                              vec_part + 2 * VEC_BLOCKS + 1);
+  const int nb = vec_blocks(n);
+  cg_init_kernel<<<nb, VEC_THREADS, 0, s>>>(n, d_b, v, r, p, dinv, vec_part);
+  finish_sum_kernel<<<1, VEC_THREADS, 0, s>>>(vec_part, nb, 2, vec_part + 2 * VEC_BLOCKS);
+  finish_sum_kernel<<<1, VEC_THREADS, 0, s>>>(vec_part + 1, nb, 2, vec_part + 2 * VEC_BLOCKS + 1);
   double h2[2];
   if ((st = cuda_status(cudaMemcpyAsync(h2, vec_part + 2 * VEC_BLOCKS, 2 * sizeof(double),
                                         cudaMemcpyDeviceToHost, s),
@@ -615,6 +629,7 @@ extern "C" mfgb_status mfgb_cg_solve_noalloc(const mfgb_operator *op, const doub
   }
   if (ctl->max_steps == 0) return MFGB_ERR_NOT_CONVERGED;
 
+  const uint32_t *bits = op->masked ? op->d_cbits : nullptr;
   CgScalars hsc{};
   hsc.rz[0] = h2[1];
   hsc.res[0] = res0;
@@ -624,7 +639,9 @@ extern "C" mfgb_status mfgb_cg_solve_noalloc(const mfgb_operator *op, const doub
   hsc.done = 0;
   if ((st = cuda_status(cudaMemcpyAsync(sc, &hsc, sizeof(hsc), cudaMemcpyHostToDevice, s),
                         "cg scalars")) ||
-      (st = cuda_status(cudaMemsetAsync(v, 0, sizeof(double) * n, s), "v = 0")))
+      (st = cuda_status(bits ? start_vmult(n, 1, bits, p, v, s)
+                             : cudaMemsetAsync(v, 0, sizeof(double) * n, s),
+                        "v = 0")))
     return st;
 
   const int K = 16;  // iterations between host checks of the done flag
@@ -635,14 +652,13 @@ extern "C" mfgb_status mfgb_cg_solve_noalloc(const mfgb_operator *op, const doub
       if ((st = noalloc_apply(op, v, p, ctl->arith, nullptr, nullptr, s, &sc->done, range_slot,
                               /*accumulate=*/true)))
         return st;
-      if (op->n_constrained)
+      if (op->n_constrained && !op->masked)
         cg_constrained_copy_kernel<<<VEC_BLOCKS, VEC_THREADS, 0, s>>>(op->n_constrained,
                                                                       op->d_constrained, p, v, sc);
-      cg_dot_pv_kernel<<<VEC_BLOCKS, VEC_THREADS, 0, s>>>(n, p, v, pap_part, sc);
-      cg_update_kernel<<<VEC_BLOCKS, VEC_THREADS, 0, s>>>(n, d_x, r, p, v, dinv, pap_part,
-                                                          VEC_BLOCKS, vec_part, sc, parity);
-      cg_direction_kernel<<<VEC_BLOCKS, VEC_THREADS, 0, s>>>(n, r, p, v, dinv, vec_part,
-                                                             VEC_BLOCKS, sc, parity);
+      cg_dot_pv_kernel<<<nb, VEC_THREADS, 0, s>>>(n, p, v, pap_part, sc);
+      cg_update_kernel<<<nb, VEC_THREADS, 0, s>>>(n, d_x, r, p, v, dinv, pap_part, nb, vec_part, sc,
+                                                  parity);
+      cg_direction_kernel<<<nb, VEC_THREADS, 0, s>>>(n, r, p, v, dinv, bits, vec_part, nb, sc, parity);
     }
     if ((st = cuda_status(cudaGetLastError(), "cg iterations")) ||
         (st = cuda_status(cudaMemcpyAsync(&out, sc, sizeof(out), cudaMemcpyDeviceToHost, s),

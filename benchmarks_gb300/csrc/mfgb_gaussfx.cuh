@@ -417,6 +417,7 @@ __global__ void __launch_bounds__(E * NQ * NQ, MB)
       df x[NQ], y[NM];
       load_line(x, U + col, 1);
       fx_line(basis.Bt, x, y);
+      if (!EVEC) cudaGridDependencySynchronize();  // dst has its start values
       auto put = [&](int i, double v) {
         if constexpr (EVEC) {  // the column's own place, written out below
           reinterpret_cast<double *>(U)[col + i] = v;

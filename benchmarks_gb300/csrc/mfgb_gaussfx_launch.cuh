@@ -77,7 +77,8 @@ inline bool fill_gauss(const double *B, const double *D, GaussBasis<NM, NQ, SYM>
 template <int NM, int NQ, class GT, bool EVEC, bool SYM, bool MASS, bool MT>
 inline cudaError_t gaussfx_run(int64_t n_cells, const uint32_t *map, const GT *G, const int *gexp,
                                const double *src, double *dst, const GaussBasis<NM, NQ, SYM> &b,
-                               cudaStream_t s, const int *done, const float2 *jxw) {
+                               cudaStream_t s, const int *done, const float2 *jxw,
+                               bool after = false) {
   using Sh = GaussShape<NM, NQ>;
   constexpr int E = Sh::E, T = E * NQ * NQ;
   constexpr size_t smem = GaussLayout<NM, NQ, E, EVEC, 6, 2>::total;
@@ -86,8 +87,8 @@ inline cudaError_t gaussfx_run(int64_t n_cells, const uint32_t *map, const GT *G
   if (per_sm < 0) per_sm = std::max(1, ctas_per_sm(kernel, T, smem));
   const int64_t batches = (n_cells + E - 1) / E;
   const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(batches, (int64_t)per_sm * num_sms()));
-  kernel<<<grid, T, smem, s>>>(n_cells, map, G, gexp, src, dst, b, done, device_error_flag(), jxw);
-  return cudaGetLastError();
+  return launch_after(after, kernel, grid, T, smem, s, n_cells, map, G, gexp, src, dst, b, done,
+                      device_error_flag(), jxw);
 }
 
 // The library's own operators on L-vectors.  Bulk copies of the dof-map tiles need a 16-byte
@@ -96,14 +97,14 @@ template <int NM, int NQ, bool MASS>
 inline cudaError_t gaussfx_pairs(int64_t n_cells, const uint32_t *map, const float2 *G,
                                  const int *gexp, const double *src, double *dst, const double *hB,
                                  const double *hDG, cudaStream_t s, const int *done,
-                                 const float2 *jxw) {
+                                 const float2 *jxw, bool after) {
   GaussBasis<NM, NQ, true> b;
   if (!fill_gauss(hB, hDG, b)) return cudaErrorInvalidValue;  // GLL and Gauss points are symmetric
   if (reinterpret_cast<uintptr_t>(map) & 15u)
     return gaussfx_run<NM, NQ, float2, false, true, MASS, false>(n_cells, map, G, gexp, src, dst, b,
-                                                                 s, done, jxw);
+                                                                 s, done, jxw, after);
   return gaussfx_run<NM, NQ, float2, false, true, MASS, true>(n_cells, map, G, gexp, src, dst, b, s,
-                                                              done, jxw);
+                                                              done, jxw, after);
 }
 
 }  // namespace mfgb

@@ -20,6 +20,10 @@ struct mfgb_operator {
   int *d_Gexp = nullptr;          // the per-cell exponent offsets of d_Gfx
   int *d_range = nullptr;         // slot of the double-float input range check
   int64_t *d_constrained = nullptr;
+  uint32_t *d_cbits = nullptr;    // one bit per DoF: constrained
+  // no map entry refers to a constrained DoF, so a result's identity rows may be written before the
+  // cell loop (always true on boxes; a caller's map may leave constrained DoFs in)
+  bool masked = false;
   double D[81] = {0};             // derivative matrix D[q*n + b]
   double gll_x[9] = {0}, gll_w[9] = {0};
   int quadrature = 0;             // 0: GLL collocation, 1: Gauss p+1 (BP5 variant), 2: Gauss p+2 (BP3)
@@ -68,11 +72,12 @@ cudaError_t bk5_df(int N, int64_t n_cells, const uint32_t *map, const float2 *G,
 // per-cell scaling (mfgb_bk5_fx.cu); G = the scaled pairs, gexp their offsets
 cudaError_t bk5_fx(int N, int64_t n_cells, const uint32_t *map, const float2 *G, const int *gexp,
                    const double *src, double *dst, const double *D, cudaStream_t s,
-                   const int *done = nullptr);
+                   const int *done = nullptr, bool after_start = false);
 // the BK6 vector Laplacian on the scaled pairs of bk5_fx: src / dst hold 3
 // interleaved components per DoF, each component scaled per cell on its own
 cudaError_t bk6_fx(int N, int64_t n_cells, const uint32_t *map, const float2 *G, const int *gexp,
-                   const double *src, double *dst, const double *D, cudaStream_t s);
+                   const double *src, double *dst, const double *D, cudaStream_t s,
+                   bool after_start = false);
 // bk5_fx on the caller's FP64 G[cell][6][N^3] (16-byte aligned) scaled per
 // cell inside the kernel, for the BK5 L-vector seam: dst += A src through map
 cudaError_t bk5_fx_g64(int N, int64_t n_cells, const uint32_t *map, const double *G,
@@ -150,13 +155,14 @@ cudaError_t dot_to_device(int64_t n, const double *a, const double *b, double *p
 cudaError_t bp3_fx(int degree, int nq, int64_t n_cells, const uint32_t *map, const float2 *Gfx,
                    const int *gexp, const double *src, double *dst, const double *hB,
                    const double *hDG, cudaStream_t s, const int *done,
-                   const float2 *jxw = nullptr);
+                   const float2 *jxw = nullptr, bool after_start = false);
 // the Helmholtz form of bp3_fx (nq = degree + 1, mfgb_helmholtz_fx.cu): the
 // Gauss p+1 Laplacian plus the mass term from jxw, JxW pairs [cell][nq^3] on
 // the scale of Gfx
 cudaError_t helmholtz_fx(int degree, int64_t n_cells, const uint32_t *map, const float2 *Gfx,
                          const int *gexp, const float2 *jxw, const double *src, double *dst,
-                         const double *hB, const double *hDG, cudaStream_t s, const int *done);
+                         const double *hB, const double *hDG, cudaStream_t s, const int *done,
+                         bool after_start = false);
 // CEED BK1 mass operator on E-vectors with offset double-float accumulation and
 // per-element scaling (mfgb_bp3_fx.cu): out = B^T (JxW o B in) per element,
 // host copy of the basis hB[q*nm+i], nq = degree + 2
@@ -184,6 +190,15 @@ cudaError_t diagonal_f64(int N, int64_t n_cells, const uint32_t *map, const doub
                          const double *D, double *diag, cudaStream_t s);
 cudaError_t set_constrained(int64_t n_constrained, const int64_t *constrained, double *v,
                             double value, cudaStream_t s);
+// bits = 0 (n bits), then the listed ones set
+cudaError_t set_cbits(int64_t n, int64_t n_constrained, const int64_t *constrained, uint32_t *bits,
+                      cudaStream_t s);
+// dst = 0 with src on the constrained DoFs (ncomp values per DoF), before a masked operator
+// accumulates into dst.  A kernel launched after it with after_start = true may begin before it has
+// ended and waits for it before its first write to dst (programmatic dependent launch).
+cudaError_t start_vmult(int64_t n, int ncomp, const uint32_t *bits, const double *src, double *dst,
+                        cudaStream_t s);
+bool starts_in_one(const mfgb_operator *op, int64_t n);  // (mfgb_api.cu)
 cudaError_t copy_constrained(int64_t n_constrained, const int64_t *constrained, const double *src,
                              double *dst, cudaStream_t s);
 cudaError_t invert_diagonal(int64_t n, double *d, cudaStream_t s);

@@ -103,6 +103,24 @@ int ctas_per_sm(K kernel, int threads, size_t smem) {
   return ps;
 }
 
+// One launch; after = true: it may begin while the kernel before it on the stream (which must let it,
+// start_vmult) still runs, and waits for that one's end inside (cudaGridDependencySynchronize).
+template <class... P, class... Q>
+cudaError_t launch_after(bool after, void (*kernel)(P...), int grid, int threads, size_t smem,
+                         cudaStream_t s, Q... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = after ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // Shapes 2 and 4 of the plain arithmetics as the line kernel (mfgb_bk5line.cuh): cells per CTA,
 // resident CTAs and work arrays.  FP32 at every degree, FP64 from N = 6 (below, the column kernel's
 // 4.05 / 3.82 ms at N = 4, 5 are not beaten: 4.62 / 3.86; the FP64 pipe is the bound and the even-odd

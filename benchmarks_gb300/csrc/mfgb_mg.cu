@@ -554,7 +554,7 @@ void free_mg(mfgb_mg *mg) {
   if (!mg) return;
   for (auto &L : mg->levels) {
     cudaFree(L.x); cudaFree(L.b); cudaFree(L.r); cudaFree(L.d); cudaFree(L.t);
-    cudaFree(L.inv_diag); cudaFree(L.inv_val); cudaFree(L.bits);
+    cudaFree(L.inv_diag); cudaFree(L.inv_val);
     if (L.op && !L.borrowed) mfgb_operator_destroy(L.op);
   }
   cudaFree(mg->coarse.A); cudaFree(mg->coarse.dinv); cudaFree(mg->coarse.work);
@@ -638,12 +638,9 @@ static mfgb_status mg_setup_impl(const mfgb_box_desc *fine, const mfgb_mg_params
     MgLevel &M = mg->levels.back();
     if ((st = dalloc(&M.x, ts * M.n)) || (st = dalloc(&M.b, ts * M.n)) ||
         (st = dalloc(&M.r, ts * M.n)) || (st = dalloc(&M.d, ts * M.n)) ||
-        (st = dalloc(&M.t, ts * M.n)) || (st = dalloc(&M.inv_diag, ts * M.n)) ||
-        (st = dalloc((void **)&M.bits, sizeof(uint32_t) * ((M.n + 31) / 32))))
+        (st = dalloc(&M.t, ts * M.n)) || (st = dalloc(&M.inv_diag, ts * M.n)))
       break;
-    cudaMemset(M.bits, 0, sizeof(uint32_t) * ((M.n + 31) / 32));
-    if (M.op->n_constrained)
-      k_set_bits<<<grid1d(M.op->n_constrained), T256>>>(M.op->n_constrained, M.op->d_constrained, M.bits);
+    M.bits = M.op->d_cbits;
     if (prm->precision == 32 && (st = ensure_g32(M.op))) break;
     if (prm->precision == 64 && (st = ensure_arith(M.op, MFGB_ARITH_FP64_DF))) break;
     // Jacobi in the V-cycle precision

@@ -14,7 +14,7 @@ struct MgLevel {
   int64_t n = 0;
   void *x = nullptr, *b = nullptr, *r = nullptr, *d = nullptr, *t = nullptr;
   void *inv_diag = nullptr;  // Jacobi (precision T)
-  uint32_t *bits = nullptr;  // one bit per DoF: constrained
+  const uint32_t *bits = nullptr;  // one bit per DoF: constrained (the operator's)
   void *inv_val = nullptr;   // 1/valence (precision T), for p-restriction from this level
   double lmax = 0;
   int to_coarse = 0;  // 1 = p-transfer, 2 = h-transfer, 0 = coarsest

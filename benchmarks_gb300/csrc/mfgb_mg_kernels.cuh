@@ -63,9 +63,6 @@ __global__ void k_convert(int64_t n, const TI *__restrict__ a, TO *__restrict__ 
 // that the next application can accumulate into it: no clearing pass and launch of its own.  The
 // identity rows of the constrained DoFs are taken from the operator's input instead of being copied
 // into its result: `bits` has one bit per DoF, set where it is constrained.
-__global__ void k_set_bits(int64_t nc, const int64_t *__restrict__ c, uint32_t *__restrict__ bits) {
-  GRID_STRIDE(t, nc) atomicOr(bits + (c[t] >> 5), 1u << (c[t] & 31));
-}
 __device__ __forceinline__ bool bit_at(const uint32_t *__restrict__ bits, int64_t t) {
   return (__ldg(bits + (t >> 5)) >> (t & 31)) & 1u;
 }

@@ -197,3 +197,48 @@ def test_plain_line_kernels(p):
     finally:
         for a, v in old.items():
             L.mfgb_set_kernel_shape(a, p, v.value)
+
+
+@pytest.mark.gpu
+def test_start_values_of_masked_and_unmasked_operators():
+    """Identity rows and cleared rows before the cell loop: vector lengths around the 256 entries a
+    warp clears, unaligned results, three components; a caller's map that leaves constrained DoFs
+    in keeps their rows as plain copies."""
+    import torch
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import benchmarks_gb300 as mf
+    from oracle import oracle
+    rng = np.random.default_rng(0)
+    for cells, p in (((1, 1, 1), 1), ((2, 1, 1), 4), ((6, 5, 7), 1), ((9, 11, 10), 2)):
+        A = mf.LaplaceOperator(mf.BoxMesh(*cells, degree=p))
+        ref = oracle.BoxProblem(*cells, p, amplitude=0.05)
+        n = ref.n_dofs
+        src = rng.uniform(-1, 1, n)
+        want = ref.apply(src)
+        for shift in (0, 1):
+            u = torch.from_numpy(np.concatenate([np.zeros(shift), src])).cuda()[shift:]
+            y = torch.full((n + shift,), 7.0, dtype=torch.float64, device="cuda")[shift:]
+            for arith in ("df", "fp64"):
+                got = A.vmult(y.fill_(7.0), u, arith=arith).cpu().numpy()
+                assert np.linalg.norm(got - want) <= 1e-12 * np.linalg.norm(want)
+                assert np.array_equal(got[ref.constrained], src[ref.constrained])
+        v = np.stack([src, 2 * src, -src], -1).reshape(-1)
+        got = A.vmult_vector(torch.full((3 * n,), 7.0, dtype=torch.float64, device="cuda"),
+                             torch.from_numpy(v).cuda()).cpu().numpy()
+        w = np.stack([want, 2 * want, -want], -1).reshape(-1)
+        assert np.linalg.norm(got - w) <= 1e-12 * np.linalg.norm(w)
+    # constrained DoFs left in the map: their rows are overwritten by the source
+    p, cells = 3, 4
+    nn = (p + 1) ** 3
+    dof_map = np.arange(cells * nn, dtype=np.uint32)
+    fixed = np.array([0, 5, nn, 3 * nn + 7], dtype=np.int64)
+    G = rng.uniform(0.5, 1.5, cells * 6 * nn)
+    B = mf.LaplaceOperator(degree=p, n_dofs=cells * nn, dof_map=dof_map, G=G, constrained=fixed)
+    D = oracle.derivative_matrix(oracle.gll(p + 1)[0])
+    src = rng.uniform(-1, 1, cells * nn)
+    want = oracle.apply(p + 1, dof_map, D, G, cells * nn, fixed, src)
+    u = torch.from_numpy(src).cuda()
+    got = B.vmult(torch.zeros_like(u), u).cpu().numpy()
+    assert np.linalg.norm(got - want) <= 1e-12 * np.linalg.norm(want)
+    assert np.array_equal(got[fixed], src[fixed])
