@@ -15,8 +15,10 @@
 //   4. direction  |r| test -> done flag; beta; p = z + beta p; v = 0 with p on the
 //                 constrained rows (operators whose map leaves constrained DoFs in
 //                 copy those rows after 1 instead)
-// The vector passes take one CTA per 1,024 entries, up to 8 CTAs an SM: with the
-// full grid at 1e5 DoFs every CTA summed 1,216 partials for 97 entries of its own.
+// The vector passes take one CTA per 1,024 entries, at most 2 an SM up to 5e6 entries
+// and 8 above: with the full grid at 1e5 DoFs every CTA summed 1,216 partials for 97
+// entries of its own, and at 1e6 the FP64 sums of 1,006 CTAs took longer than the pass
+// (update 33 us, direction 28 us).
 // Each kernel returns at once when the done flag is set, so a CUDA graph of
 // K iterations can be replayed until the host sees the flag.  All reductions
 // are two-stage with a fixed order (deterministic).
@@ -53,32 +55,22 @@ __global__ void cg_continue_kernel(cudaGraphConditionalHandle h, CgScalars *sc, 
 constexpr int VEC_THREADS = 256;
 constexpr int VEC_BLOCKS = 152 * 8;  // at most
 static int vec_blocks(int64_t n) {
-  return (int)std::max<int64_t>(1, std::min<int64_t>((n + 1023) / 1024, VEC_BLOCKS));
+  const int64_t most = n < (int64_t)VEC_BLOCKS * 4096 ? 152 * 2 : VEC_BLOCKS;
+  return (int)std::max<int64_t>(1, std::min<int64_t>((n + 1023) / 1024, most));
 }
 
-template <int T>
-__device__ __forceinline__ double block_sum(double v, double *sh) {
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  __syncthreads();
-  if (lane == 0) sh[w] = v;
-  __syncthreads();
-  double s = 0.0;
-  if (threadIdx.x == 0)
-    for (int i = 0; i < T / 32; ++i) s += sh[i];
-  return s;  // valid in thread 0
-}
-
-// every CTA sums the same partials in the same order -> identical result
+// every CTA sums the same partials in the same order -> identical result; thread 0 maps it (a
+// division by every thread costs more than the pass over the vectors at 1e6 DoFs)
+template <class F>
 __device__ __forceinline__ double sum_partials(const double *__restrict__ p, int n, int stride,
-                                               double *sh) {
+                                               double *sh, F f) {
   double v = 0.0;
   for (int i = threadIdx.x; i < n; i += blockDim.x) v += p[(size_t)i * stride];
-  double s = block_sum<VEC_THREADS>(v, sh);
-  __syncthreads();
-  if (threadIdx.x == 0) sh[32] = s;
-  __syncthreads();
-  return sh[32];
+  return cta_sum_map<VEC_THREADS>(v, sh, f);
+}
+__device__ __forceinline__ double sum_partials(const double *__restrict__ p, int n, int stride,
+                                               double *sh) {
+  return sum_partials(p, n, stride, sh, [](double v) { return v; });
 }
 
 // identity rows of the constrained DoFs: v_c = p_c (many CTAs)
@@ -97,12 +89,12 @@ __global__ void __launch_bounds__(VEC_THREADS)
     cg_dot_pv_kernel(int64_t n, const double *__restrict__ p, const double *__restrict__ v,
                      double *__restrict__ partials, const CgScalars *__restrict__ sc) {
   if (sc->done) return;
-  __shared__ double sh[40];
+  __shared__ double sh[VEC_THREADS];
   double s = 0.0;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n;
        t += (int64_t)gridDim.x * blockDim.x)
     s = __fma_rn(p[t], v[t], s);
-  const double bs = block_sum<VEC_THREADS>(s, sh);
+  const double bs = cta_sum_tree<VEC_THREADS>(s, sh);
   if (threadIdx.x == 0) partials[blockIdx.x] = bs;
 }
 
@@ -113,9 +105,9 @@ __global__ void __launch_bounds__(VEC_THREADS)
                      int n_pap, double *__restrict__ out_partials, CgScalars *__restrict__ sc,
                      int parity) {
   if (sc->done) return;
-  __shared__ double sh[40];
-  const double pap = sum_partials(pap_partials, n_pap, 1, sh);
-  const double alpha = sc->rz[parity] / pap;
+  __shared__ double sh[VEC_THREADS];
+  const double alpha = sum_partials(pap_partials, n_pap, 1, sh,
+                                    [&](double pap) { return sc->rz[parity] / pap; });
   double rr = 0.0, rz = 0.0;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n;
        t += (int64_t)gridDim.x * blockDim.x) {
@@ -127,9 +119,9 @@ __global__ void __launch_bounds__(VEC_THREADS)
     rr = __fma_rn(rt, rt, rr);
     rz = __fma_rn(rt, zt, rz);
   }
-  const double srr = block_sum<VEC_THREADS>(rr, sh);
+  const double srr = cta_sum_tree<VEC_THREADS>(rr, sh);
   __syncthreads();
-  const double srz = block_sum<VEC_THREADS>(rz, sh);
+  const double srz = cta_sum_tree<VEC_THREADS>(rz, sh);
   if (threadIdx.x == 0) {
     out_partials[2 * blockIdx.x] = srr;
     out_partials[2 * blockIdx.x + 1] = srz;
@@ -142,10 +134,8 @@ __global__ void __launch_bounds__(VEC_THREADS)
                         const uint32_t *__restrict__ bits, const double *__restrict__ partials,
                         int n_part, CgScalars *__restrict__ sc, int parity) {
   if (sc->done) return;
-  __shared__ double sh[40];
-  const double rr = sum_partials(partials, n_part, 2, sh);
-  const double rz_new = sum_partials(partials + 1, n_part, 2, sh);
-  const double res = sqrt(rr);
+  __shared__ double sh[VEC_THREADS];
+  const double res = sum_partials(partials, n_part, 2, sh, [](double rr) { return sqrt(rr); });
   const int it = sc->its[parity] + 1;
   const bool converged = res <= sc->tol_eff;
   const bool failed = !converged && (it >= sc->max_steps || isnan(res));
@@ -157,7 +147,11 @@ __global__ void __launch_bounds__(VEC_THREADS)
     }
     return;
   }
-  const double beta = rz_new / sc->rz[parity];
+  double rz_new = 0.0;  // in thread 0
+  const double beta = sum_partials(partials + 1, n_part, 2, sh, [&](double rz) {
+    rz_new = rz;
+    return rz / sc->rz[parity];
+  });
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n;
        t += (int64_t)gridDim.x * blockDim.x) {
     const double rt = r[t];
@@ -178,7 +172,7 @@ __global__ void __launch_bounds__(VEC_THREADS)
     cg_init_kernel(int64_t n, const double *__restrict__ b, const double *__restrict__ v,
                    double *__restrict__ r, double *__restrict__ p, const double *__restrict__ dinv,
                    double *__restrict__ out_partials) {
-  __shared__ double sh[40];
+  __shared__ double sh[VEC_THREADS];
   double rr = 0.0, rz = 0.0;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n;
        t += (int64_t)gridDim.x * blockDim.x) {
@@ -189,9 +183,9 @@ __global__ void __launch_bounds__(VEC_THREADS)
     rr = __fma_rn(rt, rt, rr);
     rz = __fma_rn(rt, zt, rz);
   }
-  const double srr = block_sum<VEC_THREADS>(rr, sh);
+  const double srr = cta_sum_tree<VEC_THREADS>(rr, sh);
   __syncthreads();
-  const double srz = block_sum<VEC_THREADS>(rz, sh);
+  const double srz = cta_sum_tree<VEC_THREADS>(rz, sh);
   if (threadIdx.x == 0) {
     out_partials[2 * blockIdx.x] = srr;
     out_partials[2 * blockIdx.x + 1] = srz;
@@ -201,18 +195,18 @@ __global__ void __launch_bounds__(VEC_THREADS)
 __global__ void __launch_bounds__(VEC_THREADS)
     dot_kernel(int64_t n, const double *__restrict__ a, const double *__restrict__ b,
                double *__restrict__ partials) {
-  __shared__ double sh[40];
+  __shared__ double sh[VEC_THREADS];
   double s = 0.0;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n;
        t += (int64_t)gridDim.x * blockDim.x)
     s = __fma_rn(a[t], b[t], s);
-  const double bs = block_sum<VEC_THREADS>(s, sh);
+  const double bs = cta_sum_tree<VEC_THREADS>(s, sh);
   if (threadIdx.x == 0) partials[blockIdx.x] = bs;
 }
 
 __global__ void finish_sum_kernel(const double *__restrict__ partials, int n, int stride,
                                   double *__restrict__ out) {
-  __shared__ double sh[40];
+  __shared__ double sh[VEC_THREADS];
   const double s = sum_partials(partials, n, stride, sh);
   if (threadIdx.x == 0) *out = s;
 }

@@ -111,34 +111,23 @@ __global__ void __launch_bounds__(T256)
 }
 
 // ---- outer FP64 PCG kernels ----------------------------------------------
-__device__ __forceinline__ double warp_block_sum(double v, double *sh) {
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-  __syncthreads();
-  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
-  __syncthreads();
-  double s = 0;
-  if (threadIdx.x == 0)
-    for (int w = 0; w < T256 / 32; ++w) s += sh[w];
-  return s;
-}
-
 // partial sums of a.b per CTA (deterministic order)
 __global__ void __launch_bounds__(T256)
     k_dot_partials(int64_t n, const double *__restrict__ a, const double *__restrict__ b,
                    double *__restrict__ part) {
-  __shared__ double sh[T256 / 32];
+  __shared__ double sh[T256];
   double s = 0;
   GRID_STRIDE(t, n) s = fma(a[t], b[t], s);
-  s = warp_block_sum(s, sh);
+  s = cta_sum_tree<T256>(s, sh);
   if (threadIdx.x == 0) part[blockIdx.x] = s;
 }
 
 __global__ void __launch_bounds__(T256)
     k_sum_partials(const double *__restrict__ part, int n, double *__restrict__ out) {
-  __shared__ double sh[T256 / 32];
+  __shared__ double sh[T256];
   double s = 0;
   for (int i = threadIdx.x; i < n; i += blockDim.x) s += part[i];
-  s = warp_block_sum(s, sh);
+  s = cta_sum_tree<T256>(s, sh);
   if (threadIdx.x == 0) *out = s;
 }
 
@@ -150,16 +139,11 @@ __global__ void __launch_bounds__(T256)
 // sc: [0] r.z of the current direction, [1] r.z new, [3] |r|^2.
 constexpr int PCG_BLOCKS = 152 * 6;
 
-__device__ __forceinline__ double all_partials(const double *__restrict__ part, double *sh) {
+template <class F>
+__device__ __forceinline__ double all_partials(const double *__restrict__ part, double *sh, F f) {
   double s = 0;
   for (int i = threadIdx.x; i < PCG_BLOCKS; i += T256) s += part[i];
-  s = warp_block_sum(s, sh);
-  __syncthreads();
-  if (threadIdx.x == 0) sh[0] = s;
-  __syncthreads();
-  s = sh[0];
-  __syncthreads();
-  return s;
+  return cta_sum_map<T256>(s, sh, f);
 }
 
 // partials of r.z
@@ -167,7 +151,7 @@ template <class T>
 __global__ void __launch_bounds__(T256)
     k_pcg_rz(int64_t n, const double *__restrict__ r, const T *__restrict__ z,
              double *__restrict__ part) {
-  __shared__ double sh[T256 / 32];
+  __shared__ double sh[T256];
   double s = 0;
   constexpr int W = Pack<T>::W;
   GRID_STRIDE(q, n / W) {
@@ -181,7 +165,7 @@ __global__ void __launch_bounds__(T256)
     }
   }
   GRID_STRIDE(q, n % W) s = fma(r[n / W * W + q], (double)z[n / W * W + q], s);
-  s = warp_block_sum(s, sh);
+  s = cta_sum_tree<T256>(s, sh);
   if (threadIdx.x == 0) part[blockIdx.x] = s;
 }
 
@@ -192,9 +176,11 @@ __global__ void __launch_bounds__(T256)
     k_pcg_direction(int64_t n, const T *__restrict__ z, double *__restrict__ p,
                     double *__restrict__ v, const uint32_t *__restrict__ bits,
                     const double *__restrict__ part, double *__restrict__ sc) {
-  __shared__ double sh[T256 / 32];
-  const double rz = all_partials(part, sh), beta = rz / sc[0];
-  if (blockIdx.x == 0 && threadIdx.x == 0) sc[1] = rz;
+  __shared__ double sh[T256];
+  const double beta = all_partials(part, sh, [&](double rz) {
+    if (blockIdx.x == 0) sc[1] = rz;
+    return rz / sc[0];
+  });
   constexpr int W = Pack<T>::W;
   GRID_STRIDE(q, n / W) {
     const int64_t t = q * W;
@@ -223,7 +209,7 @@ __global__ void __launch_bounds__(T256)
 __global__ void __launch_bounds__(T256)
     k_pcg_pv(int64_t n, const double *__restrict__ p, const double *__restrict__ v,
              double *__restrict__ part, double *__restrict__ sc) {
-  __shared__ double sh[T256 / 32];
+  __shared__ double sh[T256];
   if (blockIdx.x == 0 && threadIdx.x == 0) sc[0] = sc[1];
   double s = 0;
   GRID_STRIDE(q, n / 2) {
@@ -232,7 +218,7 @@ __global__ void __launch_bounds__(T256)
     s = fma(a.v[1], b.v[1], s);
   }
   if (n % 2 && blockIdx.x == 0 && threadIdx.x == 0) s = fma(p[n - 1], v[n - 1], s);
-  s = warp_block_sum(s, sh);
+  s = cta_sum_tree<T256>(s, sh);
   if (threadIdx.x == 0) part[blockIdx.x] = s;
 }
 
@@ -243,8 +229,8 @@ __global__ void __launch_bounds__(T256)
                  const double *__restrict__ p, const double *__restrict__ v, T *__restrict__ b,
                  const double *__restrict__ pv_part, const double *__restrict__ sc,
                  double *__restrict__ part) {
-  __shared__ double sh[T256 / 32];
-  const double alpha = sc[0] / all_partials(pv_part, sh);
+  __shared__ double sh[T256];
+  const double alpha = all_partials(pv_part, sh, [&](double pv) { return sc[0] / pv; });
   double s = 0;
   GRID_STRIDE(t, n) {  // (x is the caller's: no alignment beyond its own)
     x[t] = fma(alpha, p[t], x[t]);
@@ -253,7 +239,7 @@ __global__ void __launch_bounds__(T256)
     b[t] = (T)rt;
     s = fma(rt, rt, s);
   }
-  s = warp_block_sum(s, sh);
+  s = cta_sum_tree<T256>(s, sh);
   if (threadIdx.x == 0) part[blockIdx.x] = s;
 }
 
