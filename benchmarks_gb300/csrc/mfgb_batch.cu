@@ -235,6 +235,51 @@ __global__ void __launch_bounds__(T256)
       });
 }
 
+// ---- Q1 parts by assembled stencils (mfgb_mg_kernels.cuh): one row per thread ----
+struct Q1Part {
+  int64_t off, soff;  // first entry in the depth vector; first coefficient, [27][n]
+  int n, fx, fxy;
+};
+
+__global__ void __launch_bounds__(CHUNK_H)
+    kb_q1_residual(const Chunk *__restrict__ ch, const Q1Part *__restrict__ parts,
+                   const float *__restrict__ S, const uint32_t *__restrict__ bits,
+                   const float *__restrict__ x, Q1Row q) {
+  const Chunk c = ch[blockIdx.x];
+  if ((int)threadIdx.x >= c.len) return;
+  const Q1Part p = parts[c.part];
+  const int64_t t = c.start + threadIdx.x;
+  q1_residual(S + p.soff, p.n, p.fx, p.fxy, bit_at(bits, t), t - p.off, x + p.off,
+              Q1Row{q.b + p.off, q.dinv + p.off, q.r + p.off});
+}
+__global__ void __launch_bounds__(CHUNK_H)
+    kb_q1_first(const Chunk *__restrict__ ch, const Q1Part *__restrict__ parts,
+                const float *__restrict__ S, const uint32_t *__restrict__ bits,
+                const float *__restrict__ x, Q1Row q, float *__restrict__ d, float *__restrict__ y,
+                const float *__restrict__ coef, int cs) {
+  const Chunk c = ch[blockIdx.x];
+  if ((int)threadIdx.x >= c.len) return;
+  const Q1Part p = parts[c.part];
+  const int64_t t = c.start + threadIdx.x;
+  q1_first(S + p.soff, p.n, p.fx, p.fxy, bit_at(bits, t), t - p.off, x + p.off,
+           Q1Row{q.b + p.off, q.dinv + p.off, q.r + p.off}, d + p.off, y + p.off,
+           coef[(int64_t)c.part * cs]);
+}
+__global__ void __launch_bounds__(CHUNK_H)
+    kb_q1_step(const Chunk *__restrict__ ch, const Q1Part *__restrict__ parts,
+               const float *__restrict__ S, const uint32_t *__restrict__ bits,
+               const float *__restrict__ d, Q1Row q, float *__restrict__ dn, const float *x, float *y,
+               const float *__restrict__ coef, int cs, int j) {
+  const Chunk c = ch[blockIdx.x];
+  if ((int)threadIdx.x >= c.len) return;
+  const Q1Part p = parts[c.part];
+  const int64_t t = c.start + threadIdx.x;
+  const float *cf = coef + (int64_t)c.part * cs;
+  q1_step(S + p.soff, p.n, p.fx, p.fxy, bit_at(bits, t), t - p.off, d + p.off,
+          Q1Row{q.b + p.off, q.dinv + p.off, q.r + p.off}, dn + p.off, x + p.off, y + p.off,
+          cf[2 * j - 1], cf[2 * j]);
+}
+
 __global__ void __launch_bounds__(T256)
     kb_h_prolongate_add(const Chunk *__restrict__ ch, const HPart *__restrict__ hp,
                         const float *__restrict__ xc, float *__restrict__ xf) {
@@ -488,6 +533,7 @@ struct Part {
   int group = -1;        // union operator on this depth, -1 none
   int64_t cell_off = 0;  // first cell in the union operator
   int64_t cons_off = 0;  // first entry in the depth's constrained list
+  int64_t soff = -1;     // first coefficient of the part's stencil, -1 none
   double lmax = 0;
 };
 
@@ -503,8 +549,11 @@ struct DepthPlan {
   std::vector<mfgb_operator *> groups;
   const int64_t *d_cons = nullptr;
   int64_t n_cons = 0;
-  const Chunk *d_cheb = nullptr, *d_pch = nullptr, *d_hfine = nullptr, *d_hcoarse = nullptr;
-  int n_cheb = 0, n_pch = 0, n_hfine = 0, n_hcoarse = 0;
+  // smoothed parts: by operators (d_cheb) and, for Q1, by stencils (d_q1)
+  const Chunk *d_cheb = nullptr, *d_q1 = nullptr, *d_pch = nullptr, *d_hfine = nullptr,
+              *d_hcoarse = nullptr;
+  int n_cheb = 0, n_q1 = 0, n_pch = 0, n_hfine = 0, n_hcoarse = 0;
+  bool smooths() const { return n_cheb + n_q1 > 0; }
   std::vector<PGroup> pgroups;
   const HPart *d_hp = nullptr;
 };
@@ -534,8 +583,12 @@ struct Depth {
   int64_t n_cons = 0;
   float *x = nullptr, *b = nullptr, *r = nullptr, *d = nullptr, *t = nullptr, *inv_diag = nullptr,
         *inv_val = nullptr;
-  Chunk *d_cheb = nullptr;   // non-coarsest parts
+  Chunk *d_cheb = nullptr;   // non-coarsest parts (lambda_max estimates)
   int n_cheb = 0;
+  Chunk *d_ops = nullptr, *d_q1 = nullptr;  // the same by how they are smoothed
+  int n_ops = 0, n_q1 = 0;
+  float *S = nullptr, *d2 = nullptr;        // Q1 stencils of all parts, the second d
+  Q1Part *d_q1part = nullptr;               // per part
   Chunk *d_pch = nullptr;    // parts with a p-transfer to depth+1
   int n_pch = 0;
   float *d_coef = nullptr;   // [parts][cs]
@@ -653,6 +706,7 @@ void free_batch(mfgb_batch *B) {
     for (auto &pg : D.pgroups) cudaFree(pg.map_c);
     cudaFree(D.d_cons); cudaFree(D.x); cudaFree(D.b); cudaFree(D.r); cudaFree(D.d); cudaFree(D.t);
     cudaFree(D.inv_diag); cudaFree(D.inv_val); cudaFree(D.d_cheb); cudaFree(D.d_pch);
+    cudaFree(D.d_ops); cudaFree(D.d_q1); cudaFree(D.S); cudaFree(D.d2); cudaFree(D.d_q1part);
     cudaFree(D.d_coef); cudaFree(D.bits); cudaFree(D.d_hp); cudaFree(D.d_hfine); cudaFree(D.d_hcoarse);
   }
   cudaFree(B->d_coarse); cudaFree(B->d_Ainv); cudaFree(B->d_cids);
@@ -706,10 +760,13 @@ mfgb_status apply32(const Depth &V, const DepthPlan &D, const float *src, float 
 // captured; elsewhere (br == nullptr) the degrees run one after another on the caller's stream.
 struct Branches {
   static constexpr int MAX = 7;
-  cudaStream_t aux[MAX] = {};
-  cudaEvent_t fork = nullptr, done[MAX] = {};
+  cudaStream_t aux[MAX] = {}, q1 = nullptr;  // q1: the Q1 parts beside the other ones
+  cudaEvent_t fork = nullptr, done[MAX] = {}, q1_fork = nullptr, q1_done = nullptr;
   mfgb_status init() {
     cudaError_t e = cudaEventCreateWithFlags(&fork, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&q1_fork, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&q1_done, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&q1, cudaStreamNonBlocking);
     for (int k = 0; k < MAX && e == cudaSuccess; ++k) {
       e = cudaStreamCreateWithFlags(&aux[k], cudaStreamNonBlocking);
       if (e == cudaSuccess) e = cudaEventCreateWithFlags(&done[k], cudaEventDisableTiming);
@@ -722,6 +779,9 @@ struct Branches {
       if (aux[k]) cudaStreamDestroy(aux[k]);
     }
     if (fork) cudaEventDestroy(fork);
+    if (q1_fork) cudaEventDestroy(q1_fork);
+    if (q1_done) cudaEventDestroy(q1_done);
+    if (q1) cudaStreamDestroy(q1);
   }
 };
 
@@ -747,8 +807,11 @@ mfgb_status side_by_side(Branches *br, size_t n, cudaStream_t s, F f) {
 // t += A src on the unconstrained rows of one depth (FP32); t enters zero
 mfgb_status level_apply(const Depth &V, const DepthPlan &D, const float *src, cudaStream_t s,
                         Branches *br) {
-  return side_by_side(br, D.groups.size(), s, [&](size_t k, cudaStream_t q) {
-    const mfgb_operator *op = D.groups[k];
+  std::vector<const mfgb_operator *> ops;  // (Q1 parts with stencils are not applied)
+  for (const mfgb_operator *op : D.groups)
+    if (op->degree > 1 || !V.S) ops.push_back(op);
+  return side_by_side(br, ops.size(), s, [&](size_t k, cudaStream_t q) {
+    const mfgb_operator *op = ops[k];
     return cuda_status(bk5_f32(op->n, op->n_cells, op->d_map, op->d_G32, src, V.t, op->D, nullptr,
                                nullptr, q),
                        "batch A32 kernel");
@@ -787,21 +850,76 @@ mfgb_status chebyshev_b(const mfgb_batch *B, const Depth &V, const DepthPlan &D,
   return cuda_status(cudaGetLastError(), "batch chebyshev");
 }
 
+// the same for the Q1 parts with stencils (degree >= 2): x ends in V.x, kept in V.t before the last
+// step of a smoother that starts from x
+mfgb_status chebyshev_q1(const mfgb_batch *B, const Depth &V, const DepthPlan &D, bool zero_start,
+                         cudaStream_t s) {
+  const Q1Row q{V.b, V.inv_diag, V.r};
+  float *d = V.d, *dn = V.d2, *from = V.x;
+  if (zero_start) {
+    kb_cheb_first_zero<<<D.n_q1, T256, 0, s>>>(D.d_q1, V.b, V.inv_diag, V.x, V.d, V.r, V.t, V.d_coef,
+                                               B->cs);
+  } else {
+    from = V.t;
+    kb_q1_first<<<D.n_q1, CHUNK_H, 0, s>>>(D.d_q1, V.d_q1part, V.S, V.bits, V.x, q, d, from, V.d_coef,
+                                           B->cs);
+  }
+  for (int j = 1; j < B->cheb_degree; ++j) {
+    float *to = j + 1 == B->cheb_degree ? V.x : from;
+    kb_q1_step<<<D.n_q1, CHUNK_H, 0, s>>>(D.d_q1, V.d_q1part, V.S, V.bits, d, q, dn, from, to,
+                                          V.d_coef, B->cs, j);
+    std::swap(d, dn);
+  }
+  return cuda_status(cudaGetLastError(), "batch chebyshev");
+}
+
+// ops(s) for the parts smoothed by operators and q1(stream) for those with stencils, side by side
+// where br is given
+template <class F, class G>
+mfgb_status smooth_parts(const DepthPlan &D, cudaStream_t s, Branches *br, F ops, G q1) {
+  mfgb_status st = MFGB_OK;
+  const bool side = br && D.n_cheb && D.n_q1;
+  if (side) {
+    cudaEventRecord(br->q1_fork, s);
+    cudaStreamWaitEvent(br->q1, br->q1_fork, 0);
+  }
+  if (D.n_q1) st = q1(side ? br->q1 : s);
+  if (!st && D.n_cheb) st = ops();
+  if (side) {
+    cudaEventRecord(br->q1_done, br->q1);
+    cudaStreamWaitEvent(s, br->q1_done, 0);
+  }
+  return st;
+}
+
 // depth-0 x = V(b): descend every depth the plan's problems reach, all coarse
 // solves, ascend
 mfgb_status vcycle_b(const mfgb_batch *B, const Plan &P, cudaStream_t s, Branches *br = nullptr) {
   size_t nd = 1;
   for (size_t l = 0; l < P.depth.size(); ++l)
-    if (P.depth[l].n_cheb) nd = l + 2;  // depth l smooths, so depth l + 1 exists
+    if (P.depth[l].smooths()) nd = l + 2;  // depth l smooths, so depth l + 1 exists
   nd = std::min(nd, P.depth.size());
   mfgb_status st;
   for (size_t l = 0; l + 1 < nd; ++l) {
     const Depth &V = B->depth[l], &C = B->depth[l + 1];
     const DepthPlan &D = P.depth[l];
-    if (!D.n_cheb) continue;
-    if ((st = chebyshev_b(B, V, D, true, s, br))) return st;
-    if ((st = level_apply(V, D, V.x, s, br))) return st;
-    kb_residual<<<D.n_cheb, T256, 0, s>>>(D.d_cheb, V.b, V.t, V.x, V.bits, V.r);
+    if (!D.smooths()) continue;
+    st = smooth_parts(
+        D, s, br,
+        [&] {
+          mfgb_status e;
+          if ((e = chebyshev_b(B, V, D, true, s, br)) || (e = level_apply(V, D, V.x, s, br))) return e;
+          kb_residual<<<D.n_cheb, T256, 0, s>>>(D.d_cheb, V.b, V.t, V.x, V.bits, V.r);
+          return cuda_status(cudaGetLastError(), "batch residual");
+        },
+        [&](cudaStream_t q) {
+          mfgb_status e = chebyshev_q1(B, V, D, true, q);
+          if (e) return e;
+          kb_q1_residual<<<D.n_q1, CHUNK_H, 0, q>>>(D.d_q1, V.d_q1part, V.S, V.bits, V.x,
+                                                    Q1Row{V.b, V.inv_diag, V.r});
+          return cuda_status(cudaGetLastError(), "batch residual");
+        });
+    if (st) return st;
     if ((st = cuda_status(cudaMemsetAsync(C.b, 0, sizeof(float) * C.n, s), "batch coarse b = 0")))
       return st;
     // the p-transfers of each degree and the h-transfers
@@ -824,7 +942,7 @@ mfgb_status vcycle_b(const mfgb_batch *B, const Plan &P, cudaStream_t s, Branche
   for (size_t l = nd - 1; l-- > 0;) {
     const Depth &V = B->depth[l], &C = B->depth[l + 1];
     const DepthPlan &D = P.depth[l];
-    if (!D.n_cheb) continue;
+    if (!D.smooths()) continue;
     // V.t is zero (its last consumer cleared it)
     const size_t np = D.pgroups.size();
     if ((st = side_by_side(br, np + (D.n_hfine > 0), s, [&](size_t k, cudaStream_t q) {
@@ -839,7 +957,10 @@ mfgb_status vcycle_b(const mfgb_batch *B, const Plan &P, cudaStream_t s, Branche
          })))
       return st;
     if (np) kb_add_clear<<<D.n_pch, T256, 0, s>>>(D.d_pch, V.t, V.x);
-    if ((st = chebyshev_b(B, V, D, false, s, br))) return st;
+    if ((st = smooth_parts(
+             D, s, br, [&] { return chebyshev_b(B, V, D, false, s, br); },
+             [&](cudaStream_t q) { return chebyshev_q1(B, V, D, false, q); })))
+      return st;
   }
   return MFGB_OK;
 }
@@ -883,7 +1004,8 @@ mfgb_status gather_plan(const mfgb_batch *B, const std::vector<char> &active, Pl
     int64_t n_cons = 0;
     for (size_t k = 0; k < V.parts.size(); ++k) {
       const Part &Q = V.parts[k];
-      if (!active[Q.problem] || Q.group < 0) continue;
+      // (Q1 parts below depth 0 are smoothed by their stencils)
+      if (!active[Q.problem] || Q.group < 0 || (l > 0 && Q.soff >= 0)) continue;
       auto it = gidx.find(Q.degree);
       if (it == gidx.end()) {
         it = gidx.emplace(Q.degree, (int)D.groups.size()).first;
@@ -952,12 +1074,13 @@ mfgb_status gather_plan(const mfgb_batch *B, const std::vector<char> &active, Pl
       }
     }
     // chunk and h-transfer tables
-    std::vector<Chunk> cheb, pch, hfine, hcoarse;
+    std::vector<Chunk> cheb, q1, pch, hfine, hcoarse;
     std::vector<HPart> hp;
     for (size_t k = 0; k < V.parts.size(); ++k) {
       const Part &Q = V.parts[k];
       if (!active[Q.problem] || Q.kind == 0) continue;
-      append_chunks(cheb, Q.off, Q.n, (int)k, CHUNK_SMOOTH);
+      if (Q.soff >= 0) append_chunks(q1, Q.off, Q.n, (int)k, CHUNK_H);
+      else append_chunks(cheb, Q.off, Q.n, (int)k, CHUNK_SMOOTH);
       if (Q.kind == 1) append_chunks(pch, Q.off, Q.n, (int)k, CHUNK_SMOOTH);
       if (Q.kind == 2) {
         const Part &R = B->depth[l + 1].parts[part_at[Q.problem][l + 1]];
@@ -966,12 +1089,13 @@ mfgb_status gather_plan(const mfgb_batch *B, const std::vector<char> &active, Pl
         hp.push_back(HPart{hgrid(Q.box, Q.bs, R.box), Q.off, R.off});
       }
     }
-    Chunk *c1 = nullptr, *c2 = nullptr, *c3 = nullptr, *c4 = nullptr;
+    Chunk *c1 = nullptr, *c2 = nullptr, *c3 = nullptr, *c4 = nullptr, *c5 = nullptr;
     HPart *h1 = nullptr;
-    if ((st = upload(&c1, cheb)) || (st = upload(&c2, pch)) || (st = upload(&c3, hfine)) ||
-        (st = upload(&c4, hcoarse)) || (st = upload(&h1, hp)))
-      return fail(st);
-    track(c1); track(c2); track(c3); track(c4); track(h1);
+    (st = upload(&c1, cheb)) || (st = upload(&c2, pch)) || (st = upload(&c3, hfine)) ||
+        (st = upload(&c4, hcoarse)) || (st = upload(&h1, hp)) || (st = upload(&c5, q1));
+    track(c1); track(c2); track(c3); track(c4); track(h1); track(c5);
+    if (st) return fail(st);
+    D.d_q1 = c5; D.n_q1 = (int)q1.size();
     D.d_cheb = c1; D.n_cheb = (int)cheb.size();
     D.d_pch = c2; D.n_pch = (int)pch.size();
     D.d_hfine = c3; D.n_hfine = (int)hfine.size();
@@ -1105,12 +1229,23 @@ mfgb_status build_batch(mfgb_batch *B, const mfgb_box_desc *boxes, int n,
     if ((st = cuda_status(cudaMemset(D.inv_val, 0, sizeof(float) * D.n), "batch inv_val")))
       return st;
     // chunk tables
-    std::vector<Chunk> cheb, pch, hfine, hcoarse;
+    std::vector<Chunk> cheb, ops, q1, pch, hfine, hcoarse;
+    std::vector<Q1Part> q1part(D.parts.size(), Q1Part{});
+    int64_t coefs = 0;
     std::vector<HPart> hp;
     for (size_t k = 0; k < D.parts.size(); ++k) {
-      const Part &P = D.parts[k];
+      Part &P = D.parts[k];
       if (P.kind == 0) continue;
       append_chunks(cheb, P.off, P.n, (int)k, CHUNK_SMOOTH);
+      if (P.degree == 1 && B->cheb_degree >= 2) {
+        P.soff = coefs;
+        coefs += 27 * P.n;
+        const int fx = P.box.nx + 1;
+        q1part[k] = Q1Part{P.off, P.soff, (int)P.n, fx, fx * (P.box.ny + 1)};
+        append_chunks(q1, P.off, P.n, (int)k, CHUNK_H);
+      } else {
+        append_chunks(ops, P.off, P.n, (int)k, CHUNK_SMOOTH);
+      }
       if (P.kind == 1) append_chunks(pch, P.off, P.n, (int)k, CHUNK_SMOOTH);
       if (P.kind == 2) {
         const Part &Q = B->depth[l + 1].parts[part_at[P.problem][l + 1]];
@@ -1121,12 +1256,18 @@ mfgb_status build_batch(mfgb_batch *B, const mfgb_box_desc *boxes, int n,
       }
     }
     D.n_cheb = (int)cheb.size();
+    D.n_ops = (int)ops.size();
+    D.n_q1 = (int)q1.size();
     D.n_pch = (int)pch.size();
     D.n_hfine = (int)hfine.size();
     D.n_hcoarse = (int)hcoarse.size();
     if ((st = upload(&D.d_cheb, cheb)) || (st = upload(&D.d_pch, pch)) ||
         (st = upload(&D.d_hfine, hfine)) || (st = upload(&D.d_hcoarse, hcoarse)) ||
-        (st = upload(&D.d_hp, hp)))
+        (st = upload(&D.d_hp, hp)) || (st = upload(&D.d_ops, ops)) || (st = upload(&D.d_q1, q1)))
+      return st;
+    if (coefs && ((st = upload(&D.d_q1part, q1part)) ||
+                  (st = dalloc((void **)&D.S, sizeof(float) * coefs)) ||
+                  (st = dalloc((void **)&D.d2, sizeof(float) * D.n))))
       return st;
     // p-transfer groups: every part of a degree > 1 group goes to degree / 2
     for (size_t g = 0; g < D.groups.size(); ++g) {
@@ -1232,6 +1373,10 @@ mfgb_status build_batch(mfgb_batch *B, const mfgb_box_desc *boxes, int n,
       if ((st = cuda_status(cudaMemcpy(D.inv_diag + P.off, L.inv_diag, sizeof(float) * P.n,
                                        cudaMemcpyDeviceToDevice),
                             "batch inv_diag")))
+        return st;
+      if (P.soff >= 0 && (st = cuda_status(cudaMemcpy(D.S + P.soff, L.S, sizeof(float) * 27 * P.n,
+                                                      cudaMemcpyDeviceToDevice),
+                                           "batch stencils")))
         return st;
       if (P.kind == 1) {
         if ((st = cuda_status(cudaMemcpy(D.inv_val + P.off, L.inv_val, sizeof(float) * P.n,
@@ -1379,7 +1524,8 @@ mfgb_status build_batch(mfgb_batch *B, const mfgb_box_desc *boxes, int n,
     P.groups = D.groups;
     P.d_cons = D.d_cons;
     P.n_cons = D.n_cons;
-    P.d_cheb = D.d_cheb; P.n_cheb = D.n_cheb;
+    P.d_cheb = D.d_ops; P.n_cheb = D.n_ops;
+    P.d_q1 = D.d_q1; P.n_q1 = D.n_q1;
     P.d_pch = D.d_pch; P.n_pch = D.n_pch;
     P.d_hfine = D.d_hfine; P.n_hfine = D.n_hfine;
     P.d_hcoarse = D.d_hcoarse; P.n_hcoarse = D.n_hcoarse;

@@ -362,6 +362,35 @@ mfgb_status chebyshev(const MgLevel &L, int degree, double range, bool zero_star
   return cuda_status(cudaGetLastError(), "chebyshev");
 }
 
+// the same on a Q1 level with an assembled stencil (degree >= 2); x ends in L.x, a smoother that
+// starts from x keeps it in L.t until the last step
+mfgb_status chebyshev_q1(const MgLevel &L, int degree, double range, bool zero_start, cudaStream_t s) {
+  const double lmax = L.lmax, lmin = L.lmax / range;
+  const double theta = 0.5 * (lmax + lmin), delta = 0.5 * (lmax - lmin);
+  const double sigma = theta / delta;
+  double rho = 1.0 / sigma;
+  float *x = (float *)L.x, *d = (float *)L.d, *dn = L.d2, *from = x;
+  const Q1Row q{(const float *)L.b, (const float *)L.inv_diag, (float *)L.r};
+  const int fx = L.box.nx + 1, fxy = fx * (L.box.ny + 1);
+  const unsigned g = grid1d(L.n);
+  if (zero_start) {
+    k_cheb_first_zero<float><<<grid1d(L.n / 4), T256, 0, s>>>(L.n, q.b, q.dinv, x, d, q.r, (float *)L.t,
+                                                              (float)(1.0 / theta));
+  } else {
+    from = (float *)L.t;
+    k_q1_first<<<g, T256, 0, s>>>(L.n, L.S, fx, fxy, L.bits, x, q, d, from, (float)(1.0 / theta));
+  }
+  for (int k = 1; k < degree; ++k) {
+    const double rho_new = 1.0 / (2.0 * sigma - rho);
+    const double c1 = rho_new * rho, c2 = 2.0 * rho_new / delta;
+    float *to = k + 1 == degree ? x : from;
+    k_q1_step<<<g, T256, 0, s>>>(L.n, L.S, fx, fxy, L.bits, d, q, dn, from, to, (float)c1, (float)c2);
+    std::swap(d, dn);
+    rho = rho_new;
+  }
+  return cuda_status(cudaGetLastError(), "chebyshev");
+}
+
 template <class T>
 mfgb_status vcycle(mfgb_mg *mg, size_t l, cudaStream_t s) {
   MgLevel &L = mg->levels[l];
@@ -376,10 +405,19 @@ mfgb_status vcycle(mfgb_mg *mg, size_t l, cudaStream_t s) {
     return cuda_status(cudaGetLastError(), "coarse solve");
   }
   MgLevel &C = mg->levels[l + 1];
-  if ((st = chebyshev<T>(L, mg->degree, mg->range, true, prec, s))) return st;
-  if ((st = level_apply(L, prec, L.x, s))) return st;
   const unsigned g = grid1d(L.n / Pack<T>::W);
-  k_level_residual<T><<<g, T256, 0, s>>>(L.n, (const T *)L.b, (T *)L.t, (const T *)L.x, L.bits, (T *)L.r);
+  if (L.S) {
+    if ((st = chebyshev_q1(L, mg->degree, mg->range, true, s))) return st;
+    const int fx = L.box.nx + 1;
+    k_q1_residual<<<grid1d(L.n), T256, 0, s>>>(
+        L.n, L.S, fx, fx * (L.box.ny + 1), L.bits, (const float *)L.x,
+        Q1Row{(const float *)L.b, (const float *)L.inv_diag, (float *)L.r});
+  } else {
+    if ((st = chebyshev<T>(L, mg->degree, mg->range, true, prec, s))) return st;
+    if ((st = level_apply(L, prec, L.x, s))) return st;
+    k_level_residual<T><<<g, T256, 0, s>>>(L.n, (const T *)L.b, (T *)L.t, (const T *)L.x, L.bits,
+                                           (T *)L.r);
+  }
   if (L.to_coarse == 1) {
     const PTransferParams P = ptransfer(L.op, C.op);
     if ((st = cuda_status(cudaMemsetAsync(C.b, 0, sizeof(T) * C.n, s), "coarse b = 0"))) return st;
@@ -400,6 +438,7 @@ mfgb_status vcycle(mfgb_mg *mg, size_t l, cudaStream_t s) {
                                                         (T *)L.x);
   }
   if ((st = cuda_status(cudaGetLastError(), "prolongate"))) return st;
+  if (L.S) return chebyshev_q1(L, mg->degree, mg->range, false, s);
   return chebyshev<T>(L, mg->degree, mg->range, false, prec, s);
 }
 
@@ -540,7 +579,7 @@ void free_mg(mfgb_mg *mg) {
   if (!mg) return;
   for (auto &L : mg->levels) {
     cudaFree(L.x); cudaFree(L.b); cudaFree(L.r); cudaFree(L.d); cudaFree(L.t);
-    cudaFree(L.inv_diag); cudaFree(L.inv_val);
+    cudaFree(L.inv_diag); cudaFree(L.inv_val); cudaFree(L.S); cudaFree(L.d2);
     if (L.op && !L.borrowed) mfgb_operator_destroy(L.op);
   }
   cudaFree(mg->coarse.A); cudaFree(mg->coarse.dinv); cudaFree(mg->coarse.work);
@@ -627,6 +666,13 @@ static mfgb_status mg_setup_impl(const mfgb_box_desc *fine, const mfgb_mg_params
         (st = dalloc(&M.t, ts * M.n)) || (st = dalloc(&M.inv_diag, ts * M.n)))
       break;
     M.bits = M.op->d_cbits;
+    if (prm->precision == 32 && M.box.degree == 1 && M.to_coarse != 0 && mg->degree >= 2) {
+      if ((st = dalloc((void **)&M.S, sizeof(float) * 27 * M.n)) ||
+          (st = dalloc((void **)&M.d2, sizeof(float) * M.n)))
+        break;
+      k_q1_assemble<<<grid1d(M.n), T256>>>(M.box.nx, M.box.ny, M.box.nz, M.op->d_G, M.op->D[0],
+                                           M.op->D[1], M.S, M.n);
+    }
     if (prm->precision == 32 && (st = ensure_g32(M.op))) break;
     if (prm->precision == 64 && (st = ensure_arith(M.op, MFGB_ARITH_FP64_DF))) break;
     // Jacobi in the V-cycle precision

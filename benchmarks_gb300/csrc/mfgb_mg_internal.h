@@ -16,6 +16,8 @@ struct MgLevel {
   void *inv_diag = nullptr;  // Jacobi (precision T)
   const uint32_t *bits = nullptr;  // one bit per DoF: constrained (the operator's)
   void *inv_val = nullptr;   // 1/valence (precision T), for p-restriction from this level
+  // Q1 levels of an FP32 V-cycle that are smoothed: the assembled stencil and the second d (k_q1_*)
+  float *S = nullptr, *d2 = nullptr;
   double lmax = 0;
   int to_coarse = 0;  // 1 = p-transfer, 2 = h-transfer, 0 = coarsest
   bool borrowed = false;  // op belongs to the caller (mfgb_mg_setup_shared)
