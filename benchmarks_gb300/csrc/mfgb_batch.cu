@@ -1236,13 +1236,16 @@ mfgb_status build_batch(mfgb_batch *B, const mfgb_box_desc *boxes, int n,
     // chunk tables
     std::vector<Chunk> cheb, ops, q1, pch, hfine, hcoarse;
     std::vector<Q1Part> q1part(D.parts.size(), Q1Part{});
-    int64_t coefs = 0;
+    int64_t coefs = 0, q1_rows = 0;
+    for (const Part &P : D.parts)
+      if (P.kind && P.degree == 1) q1_rows += P.n;
+    const bool stencils = B->cheb_degree >= 2 && q1_fits(q1_rows);
     std::vector<HPart> hp;
     for (size_t k = 0; k < D.parts.size(); ++k) {
       Part &P = D.parts[k];
       if (P.kind == 0) continue;
       append_chunks(cheb, P.off, P.n, (int)k, CHUNK_SMOOTH);
-      if (P.degree == 1 && B->cheb_degree >= 2) {
+      if (P.degree == 1 && stencils) {
         P.soff = coefs;
         coefs += 27 * P.n;
         const int fx = P.box.nx + 1;
@@ -1379,10 +1382,11 @@ mfgb_status build_batch(mfgb_batch *B, const mfgb_box_desc *boxes, int n,
                                        cudaMemcpyDeviceToDevice),
                             "batch inv_diag")))
         return st;
-      if (P.soff >= 0 && (st = cuda_status(cudaMemcpy(D.S + P.soff, L.S, sizeof(float) * 27 * P.n,
-                                                      cudaMemcpyDeviceToDevice),
-                                           "batch stencils")))
-        return st;
+      if (P.soff >= 0) {
+        k_q1_assemble<<<grid1d(P.n), T256>>>(P.box.nx, P.box.ny, P.box.nz, L.op->d_G, L.op->D[0],
+                                             L.op->D[1], D.S + P.soff, P.n);
+        if ((st = cuda_status(cudaGetLastError(), "batch stencils"))) return st;
+      }
       if (P.kind == 1) {
         if ((st = cuda_status(cudaMemcpy(D.inv_val + P.off, L.inv_val, sizeof(float) * P.n,
                                          cudaMemcpyDeviceToDevice),

@@ -669,7 +669,8 @@ static mfgb_status mg_setup_impl(const mfgb_box_desc *fine, const mfgb_mg_params
         (st = dalloc(&M.t, ts * M.n)) || (st = dalloc(&M.inv_diag, ts * M.n)))
       break;
     M.bits = M.op->d_cbits;
-    if (prm->precision == 32 && M.box.degree == 1 && M.to_coarse != 0 && mg->degree >= 2) {
+    if (prm->precision == 32 && M.box.degree == 1 && M.to_coarse != 0 && mg->degree >= 2 && lmax &&
+        q1_fits(M.n)) {  // (a batch assembles its own)
       if ((st = dalloc((void **)&M.S, sizeof(float) * 27 * M.n)) ||
           (st = dalloc((void **)&M.d2, sizeof(float) * M.n)))
         break;
