@@ -173,6 +173,15 @@ static cudaError_t apply_range(mfgb_operator *op, int64_t cell0, int64_t n, doub
 // 410, 33M 788 / 797, 67.6M 1588 / 1635).
 bool starts_in_one(const mfgb_operator *op, int64_t n) { return op->masked && n <= 20000000; }
 
+// Whether the operator kernel may begin beside start_vmult.  The Gauss-point kernels with 7 and more
+// points a direction hold one or two CTAs an SM and run slower above about 8e5 values when the first of
+// them are placed around the other kernel's (us after it / beside it: BP3 p = 5 1.2M DoFs 85 / 88, 3M
+// 196 / 205; p = 8 97 / 103, 232 / 257; at 0.4M with a memset 39 / 31 and 39 / 29).  All others gain
+// (collocation p = 4 1.2M DoFs 45 / 39, 8M 206 / 199; Gauss p = 4 57 / 50, 281 / 273).
+static bool starts_beside(const mfgb_operator *op) {
+  return op->quadrature == 0 || op->nq <= 6 || op->n_dofs <= 800000;
+}
+
 mfgb_status vmult_impl(mfgb_operator *op, double *dst, const double *src, int arith,
                        double *partials, int *grid, cudaStream_t s, const int *done) {
   const bool full = partials == nullptr;
@@ -190,7 +199,7 @@ mfgb_status vmult_impl(mfgb_operator *op, double *dst, const double *src, int ar
   if (start) st = cuda_status(start_vmult(op->n_dofs, 1, op->d_cbits, src, dst, s), "vmult: start");
   else if (full) st = cuda_status(cudaMemsetAsync(dst, 0, sizeof(double) * op->n_dofs, s), "vmult: dst = 0");
   if (st || (st = cuda_status(apply_range(op, 0, op->n_cells, dst, src, arith, partials, grid, s, done,
-                                          start),
+                                          start && starts_beside(op)),
                               "vmult: operator kernel")))
     return st;
   if (full && !start)

@@ -103,6 +103,17 @@ int ctas_per_sm(K kernel, int threads, size_t smem) {
   return ps;
 }
 
+// The same for a kernel that starts beside the one before it (launch_after): shared memory at its
+// largest share of the SM, so that a first CTA placed while the other kernel runs does not leave the SM
+// a split into which the second one does not fit (vmult at 0.4M DoFs, us without / with: collocation
+// p = 4 18.0 / 14.7, Gauss p = 4 22.7 / 18.7, BP3 p = 8 35.1 / 29.1).
+template <class K>
+int ctas_per_sm_beside(K kernel, int threads, size_t smem) {
+  const int ps = ctas_per_sm(kernel, threads, smem);
+  cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+  return ps;
+}
+
 // One launch; after = true: it may begin while the kernel before it on the stream (which must let it,
 // start_vmult) still runs, and waits for that one's end inside (cudaGridDependencySynchronize).
 template <class... P, class... Q>

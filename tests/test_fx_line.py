@@ -242,3 +242,24 @@ def test_start_values_of_masked_and_unmasked_operators():
     got = B.vmult(torch.zeros_like(u), u).cpu().numpy()
     assert np.linalg.norm(got - want) <= 1e-12 * np.linalg.norm(want)
     assert np.array_equal(got[fixed], src[fixed])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("quadrature,p,n", [("bp3", 5, 18), ("bp3", 5, 19), ("gauss", 6, 15), ("gauss", 6, 16)])
+def test_start_values_beside_and_after_the_wide_kernels(quadrature, p, n):
+    """Both sides of the 8e5 values above which a Gauss-point kernel of 7 points a direction begins
+    after its start values, twice into a result that held something else.  1e-12 as for every apply."""
+    import torch
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import benchmarks_gb300 as mf
+    from oracle import oracle
+    A = mf.LaplaceOperator(mf.BoxMesh(n, n, n, degree=p, amplitude=0.05), quadrature=quadrature)
+    ref = oracle.GaussProblem(n, n, n, p, nq=7, amplitude=0.05)
+    assert (A.m() > 800000) == (n in (19, 16))
+    src = np.random.default_rng(n).uniform(-1, 1, A.m())
+    want = ref.apply(src)
+    u, y = torch.from_numpy(src).cuda(), torch.full((A.m(),), 7.0, dtype=torch.float64, device="cuda")
+    for _ in range(2):
+        got = A.vmult(y, u).cpu().numpy()
+        assert np.linalg.norm(got - want) <= 1e-12 * np.linalg.norm(want)
