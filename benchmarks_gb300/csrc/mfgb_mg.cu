@@ -170,7 +170,8 @@ __global__ void __launch_bounds__(T256)
 }
 
 // p = z + beta p, beta = r.z / previous r.z (infinite before the first direction: beta = 0);
-// v = 0 with p on the constrained rows, ready for v += A p
+// v = 0 with p on the constrained rows, ready for v += A p (bits: the outer operator's; nullptr: its
+// map leaves constrained DoFs in, v = 0 and their rows are copied after the application)
 template <class T>
 __global__ void __launch_bounds__(T256)
     k_pcg_direction(int64_t n, const T *__restrict__ z, double *__restrict__ p,
@@ -185,7 +186,7 @@ __global__ void __launch_bounds__(T256)
   GRID_STRIDE(q, n / W) {
     const int64_t t = q * W;
     const Pack<T> pz = pack_at(z, t);
-    const uint32_t m = __ldg(bits + (t >> 5)) >> (t & 31);
+    const uint32_t m = bits ? __ldg(bits + (t >> 5)) >> (t & 31) : 0u;
 #pragma unroll
     for (int k = 0; k < W; k += 2) {
       Pack<double> pp = pack_at(p, t + k), pv;
@@ -201,7 +202,7 @@ __global__ void __launch_bounds__(T256)
   GRID_STRIDE(q, n % W) {
     const int64_t t = n / W * W + q;
     p[t] = fma(beta, p[t], (double)z[t]);
-    v[t] = bit_at(bits, t) ? p[t] : 0.0;
+    v[t] = bits && bit_at(bits, t) ? p[t] : 0.0;
   }
 }
 
@@ -884,6 +885,8 @@ extern "C" mfgb_status mfgb_mg_cg_solve(const mfgb_operator *cop, mfgb_mg *mg, c
   double *part_rz = mg->part, *part_pv = part_rz + PCG_BLOCKS, *part_rr = part_pv + PCG_BLOCKS;
   const MgLevel &L = mg->levels[0];
   constexpr unsigned g = PCG_BLOCKS;
+  // the identity rows are those of the operator that is solved; the hierarchy's may be others
+  const uint32_t *bits = op->masked ? op->d_cbits : nullptr;
   // r = b - A x
   if ((st = vmult_impl(op, v, d_x, arith, nullptr, nullptr, s))) return st;
   k_residual<double><<<grid1d(n), T256, 0, s>>>(n, d_b, v, r);
@@ -922,8 +925,11 @@ extern "C" mfgb_status mfgb_mg_cg_solve(const mfgb_operator *cop, mfgb_mg *mg, c
     mfgb_status e = vcycle<T>(mg, 0, s);
     if (e) return e;
     k_pcg_rz<T><<<g, T256, 0, s>>>(n, r, (const T *)L.x, part_rz);
-    k_pcg_direction<T><<<g, T256, 0, s>>>(n, (const T *)L.x, p, v, L.bits, part_rz, scal);
+    k_pcg_direction<T><<<g, T256, 0, s>>>(n, (const T *)L.x, p, v, bits, part_rz, scal);
     if ((e = apply_add_impl(op, v, p, arith, s, nullptr))) return e;
+    if (!bits && (e = cuda_status(copy_constrained(op->n_constrained, op->d_constrained, p, v, s),
+                                  "pcg constrained rows")))
+      return e;
     k_pcg_pv<<<g, T256, 0, s>>>(n, p, v, part_pv, scal);
     k_pcg_update<T><<<g, T256, 0, s>>>(n, d_x, r, p, v, (T *)L.b, part_pv, scal, part_rr);
     k_sum_partials<<<1, T256, 0, s>>>(part_rr, (int)g, scal + 3);
