@@ -3,7 +3,9 @@
 #include <cmath>
 #include <cstring>
 #include <atomic>
+#include <memory>
 #include <mutex>
+#include <new>
 #include <random>
 #include <string>
 #include <vector>
@@ -635,17 +637,25 @@ mfgb_status mfgb_operator_create(int degree, int64_t n_dofs, int64_t n_cells,
       set_error("mfgb_operator_create: dof map entry out of range");
       return MFGB_ERR_INVALID_ARG;
     }
-  std::vector<bool> fixed(n_dofs, false);
-  for (int64_t c = 0; c < n_constrained; ++c) {
+  for (int64_t c = 0; c < n_constrained; ++c)
     if (h_constrained[c] < 0 || h_constrained[c] >= n_dofs) {
       set_error("mfgb_operator_create: constrained index out of range");
       return MFGB_ERR_INVALID_ARG;
     }
-    fixed[h_constrained[c]] = true;
+  // Without host memory for the marks the operator counts as unmasked: its identity rows are then
+  // copied after the cell loop, which is right for every map.
+  bool masked = n_constrained == 0 || n_cells == 0;
+  if (!masked) {
+    const std::unique_ptr<uint32_t[]> fixed(new (std::nothrow) uint32_t[(n_dofs + 31) / 32]());
+    if (fixed) {
+      for (int64_t c = 0; c < n_constrained; ++c)
+        fixed[h_constrained[c] >> 5] |= 1u << (h_constrained[c] & 31);
+      masked = true;
+      for (int64_t t = 0; t < n_cells * n3 && masked; ++t)
+        masked = h_dof_map[t] == MFGB_INVALID_DOF ||
+                 !((fixed[h_dof_map[t] >> 5] >> (h_dof_map[t] & 31)) & 1u);
+    }
   }
-  bool masked = true;
-  for (int64_t t = 0; t < n_cells * n3; ++t)
-    if (h_dof_map[t] != MFGB_INVALID_DOF && fixed[h_dof_map[t]]) masked = false;
   mfgb_operator *op = new mfgb_operator();
   init_basis(op, degree);
   op->n_dofs = n_dofs;
