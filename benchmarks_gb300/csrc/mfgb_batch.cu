@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(T256)
     kb_cheb_first_zero(const Chunk *__restrict__ ch, const float *__restrict__ b,
                        const float *__restrict__ dinv, float *__restrict__ x, float *__restrict__ d,
                        float *__restrict__ r, float *__restrict__ tz, const float *__restrict__ coef,
-                       int cs) {
+                       int cs, const uint32_t *__restrict__ bits, int *large) {
   const Chunk c = ch[blockIdx.x];
   const float it = coef[(int64_t)c.part * cs];
   chunk_packs(
@@ -113,6 +113,11 @@ __global__ void __launch_bounds__(T256)
       [&](int64_t t) {
         const P4 pb = pack_at(b, t), pi = pack_at(dinv, t);
         P4 o;
+        if (large) {
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            if (q1_large(pb.v[k]) && bit_at(bits, t + k)) *large = 1;
+        }
 #pragma unroll
         for (int k = 0; k < 4; ++k) o.v[k] = it * pi.v[k] * pb.v[k];
         if (r) put_pack(r, t, pb);
@@ -122,6 +127,7 @@ __global__ void __launch_bounds__(T256)
       },
       [&](int64_t t) {
         const float v = it * dinv[t] * b[t];
+        if (large && q1_large(b[t]) && bit_at(bits, t)) *large = 1;
         if (r) r[t] = b[t];
         if (d) d[t] = v;
         x[t] = v;
@@ -246,40 +252,46 @@ struct Q1Part {
 __global__ void __launch_bounds__(CHUNK_H)
     kb_q1_residual(const Chunk *__restrict__ ch, const Q1Part *__restrict__ parts,
                    const float *__restrict__ S, const uint32_t *__restrict__ bits,
-                   const float *__restrict__ x, Q1Row q) {
+                   const float *__restrict__ x, Q1Row q, const int *large) {
   const Chunk c = ch[blockIdx.x];
   if ((int)threadIdx.x >= c.len) return;
   const Q1Part p = parts[c.part];
   const int64_t t = c.start + threadIdx.x;
-  q1_residual(S + p.soff, p.n, p.fx, p.fxy, bit_at(bits, t), t - p.off, x + p.off,
-              Q1Row{q.b + p.off, q.dinv + p.off, q.r + p.off});
+  q1_masked(large, [&](auto m) {
+    q1_residual<decltype(m)::value>(S + p.soff, p.n, p.fx, p.fxy, bit_at(bits, t), t - p.off, x + p.off,
+                                    Q1Row{q.b + p.off, q.dinv + p.off, q.r + p.off});
+  });
 }
 __global__ void __launch_bounds__(CHUNK_H)
     kb_q1_first(const Chunk *__restrict__ ch, const Q1Part *__restrict__ parts,
                 const float *__restrict__ S, const uint32_t *__restrict__ bits,
                 const float *__restrict__ x, Q1Row q, float *__restrict__ d, float *__restrict__ y,
-                const float *__restrict__ coef, int cs) {
+                const float *__restrict__ coef, int cs, const int *large) {
   const Chunk c = ch[blockIdx.x];
   if ((int)threadIdx.x >= c.len) return;
   const Q1Part p = parts[c.part];
   const int64_t t = c.start + threadIdx.x;
-  q1_first(S + p.soff, p.n, p.fx, p.fxy, bit_at(bits, t), t - p.off, x + p.off,
-           Q1Row{q.b + p.off, q.dinv + p.off, q.r + p.off}, d + p.off, y + p.off,
-           coef[(int64_t)c.part * cs]);
+  q1_masked(large, [&](auto m) {
+    q1_first<decltype(m)::value>(S + p.soff, p.n, p.fx, p.fxy, bit_at(bits, t), t - p.off, x + p.off,
+                                 Q1Row{q.b + p.off, q.dinv + p.off, q.r + p.off}, d + p.off, y + p.off,
+                                 coef[(int64_t)c.part * cs]);
+  });
 }
 __global__ void __launch_bounds__(CHUNK_H)
     kb_q1_step(const Chunk *__restrict__ ch, const Q1Part *__restrict__ parts,
                const float *__restrict__ S, const uint32_t *__restrict__ bits,
                const float *__restrict__ d, Q1Row q, float *__restrict__ dn, const float *x, float *y,
-               const float *__restrict__ coef, int cs, int j) {
+               const float *__restrict__ coef, int cs, int j, const int *large) {
   const Chunk c = ch[blockIdx.x];
   if ((int)threadIdx.x >= c.len) return;
   const Q1Part p = parts[c.part];
   const int64_t t = c.start + threadIdx.x;
   const float *cf = coef + (int64_t)c.part * cs;
-  q1_step(S + p.soff, p.n, p.fx, p.fxy, bit_at(bits, t), t - p.off, d + p.off,
-          Q1Row{q.b + p.off, q.dinv + p.off, q.r + p.off}, dn + p.off, x + p.off, y + p.off,
-          cf[2 * j - 1], cf[2 * j]);
+  q1_masked(large, [&](auto m) {
+    q1_step<decltype(m)::value>(S + p.soff, p.n, p.fx, p.fxy, bit_at(bits, t), t - p.off, d + p.off,
+                                Q1Row{q.b + p.off, q.dinv + p.off, q.r + p.off}, dn + p.off, x + p.off,
+                                y + p.off, cf[2 * j - 1], cf[2 * j]);
+  });
 }
 
 __global__ void __launch_bounds__(T256)
@@ -591,6 +603,7 @@ struct Depth {
   int n_ops = 0, n_q1 = 0;
   float *S = nullptr, *d2 = nullptr;        // Q1 stencils of all parts, the second d
   Q1Part *d_q1part = nullptr;               // per part
+  int *large = nullptr;                     // depth 0: MgLevel::large
   Chunk *d_pch = nullptr;    // parts with a p-transfer to depth+1
   int n_pch = 0;
   float *d_coef = nullptr;   // [parts][cs]
@@ -708,7 +721,7 @@ void free_batch(mfgb_batch *B) {
     for (auto &pg : D.pgroups) cudaFree(pg.map_c);
     cudaFree(D.d_cons); cudaFree(D.x); cudaFree(D.b); cudaFree(D.r); cudaFree(D.d); cudaFree(D.t);
     cudaFree(D.inv_diag); cudaFree(D.inv_val); cudaFree(D.d_cheb); cudaFree(D.d_pch);
-    cudaFree(D.d_ops); cudaFree(D.d_q1); cudaFree(D.S); cudaFree(D.d2); cudaFree(D.d_q1part);
+    cudaFree(D.d_ops); cudaFree(D.d_q1); cudaFree(D.S); cudaFree(D.d2); cudaFree(D.d_q1part); cudaFree(D.large);
     cudaFree(D.d_coef); cudaFree(D.bits); cudaFree(D.d_hp); cudaFree(D.d_hfine); cudaFree(D.d_hcoarse);
   }
   cudaFree(B->d_coarse); cudaFree(B->d_Ainv); cudaFree(B->d_cids);
@@ -838,7 +851,7 @@ mfgb_status chebyshev_b(const mfgb_batch *B, const Depth &V, const DepthPlan &D,
   mfgb_status st;
   if (zero_start) {
     kb_cheb_first_zero<<<D.n_cheb, T256, 0, s>>>(D.d_cheb, V.b, V.inv_diag, V.x, nullptr, nullptr,
-                                                 V.t, V.d_coef, B->cs);
+                                                 V.t, V.d_coef, B->cs, nullptr, nullptr);
   } else {
     if ((st = level_apply(V, D, V.x, s, br))) return st;
     kb_cheb_first<<<D.n_cheb, T256, 0, s>>>(D.d_cheb, V.b, V.t, V.inv_diag, V.x, V.d, V.r, V.bits,
@@ -862,17 +875,18 @@ mfgb_status chebyshev_q1(const mfgb_batch *B, const Depth &V, const DepthPlan &D
   const Q1Row q{V.b, V.inv_diag, V.r};
   float *d = V.d, *dn = V.d2, *from = V.x;
   if (zero_start) {
+    if (V.large) cudaMemsetAsync(V.large, 0, sizeof(int), s);
     kb_cheb_first_zero<<<D.n_q1, T256, 0, s>>>(D.d_q1, V.b, V.inv_diag, V.x, V.d, V.r, V.t, V.d_coef,
-                                               B->cs);
+                                               B->cs, V.bits, V.large);
   } else {
     from = V.t;
     kb_q1_first<<<D.n_q1, CHUNK_H, 0, s>>>(D.d_q1, V.d_q1part, V.S, V.bits, V.x, q, d, from, V.d_coef,
-                                           B->cs);
+                                           B->cs, V.large);
   }
   for (int j = 1; j < B->cheb_degree; ++j) {
     float *to = j + 1 == B->cheb_degree ? V.x : from;
     kb_q1_step<<<D.n_q1, CHUNK_H, 0, s>>>(D.d_q1, V.d_q1part, V.S, V.bits, d, q, dn, from, to,
-                                          V.d_coef, B->cs, j);
+                                          V.d_coef, B->cs, j, V.large);
     std::swap(d, dn);
   }
   return cuda_status(cudaGetLastError(), "batch chebyshev");
@@ -921,7 +935,7 @@ mfgb_status vcycle_b(const mfgb_batch *B, const Plan &P, cudaStream_t s, Branche
           mfgb_status e = chebyshev_q1(B, V, D, true, q);
           if (e) return e;
           kb_q1_residual<<<D.n_q1, CHUNK_H, 0, q>>>(D.d_q1, V.d_q1part, V.S, V.bits, V.x,
-                                                    Q1Row{V.b, V.inv_diag, V.r});
+                                                    Q1Row{V.b, V.inv_diag, V.r}, V.large);
           return cuda_status(cudaGetLastError(), "batch residual");
         });
     if (st) return st;
@@ -1275,7 +1289,8 @@ mfgb_status build_batch(mfgb_batch *B, const mfgb_box_desc *boxes, int n,
       return st;
     if (coefs && ((st = upload(&D.d_q1part, q1part)) ||
                   (st = dalloc((void **)&D.S, sizeof(float) * coefs)) ||
-                  (st = dalloc((void **)&D.d2, sizeof(float) * D.n))))
+                  (st = dalloc((void **)&D.d2, sizeof(float) * D.n)) ||
+                  (l == 0 && (st = dalloc((void **)&D.large, sizeof(int))))))
       return st;
     // p-transfer groups: every part of a degree > 1 group goes to degree / 2
     for (size_t g = 0; g < D.groups.size(); ++g) {

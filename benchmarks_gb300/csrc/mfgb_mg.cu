@@ -348,7 +348,8 @@ mfgb_status chebyshev(const MgLevel &L, int degree, double range, bool zero_star
   const unsigned g = grid1d(L.n / Pack<T>::W);
   mfgb_status st;
   if (zero_start) {
-    k_cheb_first_zero<T><<<g, T256, 0, s>>>(L.n, b, dinv, x, nullptr, nullptr, t, (T)(1.0 / theta));
+    k_cheb_first_zero<T><<<g, T256, 0, s>>>(L.n, b, dinv, x, nullptr, nullptr, t, (T)(1.0 / theta),
+                                             nullptr, nullptr);
   } else {
     if ((st = level_apply(L, prec, x, s))) return st;
     k_cheb_first<T><<<g, T256, 0, s>>>(L.n, b, t, dinv, x, d, r, L.bits, (T)(1.0 / theta));
@@ -378,17 +379,18 @@ mfgb_status chebyshev_q1(const MgLevel &L, int degree, double range, bool zero_s
   const int fx = L.box.nx + 1, fxy = fx * (L.box.ny + 1);
   const unsigned g = grid1d(L.n);
   if (zero_start) {
-    k_cheb_first_zero<float><<<grid1d(L.n / 4), T256, 0, s>>>(L.n, q.b, q.dinv, x, d, q.r, (float *)L.t,
-                                                              (float)(1.0 / theta));
+    if (L.large) cudaMemsetAsync(L.large, 0, sizeof(int), s);
+    k_cheb_first_zero<float><<<grid1d(L.n / 4), T256, 0, s>>>(
+        L.n, q.b, q.dinv, x, d, q.r, (float *)L.t, (float)(1.0 / theta), L.bits, L.large);
   } else {
     from = (float *)L.t;
-    k_q1_first<<<g, T256, 0, s>>>(L.n, L.S, fx, fxy, L.bits, x, q, d, from, (float)(1.0 / theta));
+    k_q1_first<<<g, T256, 0, s>>>(L.n, L.S, fx, fxy, L.bits, x, q, d, from, (float)(1.0 / theta), L.large);
   }
   for (int k = 1; k < degree; ++k) {
     const double rho_new = 1.0 / (2.0 * sigma - rho);
     const double c1 = rho_new * rho, c2 = 2.0 * rho_new / delta;
     float *to = k + 1 == degree ? x : from;
-    k_q1_step<<<g, T256, 0, s>>>(L.n, L.S, fx, fxy, L.bits, d, q, dn, from, to, (float)c1, (float)c2);
+    k_q1_step<<<g, T256, 0, s>>>(L.n, L.S, fx, fxy, L.bits, d, q, dn, from, to, (float)c1, (float)c2, L.large);
     std::swap(d, dn);
     rho = rho_new;
   }
@@ -415,7 +417,7 @@ mfgb_status vcycle(mfgb_mg *mg, size_t l, cudaStream_t s) {
     const int fx = L.box.nx + 1;
     k_q1_residual<<<grid1d(L.n), T256, 0, s>>>(
         L.n, L.S, fx, fx * (L.box.ny + 1), L.bits, (const float *)L.x,
-        Q1Row{(const float *)L.b, (const float *)L.inv_diag, (float *)L.r});
+        Q1Row{(const float *)L.b, (const float *)L.inv_diag, (float *)L.r}, L.large);
   } else {
     if ((st = chebyshev<T>(L, mg->degree, mg->range, true, prec, s))) return st;
     if ((st = level_apply(L, prec, L.x, s))) return st;
@@ -583,7 +585,7 @@ void free_mg(mfgb_mg *mg) {
   if (!mg) return;
   for (auto &L : mg->levels) {
     cudaFree(L.x); cudaFree(L.b); cudaFree(L.r); cudaFree(L.d); cudaFree(L.t);
-    cudaFree(L.inv_diag); cudaFree(L.inv_val); cudaFree(L.S); cudaFree(L.d2);
+    cudaFree(L.inv_diag); cudaFree(L.inv_val); cudaFree(L.S); cudaFree(L.d2); cudaFree(L.large);
     if (L.op && !L.borrowed) mfgb_operator_destroy(L.op);
   }
   cudaFree(mg->coarse.A); cudaFree(mg->coarse.dinv); cudaFree(mg->coarse.work);
@@ -673,7 +675,8 @@ static mfgb_status mg_setup_impl(const mfgb_box_desc *fine, const mfgb_mg_params
     if (prm->precision == 32 && M.box.degree == 1 && M.to_coarse != 0 && mg->degree >= 2 && lmax &&
         q1_fits(M.n)) {  // (a batch assembles its own)
       if ((st = dalloc((void **)&M.S, sizeof(float) * 27 * M.n)) ||
-          (st = dalloc((void **)&M.d2, sizeof(float) * M.n)))
+          (st = dalloc((void **)&M.d2, sizeof(float) * M.n)) ||
+          (l == 0 && (st = dalloc((void **)&M.large, sizeof(int)))))
         break;
       k_q1_assemble<<<grid1d(M.n), T256>>>(M.box.nx, M.box.ny, M.box.nz, M.op->d_G, M.op->D[0],
                                            M.op->D[1], M.S, M.n);

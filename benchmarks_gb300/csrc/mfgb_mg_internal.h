@@ -18,6 +18,7 @@ struct MgLevel {
   void *inv_val = nullptr;   // 1/valence (precision T), for p-restriction from this level
   // Q1 levels of an FP32 V-cycle that are smoothed: the assembled stencil and the second d (k_q1_*)
   float *S = nullptr, *d2 = nullptr;
+  int *large = nullptr;      // finest level with a stencil: set where b is q1_large on a constrained row
   double lmax = 0;
   int to_coarse = 0;  // 1 = p-transfer, 2 = h-transfer, 0 = coarsest
   bool borrowed = false;  // op belongs to the caller (mfgb_mg_setup_shared)

@@ -4,6 +4,7 @@
 #pragma once
 #include <algorithm>
 #include <cstdint>
+#include <type_traits>
 
 #include "mfgb_common.cuh"
 #include "mfgb_internal.h"
@@ -83,17 +84,27 @@ template <class T> __device__ __forceinline__ void put_pack(T *p, int64_t t, con
 // The smoother's vector passes are bound by their bytes, so they move no value twice: after the first
 // step from x0 = 0, d is x and r is b (none is written), and the last step writes neither (8.5e6 DoFs
 // of degree 4 to 1e-10: 28.8 -> 28.4 ms).
+// A finite value on a constrained row that stays finite in the smoother's recurrence (coefficients of
+// a few units a step); past it, and for infinities and NaN, Q1 levels select those values away (q1_row)
+__device__ __forceinline__ bool q1_large(float v) { return !(fabsf(v) <= 1e30f); }
+
 // Chebyshev first step from x0 = 0: x = d = (1/theta) Dinv b ; r = b ; t = 0 (d, r: null where x and b
-// are read in their place)
+// are read in their place); *large (where given) is set if b is q1_large on a constrained row
 template <class T>
 __global__ void k_cheb_first_zero(int64_t n, const T *__restrict__ b, const T *__restrict__ dinv,
                                   T *__restrict__ x, T *__restrict__ d, T *__restrict__ r,
-                                  T *__restrict__ tz, T inv_theta) {
+                                  T *__restrict__ tz, T inv_theta,
+                                  const uint32_t *__restrict__ bits = nullptr, int *large = nullptr) {
   constexpr int W = Pack<T>::W;
   GRID_STRIDE(q, n / W) {
     const int64_t t = q * W;
     const Pack<T> pb = pack_at(b, t), pd = pack_at(dinv, t);
     Pack<T> o, z;
+    if (large) {
+#pragma unroll
+      for (int k = 0; k < W; ++k)
+        if (q1_large((float)pb.v[k]) && bit_at(bits, t + k)) *large = 1;
+    }
 #pragma unroll
     for (int k = 0; k < W; ++k) o.v[k] = inv_theta * pd.v[k] * pb.v[k], z.v[k] = T(0);
     if (r) put_pack(r, t, pb);
@@ -104,6 +115,7 @@ __global__ void k_cheb_first_zero(int64_t n, const T *__restrict__ b, const T *_
   GRID_STRIDE(q, n % W) {
     const int64_t t = n / W * W + q;
     const T v = inv_theta * dinv[t] * b[t];
+    if (large && q1_large((float)b[t]) && bit_at(bits, t)) *large = 1;
     if (r) r[t] = b[t];
     if (d) d[t] = v;
     x[t] = v;
@@ -246,7 +258,8 @@ __global__ void k_scale_by(int64_t n, const T *__restrict__ s, T *__restrict__ v
 // arrays and a smoother that starts from x leaves x in a third until its last step.
 // Bound by launches and latency: per multigrid iteration at 8.5e6 DoFs and degree 4 (three such levels)
 // 2.86 -> 2.67 ms, 24 mixed problems solved together 46.5 -> 44.6 ms.
-// S[s][row], s = (dk+1)*9 + (dj+1)*3 + (di+1); rows of constrained nodes are not read.
+// S[s][row], s = (dk+1)*9 + (dj+1)*3 + (di+1); rows of constrained nodes are not read.  A constrained
+// neighbour's coefficient is -0 (no other one is).
 
 // Stencils are an option: a hierarchy takes them where they need at most a quarter of the free memory
 // (112 bytes a Q1 DoF) and smooths by operators otherwise, so no size that fitted without them fails.
@@ -294,12 +307,17 @@ __global__ void __launch_bounds__(T256)
     for (int s = 0; s < 27; ++s) {
       const int ni = i + s % 3 - 1, nj = j + s / 3 % 3 - 1, nk = k + s / 9 - 1;
       const bool in = ni > 0 && nj > 0 && nk > 0 && ni < fx - 1 && nj < fy - 1 && nk < fz - 1;
-      S[s * stride + row] = in ? (float)acc[s] : 0.f;  // constrained neighbours are masked
+      S[s * stride + row] = in ? __fadd_rn((float)acc[s], 0.f) : -0.f;  // (-0 + 0 = 0)
     }
   }
 }
 
-// (A v)[t] for an unconstrained row t; S at the part's first row, v at its first value
+// (A v)[t] for an unconstrained row t; S at the part's first row, v at its first value.  -0 times a
+// finite value on a constrained row adds nothing, but an infinity or NaN there must stay there as in the
+// operators' masked gather: MASK selects it away.  Only the finest level can have such values (the
+// restriction writes 0 on those rows), and selecting in every pass cost p = 1 at 8e6 DoFs 41.4 -> 46.4
+// ms a solve, so the first smoothing pass looks at them and the others run one of two loops (37.5 ms).
+template <bool MASK>
 __device__ __forceinline__ float q1_row(const float *__restrict__ S, int64_t stride, int fx, int fxy,
                                         int64_t t, const float *__restrict__ v) {
   const float *c = S + t, *p = v + t;
@@ -310,8 +328,11 @@ __device__ __forceinline__ float q1_row(const float *__restrict__ S, int64_t str
 #pragma unroll
     for (int j = 0; j < 3; ++j)
 #pragma unroll
-      for (int i = 0; i < 3; ++i)
-        plane[k] += __ldg(c + (k * 9 + j * 3 + i) * stride) * p[(k - 1) * fxy + (j - 1) * fx + i - 1];
+      for (int i = 0; i < 3; ++i) {
+        const float a = __ldg(c + (k * 9 + j * 3 + i) * stride);
+        const float x = p[(k - 1) * fxy + (j - 1) * fx + i - 1];
+        plane[k] += a * (MASK && __float_as_uint(a) == 0x80000000u ? 0.f : x);
+      }
   }
   return plane[0] + plane[1] + plane[2];
 }
@@ -323,47 +344,67 @@ struct Q1Row {
 };
 
 // r = b - A x
+template <bool MASK>
 __device__ __forceinline__ void q1_residual(const float *S, int64_t stride, int fx, int fxy, bool fixed,
                                             int64_t t, const float *x, const Q1Row &q) {
-  q.r[t] = q.b[t] - (fixed ? x[t] : q1_row(S, stride, fx, fxy, t, x));
+  q.r[t] = q.b[t] - (fixed ? x[t] : q1_row<MASK>(S, stride, fx, fxy, t, x));
 }
 // r = b - A x; d = c2 Dinv r; y = x + d
+template <bool MASK>
 __device__ __forceinline__ void q1_first(const float *S, int64_t stride, int fx, int fxy, bool fixed,
                                          int64_t t, const float *x, const Q1Row &q, float *d, float *y,
                                          float c2) {
-  const float xt = x[t], rt = q.b[t] - (fixed ? xt : q1_row(S, stride, fx, fxy, t, x));
+  const float xt = x[t], rt = q.b[t] - (fixed ? xt : q1_row<MASK>(S, stride, fx, fxy, t, x));
   const float dt = c2 * q.dinv[t] * rt;
   q.r[t] = rt;
   d[t] = dt;
   y[t] = xt + dt;
 }
 // r -= A d; dn = c1 d + c2 Dinv r; y = x + dn
+template <bool MASK>
 __device__ __forceinline__ void q1_step(const float *S, int64_t stride, int fx, int fxy, bool fixed,
                                         int64_t t, const float *d, const Q1Row &q, float *dn,
                                         const float *x, float *y, float c1, float c2) {
-  const float dv = d[t], rt = q.r[t] - (fixed ? dv : q1_row(S, stride, fx, fxy, t, d));
+  const float dv = d[t], rt = q.r[t] - (fixed ? dv : q1_row<MASK>(S, stride, fx, fxy, t, d));
   const float dt = c1 * dv + c2 * q.dinv[t] * rt;
   q.r[t] = rt;
   dn[t] = dt;
   y[t] = x[t] + dt;
 }
 
+// f(mask) with mask = true_type where *large is set (nullptr: never)
+template <class F>
+__device__ __forceinline__ void q1_masked(const int *large, F f) {
+  if (large != nullptr && *large)
+    f(std::true_type());
+  else
+    f(std::false_type());
+}
+
 __global__ void __launch_bounds__(T256)
     k_q1_residual(int64_t n, const float *__restrict__ S, int fx, int fxy,
-                  const uint32_t *__restrict__ bits, const float *__restrict__ x, Q1Row q) {
-  GRID_STRIDE(t, n) q1_residual(S, n, fx, fxy, bit_at(bits, t), t, x, q);
+                  const uint32_t *__restrict__ bits, const float *__restrict__ x, Q1Row q,
+                  const int *large) {
+  q1_masked(large, [&](auto m) {
+    GRID_STRIDE(t, n) q1_residual<decltype(m)::value>(S, n, fx, fxy, bit_at(bits, t), t, x, q);
+  });
 }
 __global__ void __launch_bounds__(T256)
     k_q1_first(int64_t n, const float *__restrict__ S, int fx, int fxy,
                const uint32_t *__restrict__ bits, const float *__restrict__ x, Q1Row q,
-               float *__restrict__ d, float *__restrict__ y, float c2) {
-  GRID_STRIDE(t, n) q1_first(S, n, fx, fxy, bit_at(bits, t), t, x, q, d, y, c2);
+               float *__restrict__ d, float *__restrict__ y, float c2, const int *large) {
+  q1_masked(large, [&](auto m) {
+    GRID_STRIDE(t, n) q1_first<decltype(m)::value>(S, n, fx, fxy, bit_at(bits, t), t, x, q, d, y, c2);
+  });
 }
 __global__ void __launch_bounds__(T256)
     k_q1_step(int64_t n, const float *__restrict__ S, int fx, int fxy,
               const uint32_t *__restrict__ bits, const float *__restrict__ d, Q1Row q,
-              float *__restrict__ dn, const float *x, float *y, float c1, float c2) {
-  GRID_STRIDE(t, n) q1_step(S, n, fx, fxy, bit_at(bits, t), t, d, q, dn, x, y, c1, c2);
+              float *__restrict__ dn, const float *x, float *y, float c1, float c2, const int *large) {
+  q1_masked(large, [&](auto m) {
+    GRID_STRIDE(t, n)
+      q1_step<decltype(m)::value>(S, n, fx, fxy, bit_at(bits, t), t, d, q, dn, x, y, c1, c2);
+  });
 }
 
 // ---- p-transfer: fine degree pf, coarse degree pc, same cells ------------
