@@ -212,8 +212,8 @@ mfgb_status vmult_impl(mfgb_operator *op, double *dst, const double *src, int ar
 
 // kernel shape per (arithmetic class, N): 0 column, 1 point-per-thread,
 // 2 column with TMA-prefetched geometric factors (FP32, and FP64 from N = 6: the
-// line kernel), 3 / 4 the column / TMA kernels at the alternative cells per CTA
-// (AltElems, LineAlt).  Defaults are the fastest
+// line kernel where it applies, bk5_shape), 3 / 4 the column / TMA kernels at the
+// alternative cells per CTA (AltElems, LineAlt).  Defaults are the fastest
 // shape per degree measured on a GB300 at ~3e7 DoFs (autotune.py re-measures).
 static int g_shape[3][10] = {
     {0, 0, 4, 3, 2, 4, 2, 2, 2, 2},  // FP64
@@ -510,6 +510,15 @@ mfgb_status mfgb_get_kernel_shape(int arith, int degree, int *shape) {
     return MFGB_ERR_INVALID_ARG;
   }
   *shape = g_shape[arith][degree + 1];
+  return MFGB_OK;
+}
+
+mfgb_status mfgb_test_fp64_shape(int degree, int evector, int aligned, int mirror, int *shape) {
+  if (degree < 1 || degree > 8 || !shape) {
+    set_error("mfgb_test_fp64_shape: invalid argument");
+    return MFGB_ERR_INVALID_ARG;
+  }
+  *shape = bk5_shape_f64(degree + 1, evector != 0, aligned != 0, mirror != 0);
   return MFGB_OK;
 }
 

@@ -11,4 +11,16 @@ cudaError_t bk5_f64(int N, int64_t n_cells, const uint32_t *map, const double *G
   return bk5_dispatch<ArithF64, false, false>(N, n_cells, map, G, src, dst, D, nullptr, grid, s,
                                               done);
 }
+
+int bk5_shape_f64(int N, bool evec, bool aligned, bool mirror) {
+  switch (N) {
+#define MFGB_CASE(NN)                                                  \
+  case NN: return evec ? bk5_shape<NN, ArithF64, true>(aligned, mirror) \
+                       : bk5_shape<NN, ArithF64, false>(aligned, mirror);
+    MFGB_CASE(2) MFGB_CASE(3) MFGB_CASE(4) MFGB_CASE(5) MFGB_CASE(6) MFGB_CASE(7) MFGB_CASE(8)
+    MFGB_CASE(9)
+#undef MFGB_CASE
+    default: return -1;
+  }
+}
 }  // namespace mfgb

@@ -62,6 +62,8 @@ double lagrange_value(int n, const double *nodes, int j, double x);
 void derivative_matrix(int n, const double *nodes, double *D);
 
 // BK5 kernels (map == nullptr selects E-vector mode where supported)
+// the shape bk5_f64 takes (-1: no such N)
+int bk5_shape_f64(int N, bool evec, bool aligned, bool mirror);
 cudaError_t bk5_f64(int N, int64_t n_cells, const uint32_t *map, const double *G, const double *src,
                     double *dst, const double *D, double *partials, int *grid, cudaStream_t s,
                     const int *done = nullptr);

@@ -70,7 +70,8 @@ template <> struct ElemsPerCtaPt<9> { static constexpr int value = 1; };
 // 5 and 6 (double-float only, GLL operators): the offset-accumulation kernel of
 // mfgb_bk5fx.cuh at its two cells per CTA (FxDefault, FxAlt); elsewhere they run as 2 / 4.
 enum { SHAPE_COLUMN = 0, SHAPE_POINT = 1, SHAPE_TMA = 2, SHAPE_COLUMN_ALT = 3, SHAPE_TMA_ALT = 4,
-       SHAPE_FX = 5, SHAPE_FX_ALT = 6 };
+       SHAPE_FX = 5, SHAPE_FX_ALT = 6,
+       SHAPE_LINE = 7, SHAPE_LINE_ALT = 8 };  // what shapes 2 and 4 become (bk5_shape)
 int kernel_shape(int arith_class, int N);  // mfgb_api.cu
 int *device_error_flag();                  // mfgb_api.cu
 
@@ -166,6 +167,44 @@ template <> struct LineAlt<8, ArithF32> : LineShapeIs<1, 12, 3> {};
 template <> struct LineAlt<9, ArithF32> : LineShapeIs<1, 8, 3> {};
 template <> struct LineAlt<6, ArithF64> : LineShapeIs<3, 5, 2> {};
 
+// The shape of degrees with a line kernel where that one does not apply: element vectors, arrays that
+// are not 16-byte aligned, a caller's matrix without the mirror symmetry.  FP64, ms at 6e6 values as
+// this shape / the column kernel: element vectors N = 7 0.585 / 0.659, 9 0.699 / 0.916 (N = 6 and 8 run
+// the column kernel: no bulk copies there); L-vectors with a general matrix N = 6..9 0.973 / 0.999,
+// 0.988 / 1.149, 1.029 / 1.052, 1.047 / 1.319.
+template <int N, class A> struct LineFallback { static constexpr int value = SHAPE_COLUMN; };
+template <> struct LineFallback<6, ArithF64> { static constexpr int value = SHAPE_TMA; };
+template <> struct LineFallback<7, ArithF64> { static constexpr int value = SHAPE_POINT; };
+template <> struct LineFallback<8, ArithF64> { static constexpr int value = SHAPE_TMA; };
+template <> struct LineFallback<9, ArithF64> { static constexpr int value = SHAPE_POINT; };
+// whether the column kernel with bulk copies can be chosen
+template <int N, class A, bool EVEC>
+constexpr bool has_tma() {
+  return !EVEC && (LineShape<N, A>::E == 0 || LineFallback<N, A>::value == SHAPE_TMA);
+}
+
+// The kernel a launch takes, from the shape table's entry: aligned: G and the map on 16 bytes, mirror:
+// the matrix has the mirror symmetry of symmetric points (Basis::eo).  Shapes 5 / 6 are the
+// double-float operators' own and run as 2 / 4 here; without an alternative cells-per-CTA
+// instantiation (E-vectors, other arithmetic, large N) 3 / 4 run as 0 / 2; bulk copies need aligned
+// tiles of L-vectors.
+template <int N, class A, bool EVEC>
+int bk5_shape(bool aligned, bool mirror) {
+  int shape = kernel_shape(ArithClass<A>::value, N);
+  if (shape == SHAPE_FX) shape = SHAPE_TMA;
+  if (shape == SHAPE_FX_ALT) shape = SHAPE_TMA_ALT;
+  if (LineShape<N, A>::E > 0 && (shape == SHAPE_TMA || shape == SHAPE_TMA_ALT)) {
+    if (!EVEC && aligned && mirror) return shape == SHAPE_TMA ? SHAPE_LINE : SHAPE_LINE_ALT;
+    shape = LineFallback<N, A>::value;
+  }
+  if (EVEC || AltElems<N, A>::value == 0) {
+    if (shape == SHAPE_COLUMN_ALT) shape = SHAPE_COLUMN;
+    if (shape == SHAPE_TMA_ALT) shape = SHAPE_TMA;
+  }
+  if ((shape == SHAPE_TMA || shape == SHAPE_TMA_ALT) && (EVEC || !aligned)) shape = SHAPE_COLUMN;
+  return shape;
+}
+
 // one launch of the line kernel
 template <int N, class A, class Sh>
 cudaError_t line_run(int64_t n_cells, const uint32_t *map, const typename A::GType *G,
@@ -199,7 +238,7 @@ int bk5_grid(int64_t n_cells, int shape) {
                          EA * N * N, 0);
     }
   } else if (shape == SHAPE_TMA_ALT) {
-    if constexpr (EA > 0 && !EVEC && LineShape<N, A>::E == 0) {
+    if constexpr (EA > 0 && has_tma<N, A, EVEC>()) {
       E = EA;
       if (ps < 0)
         ps = ctas_per_sm(bk5_tma_kernel<N, EA, A, EN, AltMinBlocks<N, EA, A>::value>, EA * N * N,
@@ -209,7 +248,7 @@ int bk5_grid(int64_t n_cells, int shape) {
     E = ElemsPerCtaPt<N>::value;
     if (ps < 0) ps = ctas_per_sm(bk5_pt_kernel<N, ElemsPerCtaPt<N>::value, A, EVEC, EN>, E * N * N * N, 0);
   } else if (shape == SHAPE_TMA) {
-    if constexpr (!EVEC && LineShape<N, A>::E == 0) {
+    if constexpr (has_tma<N, A, EVEC>()) {
       constexpr int ET = ElemsPerCtaTma<N, A>::value;
       E = ET;
       if (ps < 0)
@@ -235,39 +274,21 @@ cudaError_t bk5_launch(int64_t n_cells, const uint32_t *map, const typename A::G
                        const typename A::VecT *src, typename A::VecT *dst,
                        const Basis<N, A> &basis, double *partials, int *grid_used,
                        cudaStream_t stream, const int *done_flag = nullptr) {
-  int shape = kernel_shape(ArithClass<A>::value, N);
-  if (shape == SHAPE_FX) shape = SHAPE_TMA;
-  if (shape == SHAPE_FX_ALT) shape = SHAPE_TMA_ALT;
-  // the line kernel (even-odd bases: the operators' own, not every caller's matrix)
+  const bool aligned = !((reinterpret_cast<uintptr_t>(G) | reinterpret_cast<uintptr_t>(map)) & 15u);
+  const int shape = bk5_shape<N, A, EVEC>(aligned, basis.eo);
   if constexpr (!EVEC && LineShape<N, A>::E > 0) {
-    if (shape == SHAPE_TMA || shape == SHAPE_TMA_ALT) {
-      if (basis.eo && !((reinterpret_cast<uintptr_t>(G) | reinterpret_cast<uintptr_t>(map)) & 15u)) {
-        using Sh = LineShape<N, A>;
-        using Alt = LineAlt<N, A>;
-        if (shape == SHAPE_TMA_ALT || n_cells <= (int64_t)Sh::E * Sh::MB * num_sms())
-          return line_run<N, A, Alt>(n_cells, map, G, src, dst, basis, grid_used, stream, done_flag);
-        return line_run<N, A, Sh>(n_cells, map, G, src, dst, basis, grid_used, stream, done_flag);
-      }
-      shape = SHAPE_COLUMN;
-    }
+    using Sh = LineShape<N, A>;
+    if (shape == SHAPE_LINE_ALT || (shape == SHAPE_LINE && n_cells <= (int64_t)Sh::E * Sh::MB * num_sms()))
+      return line_run<N, A, LineAlt<N, A>>(n_cells, map, G, src, dst, basis, grid_used, stream, done_flag);
+    if (shape == SHAPE_LINE)
+      return line_run<N, A, Sh>(n_cells, map, G, src, dst, basis, grid_used, stream, done_flag);
   }
-  // without an alternative cells-per-CTA instantiation (E-vector mode, other
-  // arithmetic, large N) shapes 3 / 4 run as 0 / 2; bulk copies need 16-byte
-  // aligned tiles: caller arrays that are not 16-byte aligned use the column
-  // kernel
-  if (EVEC || AltElems<N, A>::value == 0) {
-    if (shape == SHAPE_COLUMN_ALT) shape = SHAPE_COLUMN;
-    if (shape == SHAPE_TMA_ALT) shape = SHAPE_TMA;
-  }
-  if ((shape == SHAPE_TMA || shape == SHAPE_TMA_ALT) &&
-      (EVEC || ((reinterpret_cast<uintptr_t>(G) | reinterpret_cast<uintptr_t>(map)) & 15u)))
-    shape = SHAPE_COLUMN;
   const int grid = bk5_grid<N, A, EVEC, EN>(n_cells, shape);
   if (grid_used) *grid_used = grid;
   if (n_cells <= 0) return cudaSuccess;
   constexpr int EA = AltElems<N, A>::value;
   constexpr int MBA = AltMinBlocks<N, EA, A>::value;
-  constexpr bool TMA = !EVEC && LineShape<N, A>::E == 0;  // the column kernel with bulk copies
+  constexpr bool TMA = has_tma<N, A, EVEC>();
   if (shape == SHAPE_COLUMN_ALT) {
     if constexpr (EA > 0 && !EVEC)
       bk5_kernel_mb<N, EA, A, EVEC, EN, MBA><<<grid, EA * N * N, 0, stream>>>(

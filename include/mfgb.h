@@ -117,9 +117,14 @@ mfgb_status mfgb_check_device_errors(void *stream);
    GLL operator (the offset-accumulation kernel) arm their first geometric-
    factor copy wait without issuing the copy and give up after 1 ms, so the
    bounded wait runs out with nothing in flight: the result is void and
-   mfgb_check_device_errors returns MFGB_ERR_TIMEOUT. */
+   mfgb_check_device_errors returns MFGB_ERR_TIMEOUT.
+   mfgb_test_fp64_shape: the shape an MFGB_ARITH_FP64 GLL application takes
+   under the present table (0..4, or 7 / 8 = the line kernel that shapes 2 / 4
+   become), for element vectors or L-vectors, arrays on 16 bytes or not, and a
+   matrix with or without the mirror symmetry of symmetric points. */
 mfgb_status mfgb_test_fail_allocation(int n);
 mfgb_status mfgb_test_expire_copy_wait(int n);
+mfgb_status mfgb_test_fp64_shape(int degree, int evector, int aligned, int mirror, int *shape);
 
 const char *mfgb_status_string(mfgb_status s);
 const char *mfgb_last_error(void);
