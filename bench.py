@@ -775,13 +775,17 @@ def kernel_name(degree, arith):
 
     import benchmarks_gb300 as mf
     shape = ctypes.c_int()
-    mf.lib().mfgb_get_kernel_shape(arith, degree, ctypes.byref(shape))
+    if arith == 1:
+        mf.lib().mfgb_get_kernel_shape(arith, degree, ctypes.byref(shape))
+    else:  # of an operator's own arrays
+        mf.lib().mfgb_test_fp64_shape(degree, 0, 1, 1, ctypes.byref(shape))
     n = degree + 1
     pol = "ArithDF" if arith == 1 else "ArithF64"
     return {0: f"bk5_kernel<{n},{pol}>", 1: f"bk5_pt_kernel<{n},{pol}>",
             2: f"bk5_tma_kernel<{n},{pol}>", 3: f"bk5_kernel_mb<{n},{pol}>",
             4: f"bk5_tma_kernel<{n},alt,{pol}>", 5: f"bk5fx_kernel<{n}>",
-            6: f"bk5fx_kernel<{n},alt>"}.get(shape.value, "bk5")
+            6: f"bk5fx_kernel<{n},alt>", 7: f"bk5_line_kernel<{n},{pol}>",
+            8: f"bk5_line_kernel<{n},alt,{pol}>"}.get(shape.value, "bk5")
 
 
 def main():
