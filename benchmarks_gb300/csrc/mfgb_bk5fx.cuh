@@ -25,9 +25,12 @@
 //   and at the end hi = T - C is exact (Sterbenz), lo = S.  That is 6 FP32-pipe
 //   instructions per multiply-add (5 for the first), against 12 for the
 //   TwoSum-based form of ArithDF, with an error of about 2^-46 of C.  The bounds
-//   B come from the data at hand: |u| < 1 for the gradient, max |q| times the
-//   row sum of |G| per point for the metric, and each line's maximum for the
-//   transpose.
+//   B come from the data at hand: each line's maximum for the gradient and the
+//   transpose, max |q| times the row sum of |G| per point for the metric.  (The
+//   cell's bound |u| < 1 for the gradient was 0.6 % faster, but with the two sums
+//   of the even-odd form its error exceeded the plain form's on values that are
+//   not spread evenly: up to 1.5 times at p = 2 on a constant plus small changes,
+//   1.1 to 1.35 on values over 60 binades.)
 //
 // * Line ownership (mfgb_fxline.cuh).  In every contraction a thread owns a whole
 //   line, with the derivative matrix in even-odd form.
@@ -117,19 +120,23 @@ __device__ __forceinline__ int fx_offset(int emax) { return emax > 0 ? emax - 10
 // The same for the gathered values of a cell whose largest exponent is that of a
 // normal finite number (0 < emax < 0x7FF), without branches: values more than 126
 // binades below the cell's largest come out as denormal floats instead of zeros,
-// which the rounding to the grid of 2^-22 removes.  Returns the pair on that grid
-// (offset 3, |x| < 1).
+// which the rounding to the grid of 2^-23 removes.  Returns the pair on that grid:
+// 1 + |x| lies in one binade, so it is twice as fine as the grid of signed values,
+// and sums and differences of two (at most 2 = 2^24 steps) are exact.
 __device__ __forceinline__ df fx_from_double_grid(double x, int off) {
   const unsigned long long b = (unsigned long long)__double_as_longlong(x);
   const unsigned hw = (unsigned)(b >> 32), lw = (unsigned)b;
   const unsigned sign = hw & 0x80000000u;
   const int f = max((int)((hw >> 20) & 0x7FFu) - (off + 896), 0);  // float exponent field
   const unsigned hm = __funnelshift_l(lw, hw, 3) & 0x7FFFFFu;
-  const unsigned scale = sign | ((unsigned)(max(f, 53) - 52) << 23);  // 2^-23 ulp units of lo
+  const float scale = __uint_as_float((unsigned)(max(f, 53) - 52) << 23);  // 2^-23 ulp units of lo
+  const float x24 = __uint_as_float(((unsigned)f << 23) | hm);             // 24 bits of |x|
+  const float h = __fsub_rn(__fadd_rn(1.f, x24), 1.f);
+  const float l = __fmaf_rn(__uint2float_rn(lw & 0x1FFFFFFFu), scale, __fsub_rn(x24, h));
   df r;
-  r.hi = __uint_as_float(sign | ((unsigned)f << 23) | hm);
-  r.lo = __fmul_rn(__uint2float_rn(lw & 0x1FFFFFFFu), __uint_as_float(scale));
-  return fx_grid(r, 3.f);
+  r.hi = __uint_as_float(__float_as_uint(h) ^ sign);
+  r.lo = __uint_as_float(__float_as_uint(l) ^ sign);
+  return r;
 }
 
 // The derivative matrix in both directions: G for the gradient, T transposed.
@@ -373,7 +380,7 @@ __global__ void __launch_bounds__(E * N * N, MB)
       }
 #pragma unroll
       for (int i = 0; i < N; ++i) s_u[col + i * S::i] = x[i];
-      fx_line_grid(basis.G, x, 1.f, qr);
+      fx_line_grid(basis.G, x, fx_line_max(x), qr);
       __syncthreads();  // barrier B: s_u ready, s_emax[slot] read (c = 0: the map tile is free)
       if (jk == 0) s_emax[slot][el] = 0;  // next written two components on
       if constexpr (G64)
@@ -387,12 +394,12 @@ __global__ void __launch_bounds__(E * N * N, MB)
         df y[N];
 #pragma unroll
         for (int m = 0; m < N; ++m) x[m] = s_u[sline + m * S::j];
-        fx_line_grid(basis.G, x, 1.f, y);
+        fx_line_grid(basis.G, x, fx_line_max(x), y);
 #pragma unroll
         for (int m = 0; m < N; ++m) s_s[sline + m * S::j] = y[m];
 #pragma unroll
         for (int m = 0; m < N; ++m) x[m] = s_u[tline + m];
-        fx_line_grid(basis.G, x, 1.f, y);
+        fx_line_grid(basis.G, x, fx_line_max(x), y);
         if (NB == 2) __syncthreads();  // every s-line has been read
 #pragma unroll
         for (int m = 0; m < N; ++m) s_t[tline + m] = y[m];

@@ -258,7 +258,7 @@ __global__ void __launch_bounds__(E * NQ * NQ, MB)
     if (has_col) {
       df x[NM], y[NQ];
       fx_column(raw, s_emax[slot][gc], x);
-      fx_line_grid(basis.B, x, 1.f, y);
+      fx_line_grid(basis.B, x, fx_line_max(x), y);
       store_line(y, U + col, 1);
     }
     __syncthreads();  // barrier B: s_emax[slot] read; the map tile is free
@@ -520,7 +520,7 @@ __global__ void __launch_bounds__(E * NQ * NQ, MB)
       if constexpr (SUMS)
         fx_line_sums(B, x, y);
       else
-        fx_line_grid(B, x, 1.f, y);
+        fx_line_grid(B, x, fx_line_max(x), y);
       store_line(y, U + col, 1);
     }
     __syncthreads();  // the exponents have been read
