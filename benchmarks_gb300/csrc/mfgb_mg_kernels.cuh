@@ -660,33 +660,80 @@ struct HGrid {
 // Weight of the right-hand coarse neighbour (I+1)/2 of an odd fine node I (its left-hand one has the
 // rest): the fraction of their distance the node's position gives, 1/2 unless the last coarse cell is
 // narrower.  An even node is coarse node I/2.
-__device__ __forceinline__ double h_right(int I, int nf, int s) {
+__host__ __device__ __forceinline__ double h_right(int I, int nf, int s) {
   const int A = (I - 1) * s, P = min(I * s, nf), B = min((I + 1) * s, nf);
   return B - A == 2 * s ? 0.5 : (double)(P - A) / (double)(B - A);
 }
 
+// a * b of pairs, the sum of h and l rounded once and not contracted
+__host__ __device__ __forceinline__ float h_sum(float h, float l) {
+#ifdef __CUDA_ARCH__
+  return __fadd_rn(h, l);
+#else
+  const volatile float s = h + l;
+  return s;
+#endif
+}
+__host__ __device__ __forceinline__ df h_mul(df a, df b) {
+  const float h = a.hi * b.hi;
+  const float l = fmaf(a.hi, b.lo, fmaf(a.lo, b.hi, fmaf(a.hi, b.hi, -h))), s = h_sum(h, l);
+  return df{s, h_sum(l, -h_sum(s, -h))};
+}
+
 // Both transfers go one axis at a time with the axis weights found once per node, and 32-bit indices
 // (Q1 levels are below 2^31 nodes): with three FP64 weights, a division among them, for each of the
-// 27 neighbours and 64-bit index divisions, a restriction of 8e4 nodes took 70 us.
+// 27 neighbours and 64-bit index divisions, a restriction of 8e4 nodes took 70 us.  In FP32 that loses
+// nothing where at most one weight is not a half or 1 (error against 64 bits 0.97 of the form with
+// products of weights), nor in the restriction (0.71, and 0.76 at other nodes: 27 terms in a row are
+// rounded more often); a prolongation between two or three narrower cells had 1.44 of it, so those few
+// nodes take the products, rounded once, from pairs.
 
 // x_f[t] += (P x_c)[t] for fine node t (interior nodes only)
 template <class T>
-__device__ __forceinline__ void h_prolongate_node(const HGrid &g, int64_t node,
-                                                  const T *__restrict__ xc, T *__restrict__ xf) {
+__host__ __device__ __forceinline__ void h_prolongate_node(const HGrid &g, int64_t node,
+                                                           const T *__restrict__ xc,
+                                                           T *__restrict__ xf) {
   const unsigned t = (unsigned)node, row = t / (unsigned)g.fx;
   const int I = (int)(t - row * g.fx), K = (int)(row / (unsigned)g.fy), J = (int)(row - (unsigned)K * g.fy);
   if (I == 0 || J == 0 || K == 0 || I == g.fx - 1 || J == g.fy - 1 || K == g.fz - 1) return;
   T w[3][2] = {{T(1), T(0)}, {T(1), T(0)}, {T(1), T(0)}};
   const int at[3] = {I, J, K};
+  int uneven = 0;
 #pragma unroll
   for (int a = 0; a < 3; ++a)
     if (at[a] & 1) {
       const double r = h_right(at[a], g.nf[a], g.s);
       w[a][0] = (T)(1.0 - r);
       w[a][1] = (T)r;
+      uneven += w[a][1] != T(0.5);
     }
   const T *x0 = xc + I / 2 + (int64_t)g.cx * (J / 2 + (int64_t)g.cy * (K / 2));
   T acc = 0;
+  if (sizeof(T) == 4 && uneven > 1) {
+    df p[3][2];  // the axis weights as pairs
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      p[a][0] = p[a][1] = df{1.f, 0.f};
+      if (at[a] & 1) {
+        const int A = (at[a] - 1) * g.s, P = min(at[a] * g.s, g.nf[a]), B = min((at[a] + 1) * g.s, g.nf[a]);
+        const float den = (float)(B - A), inv = 1.f / den, l = (float)w[a][0], r = (float)w[a][1];
+        p[a][0] = df{l, fmaf(-l, den, (float)(B - P)) * inv};
+        p[a][1] = df{r, fmaf(-r, den, (float)(P - A)) * inv};
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        if (k > (K & 1) || j > (J & 1)) continue;
+        const T *x = x0 + (int64_t)g.cx * (j + (int64_t)g.cy * k);
+        const df q = h_mul(p[2][k], p[1][j]);
+        acc += (T)h_mul(q, p[0][0]).hi * x[0];
+        if (I & 1) acc += (T)h_mul(q, p[0][1]).hi * x[1];
+      }
+    xf[node] += acc;
+    return;
+  }
   for (int k = 0; k <= (K & 1); ++k) {
     T plane = 0;
     for (int j = 0; j <= (J & 1); ++j) {
