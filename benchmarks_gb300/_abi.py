@@ -97,6 +97,7 @@ def lib():
         "mfgb_cell_error_reduction": ([P, P, I32, ctypes.c_uint64, P, P], I32),
         "mfgb_test_fail_allocation": ([I32], I32),
         "mfgb_test_expire_copy_wait": ([I32], I32),
+        "mfgb_test_stencil_levels": ([P, P, ctypes.POINTER(I32)], I32),
         "mfgb_test_fp64_shape": ([I32, I32, I32, I32, ctypes.POINTER(I32)], I32),
         "mfgb_mg_set_smoother_weights": ([P, P], I32),
         "mfgb_mlp_n_params": ([], I32),

@@ -601,7 +601,7 @@ struct Depth {
   int n_cheb = 0;
   Chunk *d_ops = nullptr, *d_q1 = nullptr;  // the same by how they are smoothed
   int n_ops = 0, n_q1 = 0;
-  float *S = nullptr, *d2 = nullptr;        // Q1 stencils of all parts, the second d
+  float *S = nullptr;                       // Q1 stencils of all parts
   Q1Part *d_q1part = nullptr;               // per part
   int *large = nullptr;                     // depth 0: MgLevel::large
   Chunk *d_pch = nullptr;    // parts with a p-transfer to depth+1
@@ -683,6 +683,7 @@ struct mfgb_batch {
   int n_problems = 0;
   int cheb_degree = 5;
   int cs = 0;  // coefficients per part
+  bool stencils = true;  // smooth Q1 parts by assembled stencils
   std::vector<mfgb_box_desc> boxes;
   std::vector<mfgb::Depth> depth;
   // coarse solves
@@ -698,7 +699,7 @@ struct mfgb_batch {
   int *d_cbeg = nullptr, *d_pid = nullptr;
   int2 *d_range = nullptr;
   mfgb::Plan full;
-  double *r = nullptr, *z = nullptr, *p = nullptr, *v = nullptr, *part = nullptr;
+  double *r = nullptr, *p = nullptr, *v = nullptr, *part = nullptr;
   mfgb::BScal *d_scal = nullptr;
   int *d_active = nullptr;
   int *h_active = nullptr;  // pinned
@@ -721,13 +722,13 @@ void free_batch(mfgb_batch *B) {
     for (auto &pg : D.pgroups) cudaFree(pg.map_c);
     cudaFree(D.d_cons); cudaFree(D.x); cudaFree(D.b); cudaFree(D.r); cudaFree(D.d); cudaFree(D.t);
     cudaFree(D.inv_diag); cudaFree(D.inv_val); cudaFree(D.d_cheb); cudaFree(D.d_pch);
-    cudaFree(D.d_ops); cudaFree(D.d_q1); cudaFree(D.S); cudaFree(D.d2); cudaFree(D.d_q1part); cudaFree(D.large);
+    cudaFree(D.d_ops); cudaFree(D.d_q1); cudaFree(D.S); cudaFree(D.d_q1part); cudaFree(D.large);
     cudaFree(D.d_coef); cudaFree(D.bits); cudaFree(D.d_hp); cudaFree(D.d_hfine); cudaFree(D.d_hcoarse);
   }
   cudaFree(B->d_coarse); cudaFree(B->d_Ainv); cudaFree(B->d_cids);
   cudaFree(B->d_all); cudaFree(B->d_cbeg); cudaFree(B->d_pid);
   cudaFree(B->d_range);
-  cudaFree(B->r); cudaFree(B->z); cudaFree(B->p); cudaFree(B->v); cudaFree(B->part);
+  cudaFree(B->r); cudaFree(B->p); cudaFree(B->v); cudaFree(B->part);
   cudaFree(B->d_scal); cudaFree(B->d_active);
   cudaFree(B->d_pdofs); cudaFree(B->d_active_dofs); cudaFree(B->d_iter);
   if (B->h_active) cudaFreeHost(B->h_active);
@@ -827,6 +828,7 @@ mfgb_status level_apply(const Depth &V, const DepthPlan &D, const float *src, cu
     if (op->degree > 1 || !V.S) ops.push_back(op);
   return side_by_side(br, ops.size(), s, [&](size_t k, cudaStream_t q) {
     const mfgb_operator *op = ops[k];
+    if (op->n_cells > 0 && !op->d_G32) return cuda_status(cudaErrorInvalidValue, "batch A32: no factors");
     return cuda_status(bk5_f32(op->n, op->n_cells, op->d_map, op->d_G32, src, V.t, op->D, nullptr,
                                nullptr, q),
                        "batch A32 kernel");
@@ -869,11 +871,11 @@ mfgb_status chebyshev_b(const mfgb_batch *B, const Depth &V, const DepthPlan &D,
 }
 
 // the same for the Q1 parts with stencils (degree >= 2): x ends in V.x, kept in V.t before the last
-// step of a smoother that starts from x
+// step of a smoother that starts from x; the second d is inv_val, which only p-transfers read
 mfgb_status chebyshev_q1(const mfgb_batch *B, const Depth &V, const DepthPlan &D, bool zero_start,
                          cudaStream_t s) {
   const Q1Row q{V.b, V.inv_diag, V.r};
-  float *d = V.d, *dn = V.d2, *from = V.x;
+  float *d = V.d, *dn = V.inv_val, *from = V.x;
   if (zero_start) {
     if (V.large) cudaMemsetAsync(V.large, 0, sizeof(int), s);
     kb_cheb_first_zero<<<D.n_q1, T256, 0, s>>>(D.d_q1, V.b, V.inv_diag, V.x, V.d, V.r, V.t, V.d_coef,
@@ -1046,8 +1048,9 @@ mfgb_status gather_plan(const mfgb_batch *B, const std::vector<char> &active, Pl
       mfgb_operator *op = D.groups[g];
       op->n_cells = gcells[g];
       const int64_t n3 = (int64_t)op->n * op->n * op->n;
+      const bool g32 = F.groups[V.parts[gparts[g][0]].group]->d_G32 != nullptr;  // (stencils: none)
       if ((st = dalloc((void **)&op->d_map, sizeof(uint32_t) * op->n_cells * n3)) ||
-          (st = dalloc((void **)&op->d_G32, sizeof(float) * op->n_cells * 6 * n3)) ||
+          (g32 && (st = dalloc((void **)&op->d_G32, sizeof(float) * op->n_cells * 6 * n3))) ||
           (l == 0 && (st = dalloc((void **)&op->d_Gfx, sizeof(float2) * op->n_cells * 6 * n3))) ||
           (l == 0 && (st = dalloc((void **)&op->d_Gexp, sizeof(int) * op->n_cells))))
         return fail(st);
@@ -1057,8 +1060,9 @@ mfgb_status gather_plan(const mfgb_batch *B, const std::vector<char> &active, Pl
         const mfgb_operator *src = F.groups[Q.group];
         cudaMemcpyAsync(op->d_map + c0 * n3, src->d_map + Q.cell_off * n3,
                         sizeof(uint32_t) * Q.n_cells * n3, cudaMemcpyDeviceToDevice, s);
-        cudaMemcpyAsync(op->d_G32 + c0 * 6 * n3, src->d_G32 + Q.cell_off * 6 * n3,
-                        sizeof(float) * Q.n_cells * 6 * n3, cudaMemcpyDeviceToDevice, s);
+        if (g32)
+          cudaMemcpyAsync(op->d_G32 + c0 * 6 * n3, src->d_G32 + Q.cell_off * 6 * n3,
+                          sizeof(float) * Q.n_cells * 6 * n3, cudaMemcpyDeviceToDevice, s);
         if (l == 0) {
           cudaMemcpyAsync(op->d_Gfx + c0 * 6 * n3, src->d_Gfx + Q.cell_off * 6 * n3,
                           sizeof(float2) * Q.n_cells * 6 * n3, cudaMemcpyDeviceToDevice, s);
@@ -1250,10 +1254,8 @@ mfgb_status build_batch(mfgb_batch *B, const mfgb_box_desc *boxes, int n,
     // chunk tables
     std::vector<Chunk> cheb, ops, q1, pch, hfine, hcoarse;
     std::vector<Q1Part> q1part(D.parts.size(), Q1Part{});
-    int64_t coefs = 0, q1_rows = 0;
-    for (const Part &P : D.parts)
-      if (P.kind && P.degree == 1) q1_rows += P.n;
-    const bool stencils = B->cheb_degree >= 2 && q1_fits(q1_rows);
+    int64_t coefs = 0;
+    const bool stencils = B->stencils && B->cheb_degree >= 2;
     std::vector<HPart> hp;
     for (size_t k = 0; k < D.parts.size(); ++k) {
       Part &P = D.parts[k];
@@ -1289,7 +1291,6 @@ mfgb_status build_batch(mfgb_batch *B, const mfgb_box_desc *boxes, int n,
       return st;
     if (coefs && ((st = upload(&D.d_q1part, q1part)) ||
                   (st = dalloc((void **)&D.S, sizeof(float) * coefs)) ||
-                  (st = dalloc((void **)&D.d2, sizeof(float) * D.n)) ||
                   (l == 0 && (st = dalloc((void **)&D.large, sizeof(int))))))
       return st;
     // p-transfer groups: every part of a degree > 1 group goes to degree / 2
@@ -1330,7 +1331,6 @@ mfgb_status build_batch(mfgb_batch *B, const mfgb_box_desc *boxes, int n,
         (st = upload(&B->d_range, range)))
       return st;
     if ((st = dalloc((void **)&B->r, sizeof(double) * D.n)) ||
-        (st = dalloc((void **)&B->z, sizeof(double) * D.n)) ||
         (st = dalloc((void **)&B->p, sizeof(double) * D.n)) ||
         (st = dalloc((void **)&B->v, sizeof(double) * D.n)) ||
         (st = dalloc((void **)&B->part, sizeof(double) * 3 * std::max(1, B->n_all))) ||
@@ -1473,7 +1473,7 @@ mfgb_status build_batch(mfgb_batch *B, const mfgb_box_desc *boxes, int n,
       return st;
     }
     struct Free2 { void *a, *b; ~Free2() { cudaFree(a); cudaFree(b); } } f2{d_poff, acc};
-    double *v = B->r, *w = B->z;  // depth-0-sized FP64 work vectors, free until the first solve
+    double *v = B->r, *w = B->p;  // depth-0-sized FP64 work vectors, written by every solve before use
     DepthPlan DP;
     DP.groups = D.groups;
     DP.d_cons = D.d_cons;
@@ -1499,6 +1499,11 @@ mfgb_status build_batch(mfgb_batch *B, const mfgb_box_desc *boxes, int n,
       return st;
     for (int k = 0; k < np; ++k)
       if (D.parts[k].kind != 0) D.parts[k].lmax = 1.2 * lam[k];
+    for (mfgb_operator *op : D.groups)  // Q1 parts with stencils are not applied in FP32 again
+      if (D.S && op->degree == 1) {
+        cudaFree(op->d_G32);
+        op->d_G32 = nullptr;
+      }
   }
   // ---- Chebyshev coefficients per part (the single-problem recurrence) ------
   for (auto &D : B->depth) {
@@ -1609,14 +1614,35 @@ mfgb_status mfgb_batch_create(const mfgb_box_desc *boxes, int n_problems,
   *out = nullptr;
   mfgb_status st = check_params(boxes, n_problems, params);
   if (st) return st;
-  mfgb_batch *B = new mfgb_batch();
-  st = build_batch(B, boxes, n_problems, params);
-  if (st) {
+  // every batch takes stencils (they end in less memory than the operators' factors); where the device
+  // has no room for both during the set-up, it is built again without them
+  for (const bool stencils : {true, false}) {
+    mfgb_batch *B = new mfgb_batch();
+    B->stencils = stencils;
+    st = build_batch(B, boxes, n_problems, params);
+    if (!st) {
+      *out = B;
+      return MFGB_OK;
+    }
     cudaDeviceSynchronize();
+    bool took = false;
+    for (const Depth &D : B->depth) took = took || D.S || D.n_q1;
     free_batch(B);
-    return st;
+    if (st != MFGB_ERR_OUT_OF_MEMORY || !took) break;
   }
-  *out = B;
+  return st;
+}
+
+mfgb_status mfgb_test_stencil_levels(const mfgb_mg *mg, const mfgb_batch *batch, int *levels) {
+  if (!levels || !mg == !batch) {
+    set_error("mfgb_test_stencil_levels: invalid argument");
+    return MFGB_ERR_INVALID_ARG;
+  }
+  *levels = 0;
+  if (mg)
+    for (const MgLevel &L : mg->levels) *levels += L.S != nullptr;
+  else
+    for (const Depth &D : batch->depth) *levels += D.S != nullptr;
   return MFGB_OK;
 }
 

@@ -306,6 +306,13 @@ void mg_plan_levels(const mfgb_box_desc &fine, int coarse_cells, std::vector<mfg
 
 namespace {
 
+// a level with a stencil keeps no FP32 factors: nothing may apply its operator
+mfgb_status has_g32(const mfgb_operator *op) {
+  if (op->d_G32 || op->n_cells == 0) return MFGB_OK;
+  set_error("multigrid level without FP32 geometric factors");
+  return MFGB_ERR_CUDA;
+}
+
 size_t tsize(int prec) { return prec == 32 ? sizeof(float) : sizeof(double); }
 
 // dst = A src on one level in the V-cycle precision
@@ -313,6 +320,7 @@ mfgb_status level_vmult(mfgb_operator *op, int prec, void *dst, const void *src,
   if (prec == 64) return vmult_impl(op, (double *)dst, (const double *)src, MFGB_ARITH_FP64_DF,
                                     nullptr, nullptr, s);
   mfgb_status st;
+  if ((st = has_g32(op))) return st;
   if ((st = cuda_status(cudaMemsetAsync(dst, 0, sizeof(float) * op->n_dofs, s), "A32: dst = 0")))
     return st;
   if ((st = cuda_status(bk5_f32(op->n, op->n_cells, op->d_map, op->d_G32, (const float *)src,
@@ -330,6 +338,7 @@ mfgb_status level_vmult(mfgb_operator *op, int prec, void *dst, const void *src,
 mfgb_status level_apply(const MgLevel &L, int prec, const void *src, cudaStream_t s) {
   if (prec == 64)
     return apply_add_impl(L.op, (double *)L.t, (const double *)src, MFGB_ARITH_FP64_DF, s, nullptr);
+  if (const mfgb_status st = has_g32(L.op)) return st;
   return cuda_status(bk5_f32(L.op->n, L.op->n_cells, L.op->d_map, L.op->d_G32, (const float *)src,
                              (float *)L.t, L.op->D, nullptr, nullptr, s),
                      "A32 kernel");
@@ -581,11 +590,41 @@ mfgb_status estimate_lmax(MgLevel &L, int prec, int iters, double *lmax,
   return cuda_status(cudaGetLastError(), "lmax");
 }
 
+void drop_stencil(MgLevel &L) {
+  cudaFree(L.S); cudaFree(L.d2); cudaFree(L.large);
+  L.S = L.d2 = nullptr;
+  L.large = nullptr;
+}
+
+// The FP32 factors of an operator of the hierarchy's own are not needed beside its stencil.  (A
+// borrowed operator's are its owner's.)
+void free_g32(MgLevel &L) {
+  if (L.borrowed) return;
+  cudaFree(L.op->d_G32);
+  L.op->d_G32 = nullptr;
+}
+
+// The stencil of a Q1 level: 112 bytes a DoF in the place of the operator's FP32 factors, 192 a cell.
+// Every hierarchy takes it, so results and times do not depend on the free memory of the moment; only
+// where the allocation itself fails the level is smoothed by its operator as before.
+mfgb_status take_stencil(MgLevel &L, bool finest) {
+  free_g32(L);
+  if (!dalloc((void **)&L.S, sizeof(float) * 27 * L.n) && !dalloc((void **)&L.d2, sizeof(float) * L.n) &&
+      (!finest || !dalloc((void **)&L.large, sizeof(int)))) {
+    k_q1_assemble<<<grid1d(L.n), T256>>>(L.box.nx, L.box.ny, L.box.nz, L.op->d_G, L.op->D[0], L.op->D[1],
+                                         L.S, L.n);
+    return cuda_status(cudaGetLastError(), "mg stencil");
+  }
+  drop_stencil(L);
+  return ensure_g32(L.op);
+}
+
 void free_mg(mfgb_mg *mg) {
   if (!mg) return;
   for (auto &L : mg->levels) {
     cudaFree(L.x); cudaFree(L.b); cudaFree(L.r); cudaFree(L.d); cudaFree(L.t);
-    cudaFree(L.inv_diag); cudaFree(L.inv_val); cudaFree(L.S); cudaFree(L.d2); cudaFree(L.large);
+    cudaFree(L.inv_diag); cudaFree(L.inv_val);
+    drop_stencil(L);
     if (L.op && !L.borrowed) mfgb_operator_destroy(L.op);
   }
   cudaFree(mg->coarse.A); cudaFree(mg->coarse.dinv); cudaFree(mg->coarse.work);
@@ -672,15 +711,6 @@ static mfgb_status mg_setup_impl(const mfgb_box_desc *fine, const mfgb_mg_params
         (st = dalloc(&M.t, ts * M.n)) || (st = dalloc(&M.inv_diag, ts * M.n)))
       break;
     M.bits = M.op->d_cbits;
-    if (prm->precision == 32 && M.box.degree == 1 && M.to_coarse != 0 && mg->degree >= 2 && lmax &&
-        q1_fits(M.n)) {  // (a batch assembles its own)
-      if ((st = dalloc((void **)&M.S, sizeof(float) * 27 * M.n)) ||
-          (st = dalloc((void **)&M.d2, sizeof(float) * M.n)) ||
-          (l == 0 && (st = dalloc((void **)&M.large, sizeof(int)))))
-        break;
-      k_q1_assemble<<<grid1d(M.n), T256>>>(M.box.nx, M.box.ny, M.box.nz, M.op->d_G, M.op->D[0],
-                                           M.op->D[1], M.S, M.n);
-    }
     if (prm->precision == 32 && (st = ensure_g32(M.op))) break;
     if (prm->precision == 64 && (st = ensure_arith(M.op, MFGB_ARITH_FP64_DF))) break;
     // Jacobi in the V-cycle precision
@@ -768,6 +798,11 @@ static mfgb_status mg_setup_impl(const mfgb_box_desc *fine, const mfgb_mg_params
       }
     }
   }
+  // last of all, so that no other allocation of the set-up misses their memory (a batch assembles its own)
+  if (prm->precision == 32 && mg->degree >= 2 && lmax)
+    for (size_t l = 0; l < mg->levels.size() && !st; ++l)
+      if (mg->levels[l].box.degree == 1 && mg->levels[l].to_coarse != 0)
+        st = take_stencil(mg->levels[l], l == 0);
   if (!st) st = cuda_status(cudaDeviceSynchronize(), "mg set-up");
   if (st) {
     free_mg(mg);
@@ -805,7 +840,9 @@ extern "C" mfgb_status mfgb_mg_set_smoother_weights(mfgb_mg *mg, const double *d
   }
   if (!st) st = cuda_status(invert_diagonal(L.n, d64, nullptr), "invert diag");
   double lam = 0;
+  if (!st && mg->precision == 32) st = ensure_g32(L.op);
   if (!st) st = estimate_lmax(L, mg->precision, 20, &lam, d64);
+  if (L.S) free_g32(L);
   if (!st) {
     L.lmax = 1.2 * lam;
     if (mg->precision == 32)
@@ -861,10 +898,12 @@ extern "C" mfgb_status mfgb_mg_cg_solve(const mfgb_operator *cop, mfgb_mg *mg, c
   mfgb_operator *op = const_cast<mfgb_operator *>(cop);
   const int64_t n = op->n_dofs;
   mfgb_status st;
-  if (mg->outer_n != n) {
+  auto outer_vectors = [&]() -> mfgb_status {
+    if (mg->outer_n == n) return MFGB_OK;
     cudaFree(mg->r); cudaFree(mg->p); cudaFree(mg->v); cudaFree(mg->part); cudaFree(mg->scal);
     mg->r = mg->p = mg->v = mg->part = mg->scal = nullptr;
     mg->outer_n = -1;
+    mfgb_status st;
     if ((st = dalloc((void **)&mg->r, sizeof(double) * n)) ||
         (st = dalloc((void **)&mg->p, sizeof(double) * n)) ||
         (st = dalloc((void **)&mg->v, sizeof(double) * n)) ||
@@ -872,7 +911,20 @@ extern "C" mfgb_status mfgb_mg_cg_solve(const mfgb_operator *cop, mfgb_mg *mg, c
         (st = dalloc((void **)&mg->scal, sizeof(double) * 8)))
       return st;
     mg->outer_n = n;
+    return MFGB_OK;
+  };
+  // the stencil of a borrowed finest Q1 level is memory beside its operator's FP32 factors: where the
+  // solve's own allocations miss it, they come first
+  auto allocate = [&]() -> mfgb_status {
+    const mfgb_status st = outer_vectors();
+    return st ? st : ensure_arith(op, ctl->arith);
+  };
+  st = allocate();
+  if (st == MFGB_ERR_OUT_OF_MEMORY && mg->levels[0].S && mg->levels[0].borrowed) {
+    drop_stencil(mg->levels[0]);
+    st = allocate();
   }
+  if (st) return st;
   cudaStream_t s = nullptr;
   if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess)
     return cuda_status(cudaErrorUnknown, "stream create");
@@ -883,7 +935,6 @@ extern "C" mfgb_status mfgb_mg_cg_solve(const mfgb_operator *cop, mfgb_mg *mg, c
   cudaStreamWaitEvent(s, ev, 0);
   cudaEventDestroy(ev);
   const int arith = ctl->arith;
-  if ((st = ensure_arith(op, arith))) return st;
   double *r = mg->r, *p = mg->p, *v = mg->v, *scal = mg->scal;
   double *part_rz = mg->part, *part_pv = part_rz + PCG_BLOCKS, *part_rr = part_pv + PCG_BLOCKS;
   const MgLevel &L = mg->levels[0];

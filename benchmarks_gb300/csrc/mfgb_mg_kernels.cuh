@@ -261,17 +261,6 @@ __global__ void k_scale_by(int64_t n, const T *__restrict__ s, T *__restrict__ v
 // S[s][row], s = (dk+1)*9 + (dj+1)*3 + (di+1); rows of constrained nodes are not read.  A constrained
 // neighbour's coefficient is -0 (no other one is).
 
-// Stencils are an option: a hierarchy takes them where they need at most a quarter of the free memory
-// (112 bytes a Q1 DoF) and smooths by operators otherwise, so no size that fitted without them fails.
-inline bool q1_fits(int64_t rows) {
-  size_t avail = 0, total = 0;
-  if (cudaMemGetInfo(&avail, &total) != cudaSuccess) {
-    cudaGetLastError();
-    return false;
-  }
-  return sizeof(float) * 28 * (size_t)rows <= avail / 4;
-}
-
 // One row per thread: the rows of the up to 8 cells around node (i, j, k) that belong to it.
 __global__ void __launch_bounds__(T256)
     k_q1_assemble(int nx, int ny, int nz, const double *__restrict__ G, double d0, double d1,

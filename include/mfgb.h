@@ -121,8 +121,12 @@ mfgb_status mfgb_check_device_errors(void *stream);
    mfgb_test_fp64_shape: the shape an MFGB_ARITH_FP64 GLL application takes
    under the present table (0..4, or 7 / 8 = the line kernel that shapes 2 / 4
    become), for element vectors or L-vectors, arrays on 16 bytes or not, and a
-   matrix with or without the mirror symmetry of symmetric points. */
+   matrix with or without the mirror symmetry of symmetric points.
+   mfgb_test_stencil_levels: how many levels of a hierarchy or depths of a
+   batch (the other one NULL) are smoothed by assembled stencils. */
 mfgb_status mfgb_test_fail_allocation(int n);
+mfgb_status mfgb_test_stencil_levels(const struct mfgb_mg *mg, const struct mfgb_batch *batch,
+                                     int *levels);
 mfgb_status mfgb_test_expire_copy_wait(int n);
 mfgb_status mfgb_test_fp64_shape(int degree, int evector, int aligned, int mirror, int *shape);
 
