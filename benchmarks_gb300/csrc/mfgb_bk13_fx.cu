@@ -35,8 +35,8 @@ cudaError_t bk1_run(int64_t nelmt, const double *in, const double *JxW, double *
   constexpr int E = Sh::E, T = E * NQ * NQ;
   constexpr size_t smem = sizeof(df) * E * GaussStride<NQ>::cell;
   const auto kernel = bk1fx_kernel<NM, NQ, E, Sh::MB, SYM>;
-  static int per_sm = -1;
-  if (per_sm < 0) per_sm = std::max(1, ctas_per_sm(kernel, T, smem));
+  static PerDevice found;
+  const int per_sm = found([&] { return std::max(1, ctas_per_sm(kernel, T, smem)); });
   const int64_t batches = (nelmt + E - 1) / E;
   const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(batches, (int64_t)per_sm * num_sms()));
   kernel<<<grid, T, smem, s>>>(nelmt, in, JxW, out, b.B, b.Bt, b.K);

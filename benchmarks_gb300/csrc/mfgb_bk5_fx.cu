@@ -67,8 +67,8 @@ static cudaError_t fx_run(int64_t n_cells, const uint32_t *map, const GT *G, con
   constexpr int E = Sh::E, T = E * N * N;
   constexpr size_t smem = FxLayout<N, E, GT, EVEC, Sh::NB>::total;
   const auto kernel = bk5fx_kernel<N, E, Sh::MB, Sh::NB, GT, EVEC, NC, SYM, MT, EXPIRE>;
-  static int per_sm = -1;
-  if (per_sm < 0) per_sm = std::max(1, ctas_per_sm_beside(kernel, T, smem));
+  static PerDevice found;
+  const int per_sm = found([&] { return std::max(1, ctas_per_sm_beside(kernel, T, smem)); });
   const int64_t nb = (n_cells + E - 1) / E;
   const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(nb, (int64_t)per_sm * num_sms()));
   return launch_after(after, kernel, grid, T, smem, s, n_cells, map, G, gexp, src, dst, b, done,

@@ -83,8 +83,8 @@ inline cudaError_t gaussfx_run(int64_t n_cells, const uint32_t *map, const GT *G
   constexpr int E = Sh::E, T = E * NQ * NQ;
   constexpr size_t smem = GaussLayout<NM, NQ, E, EVEC, 6, 2>::total;
   const auto kernel = gaussfx_kernel<NM, NQ, E, Sh::MB, GT, EVEC, SYM, MASS, MT>;
-  static int per_sm = -1;
-  if (per_sm < 0) per_sm = std::max(1, ctas_per_sm_beside(kernel, T, smem));
+  static PerDevice found;
+  const int per_sm = found([&] { return std::max(1, ctas_per_sm_beside(kernel, T, smem)); });
   const int64_t batches = (n_cells + E - 1) / E;
   const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(batches, (int64_t)per_sm * num_sms()));
   return launch_after(after, kernel, grid, T, smem, s, n_cells, map, G, gexp, src, dst, b, done,

@@ -1,12 +1,36 @@
 // mfgb_internal.h -- host-side internals shared by the library's translation units.
 #pragma once
 #include <cuda_runtime.h>
+#include <atomic>
 #include <cstdint>
 #include <string>
 
 #include <vector>
 
 #include "mfgb.h"
+
+namespace mfgb {
+// A kernel's launch limit, found once per device by f() >= 0, which also sets the kernel's attributes
+// there (they are per device too).
+class PerDevice {
+  std::atomic<int> found_[64] = {};  // value + 1, 0: not found yet
+
+ public:
+  template <class F>
+  int get(int dev, F f) {
+    if (dev < 0 || dev >= 64) return f();
+    int v = found_[dev].load(std::memory_order_acquire);
+    if (!v) found_[dev].store(v = f() + 1, std::memory_order_release);
+    return v - 1;
+  }
+  template <class F>
+  int operator()(F f) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    return get(dev, f);
+  }
+};
+}  // namespace mfgb
 
 struct mfgb_operator {
   int degree = 0;

@@ -3,6 +3,7 @@
 #include <algorithm>
 #include "mfgb_bk5.cuh"
 #include "mfgb_bk5line.cuh"
+#include "mfgb_internal.h"
 
 namespace mfgb {
 
@@ -213,8 +214,8 @@ cudaError_t line_run(int64_t n_cells, const uint32_t *map, const typename A::GTy
   constexpr int E = Sh::E, T = E * N * N;
   constexpr size_t smem = LineLayout<N, E, typename A::VecT, Sh::NB>::total;
   const auto kernel = bk5_line_kernel<N, E, Sh::MB, Sh::NB, A>;
-  static int per_sm = -1;
-  if (per_sm < 0) per_sm = std::max(1, ctas_per_sm(kernel, T, smem));
+  static PerDevice found;
+  const int per_sm = found([&] { return std::max(1, ctas_per_sm(kernel, T, smem)); });
   const int64_t nb = (n_cells + E - 1) / E;
   const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(nb, (int64_t)per_sm * num_sms()));
   if (grid_used) *grid_used = grid;

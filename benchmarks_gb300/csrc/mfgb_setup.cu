@@ -599,13 +599,13 @@ cudaError_t set_cbits(int64_t n, int64_t nc, const int64_t *c, uint32_t *bits, c
 cudaError_t start_vmult(int64_t n, int ncomp, const uint32_t *bits, const double *src, double *dst,
                         cudaStream_t s) {
   if (n == 0) return cudaSuccess;
-  static const bool split = [] {  // the split of the SM the operator kernels ask for
+  static PerDevice split;  // of the SM, as the operator kernels ask for it
+  split([] {
     for (auto kernel : {start_vmult_kernel<1>, start_vmult_kernel<3>})
       cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                            cudaSharedmemCarveoutMaxShared);
-    return true;
-  }();
-  (void)split;
+    return 1;
+  });
   if (ncomp == 3)
     start_vmult_kernel<3><<<grid_for((n + 7) / 8), 256, 0, s>>>(n, bits, src, dst);
   else
