@@ -217,7 +217,7 @@ mfgb_status vmult_impl(mfgb_operator *op, double *dst, const double *src, int ar
 // shape per degree measured on a GB300 at ~3e7 DoFs (autotune.py re-measures).
 static int g_shape[3][10] = {
     {0, 0, 4, 3, 2, 4, 2, 2, 2, 2},  // FP64
-    {2, 2, 5, 5, 5, 5, 5, 5, 5, 5},  // double-float (5, 6: offset accumulation)
+    {2, 2, 5, 5, 5, 5, 5, 5, 5, 6},  // double-float (5, 6: offset accumulation)
     {0, 0, 3, 2, 2, 2, 2, 2, 2, 2},  // FP32
 };
 
@@ -889,9 +889,9 @@ mfgb_status mfgb_vmult_host(const mfgb_operator *cop, double *h_dst, const doubl
   const int nz = op->is_box ? op->box.nz : 1;
   // >= 2 cell layers a slab.  Every slab costs two copies and two launches, and the first copy in
   // and the last one out are not overlapped: the best count grows with the square root of the
-  // vector.  Measured best counts (double-float, us against 16 slabs): 8 MB 2 (120 / 189), 17 MB 3
-  // (193 / 342), 33 MB 6 (303 / 415), 65 MB 6-10 (530 / 541), 136 MB 8 (999 / 1020), 159 MB 10
-  // (1166 / 1184), 456 MB 16-24 (3006 / 3021).
+  // vector.  Double-float p = 4, us against 16 slabs: 8 MB 122 / 191, 17 MB 198 / 342, 33 MB 312 / 426,
+  // 65 MB 542 / 535, 136 MB 995 / 1026 on one box and 1,018 with either on another, 163 MB 1,165 /
+  // 1,200, 255 MB 1,763 / 1,783; from 457 MB the count is 16 and more.
   const int fit = std::max(2, (int)std::lround(0.75 * std::sqrt(8e-6 * (double)op->n_dofs)));
   const int want = g_host_slabs > 0 ? g_host_slabs : std::min(fit, 24);
   const int S = op->is_box ? std::max(1, std::min(want, nz / 2)) : 1;

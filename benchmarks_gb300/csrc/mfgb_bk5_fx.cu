@@ -14,11 +14,13 @@ namespace mfgb {
 // Cells per CTA, resident CTAs per SM and work arrays of the two thread-block shapes (5 and 6 of
 // the shape table).  Cells per CTA fill whole warps as far as they can (n = 5: 125 of 128 lanes,
 // n = 6: 108 of 128, n = 7: 147 of 160); from n = 5 the two-array form buys one more resident CTA
-// (n = 5: 44.8 KB a CTA, 96 registers, 5 CTAs: 0.649 ms at 3e7 DoFs; three arrays, 4 CTAs: 0.654).
-// ms at 3e7 DoFs, shape 5 / 6: n = 2 3.05 / 3.11, 3 1.21 / 1.21, 4 0.74 / 0.75, 5 0.65 / 0.65,
-// 6 0.70 / 0.73, 7 0.72 / 0.81, 8 0.63 / 0.65, 9 0.80 / 0.80 (the kernel with one contraction
-// output per thread and step that this one replaced, its better shape: 3.90, 1.97, 1.06, 1.00,
-// 1.14, 1.33, 1.07, 1.83).
+// (n = 5: 44.8 KB a CTA, 96 registers, 5 CTAs).
+// Kernel ms at 3e7 DoFs, shape 5 / 6: n = 2 3.07 / 3.12, 3 1.23 / 1.22, 4 0.745 / 0.745, 5 0.653 / 0.660,
+// 6 0.708 / 0.706, 7 0.722 / 0.779, 8 0.629 / 0.652, 9 0.837 / 0.830 and at 8e6 DoFs 0.239 / 0.229 (its
+// default is shape 6).  The kernel with one contraction output per thread and step that this one replaced,
+// its better shape: 3.47, 1.85, 0.93, 0.92, 1.02, 1.20, 1.00, 1.45.  Measured for the scalar operator on
+// pairs; BK6 (three components) and the seams on the caller's FP64 G take the cells per CTA of shape 5,
+// which were not tried one by one for them.
 template <int E_, int MB_, int NB_> struct FxShape {
   static constexpr int E = E_, MB = MB_, NB = NB_;
 };
