@@ -27,7 +27,7 @@
 //   TwoSum-based form of ArithDF, with an error of about 2^-46 of C.  The bounds
 //   B come from the data at hand: each line's maximum for the gradient and the
 //   transpose, max |q| times the row sum of |G| per point for the metric.  (The
-//   cell's bound |u| < 1 for the gradient was 0.6 % faster, but with the two sums
+//   cell's bound |u| < 1 for the gradient was 0.6 to 1.8 % faster, but with the two sums
 //   of the even-odd form its error exceeded the plain form's on values that are
 //   not spread evenly: up to 1.5 times at p = 2 on a constant plus small changes,
 //   1.1 to 1.35 on values over 60 binades.)
@@ -35,12 +35,11 @@
 // * Line ownership (mfgb_fxline.cuh).  In every contraction a thread owns a whole
 //   line, with the derivative matrix in even-odd form.
 //
-// What bounds it (p = 4, ncu at 3e7 DoFs, before the lines were dealt to banks): 1,250
-// warp-instructions a cell against 1,637 of the kernel with one output per thread and step (FADD +
-// FFMA 751 against 963, shared loads and stores 82 against 133), 70 % of the issue slots, 73 % of
-// the shared-memory pipe, 5 CTAs an SM instead of 4.  67.6M DoFs: a vmult 2.22 -> 1.59 ms; 43 -> 45 GDoF/s at
-// 3e7 with the dealt lines, 79 % of the measured copy bandwidth; p = 6 and 8 (n^4 arithmetic per
-// n^3 bytes) stay at 62 % and 51 %, bound by issue.
+// What bounds it (p = 4, ncu at 8.5e6 DoFs): 1,299 warp-instructions a cell against 1,637 of the
+// kernel with one output per thread and step, 69 % of the issue slots, 70 % of the shared-memory
+// pipe, 5 CTAs an SM instead of 4.  67.6M DoFs: a vmult 2.22 -> 1.60 ms, 77 % of the measured copy
+// bandwidth in the kernel; p = 6 and 8 (n^4 arithmetic per n^3 bytes) stay near 61 % and 49 %, bound by
+// issue.
 //
 // Float32 restatements of this arithmetic with their error bounds are in
 // tests/test_fx_arith.py and tests/test_fx_line.py.
@@ -350,7 +349,6 @@ __global__ void __launch_bounds__(E * N * N, MB)
     const bool okg = mbar_wait(mbar_g, ph_g, wlim);
     if (__syncthreads_or(!okg)) { fail(ph_g, ph_m); return; }  // barrier A
     ph_g ^= 1u;
-    T.load_g_plain(batch, tid, blockDim.x);  // ordered before the metric by barrier B
     const bool valid = el < T.cells_of(batch);
     const GT *Gc = sG + el * 6 * N3 + jk;
     if constexpr (G64) {  // the cell's largest G exponent (read after barrier B)

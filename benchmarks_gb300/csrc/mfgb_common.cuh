@@ -252,7 +252,7 @@ __device__ __forceinline__ void even_odd_apply(const typename A::V (&P)[(N + 1) 
 }
 
 // Sum of v over the T threads of a CTA (a power of two >= 64), valid in thread 0; sh holds T doubles
-// and may be reused after a barrier.  FP64 additions run at 1/48 of the FP32 rate here, so the tree
+// and may be reused after a barrier.  FP64 instructions run at 1/70 of the FP32 rate here, so the tree
 // keeps idle lanes out of them: 12 warp-instructions at T = 256, against 40 of shuffles in every
 // warp.
 template <int T>

@@ -10,8 +10,9 @@
 
 namespace mfgb {
 
-// Cells per CTA and resident CTAs per SM, the fastest of two to four tried per size (1.5e7 DoFs, ms;
-// in brackets the best other one).  NQ = NM: 2 1.89 [1.91], 3 0.79 [0.79], 4 0.52 [0.52], 5 0.467
+// Cells per CTA and resident CTAs per SM, the fastest of two to four tried per size for the operators on
+// pairs (1.5e7 DoFs, kernel ms; in brackets the best other one; BK3 on the caller's FP64 G takes the
+// same, not tried for it).  NQ = NM: 2 1.89 [1.91], 3 0.79 [0.79], 4 0.52 [0.52], 5 0.467
 // [0.469], 6 0.547 [0.550], 7 0.56 [0.63], 8 0.51 [0.52], 9 0.72 [0.74].  NQ = NM + 1: 3 5.22
 // [5.43], 4 1.50 [1.55], 5 0.98 [1.00], 6 0.85 [0.92], 7 0.84 [0.87], 8 0.73 [0.74], 9 0.83 [0.88],
 // 10 1.05 [1.13].

@@ -137,9 +137,10 @@ cudaError_t launch_after(bool after, void (*kernel)(P...), int grid, int threads
 // Shapes 2 and 4 of the plain arithmetics as the line kernel (mfgb_bk5line.cuh): cells per CTA,
 // resident CTAs and work arrays.  FP32 at every degree, FP64 from N = 6 (below, the column kernel's
 // 4.05 / 3.82 ms at N = 4, 5 are not beaten: 4.62 / 3.86; the FP64 pipe is the bound and the even-odd
-// additions cost as much as the multiply-adds they save).  Kernel ms at 3e7 DoFs, FP32, N = 3..9: 0.67,
-// 0.40, 0.32, 0.28, 0.26, 0.23, 0.24 (vmult with the best earlier shape: 0.75, 0.44, 0.43, 0.36, 0.51,
-// 0.28, 0.42); FP64, N = 6..9: 4.24, 4.16, 3.87, 4.67 (4.48, 4.63, 4.18, 4.99).
+// additions cost as much as the multiply-adds they save).  One application (clearing, kernel, identity
+// rows) at 3e7 DoFs in ms against the same with the best earlier shape: FP32, N = 3..9 0.68 / 0.75, 0.42 /
+// 0.50, 0.36 / 0.51, 0.32 / 0.36, 0.30 / 0.51, 0.27 / 0.28, 0.28 / 0.42; FP64, N = 6..9 4.28 / 4.49, 4.21 /
+// 4.63, 3.91 / 4.34, 4.71 / 5.00.
 template <int E_, int MB_, int NB_> struct LineShapeIs {
   static constexpr int E = E_, MB = MB_, NB = NB_;
 };
